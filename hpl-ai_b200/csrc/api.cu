@@ -1180,6 +1180,7 @@ int refine_core(hplai_ctx *c, int mode, bool trans, const double *rhs, double no
 	if (err) *err = hplai_ir_errors{-1.0, -1.0};
 	if (iters) *iters = 0;
 	if (mode == HPLAI_GMRES) HPLAI_TRY(ensure_gmres_buffers(c));
+	HPLAI_TRY(trsv_status_reset(c->trsv_work, st));
 	PhaseEvents pe;
 	// x_0 = b ./ diag(A)   (iterative_refinement.hpp:31-34)
 	HPLAI_TRY(launch_div(n, rhs, c->d, x, st));

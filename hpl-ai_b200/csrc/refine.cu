@@ -9,6 +9,7 @@
 //  infnorm, div, axpy   the vector helpers of panel_norm.hpp / panel.hpp.
 #include "common.cuh"
 #include "internal.h"
+#include "tri_inv.cuh"
 
 #include <mutex>
 
@@ -208,66 +209,69 @@ __global__ void __launch_bounds__(GEMV_ROWS) higham_partial_kernel(int n, double
 // ---------------------------------------------------------------------------
 // Triangular solves.  Block rows of TB; CTA c handles block rows c, c+G, ...
 // in solve order, accumulating the off-diagonal products as the block
-// columns it depends on are published (flag[cb] == epoch), then solving its
-// diagonal block with warp shuffles and publishing x for that block.
+// columns it depends on are published, then applying the FP64 inverse of its
+// diagonal block and publishing x for that block.
 // Progress is guaranteed because every CTA is resident (cooperative launch)
 // and each works through its rows in dependency order.  Every spin is
 // bounded; a timeout sets the status word and the kernel returns.
 // ---------------------------------------------------------------------------
-constexpr int TB = 128;
-constexpr int TRSV_THREADS = 256;
+constexpr int TB = kTriBlock;
+constexpr int TRSV_THREADS = kTriThreads;
 
+// Zeroed once by the caller.  `epoch` counts the solves done on this
+// workspace; the last CTA of a launch (counted in `done`) advances it.
 struct TrsvWork {
 	uint32_t epoch;
 	uint32_t status;
-	uint32_t pad[2];
-	// followed by flags[nbt]
+	uint32_t done;
+	uint32_t pad;
+	// followed, 16-byte aligned, by the published solution: element j as two
+	// 64-bit words, each the launch's epoch (high half) and one half of the
+	// double's bits, so that a reader sees value and flag in one load
 };
 
-__global__ void trsv_epoch_kernel(TrsvWork *w)
+__device__ __forceinline__ void xt_publish(ulonglong2 *p, double v, uint32_t epoch)
 {
-	w->epoch += 1;
-	w->status = 0;
+	const uint64_t e = static_cast<uint64_t>(epoch) << 32;
+	const uint64_t lo = e | static_cast<uint32_t>(__double2loint(v)), hi = e | static_cast<uint32_t>(__double2hiint(v));
+	asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(lo), "l"(hi) : "memory");
+}
+
+__device__ __forceinline__ ulonglong2 xt_load(const ulonglong2 *p)
+{
+	ulonglong2 v;
+	asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+	return v;
+}
+
+__device__ __forceinline__ bool xt_ready(ulonglong2 v, uint32_t epoch)
+{
+	return static_cast<uint32_t>(v.x >> 32) == epoch && static_cast<uint32_t>(v.y >> 32) == epoch;
+}
+
+__device__ __forceinline__ double xt_value(ulonglong2 v)
+{
+	return __hiloint2double(static_cast<int>(static_cast<uint32_t>(v.y)), static_cast<int>(static_cast<uint32_t>(v.x)));
 }
 
 // FP64 inverses of the TB x TB diagonal blocks of the stored factors:
 // dinv[(2*r + 0) * TB*TB + c*TB + i] = (L_rr^{-1})[i][c] (unit lower) and
 // dinv[(2*r + 1) * TB*TB + c*TB + i] = (U_rr^{-1})[i][c], rows/columns past
-// n padded with the identity.  Thread c solves T x = e_c by substitution in
-// FP64 (the FP32 factor entries convert exactly).  Computed once per
-// factorisation; the triangular solves then apply a block as one product.
-__global__ void __launch_bounds__(TB) trsv_dinv_kernel(int n, const float *__restrict__ a, int64_t lda,
+// n padded with the identity.  Computed once per factorisation; the
+// triangular solves then apply a block as one product.
+__global__ void __launch_bounds__(TRSV_THREADS) trsv_dinv_kernel(int n, const float *__restrict__ a, int64_t lda,
 	double *__restrict__ dinv, int blk0)
 {
 	extern __shared__ __align__(16) float dyn_smem[];
-	float (*tb)[TB + 1] = reinterpret_cast<float (*)[TB + 1]>(dyn_smem);                 // tb[i][j] = A[r0+i][r0+j]
-	double *xc = reinterpret_cast<double *>(dyn_smem + TB * (TB + 1) + 1);             // xc[i * TB + c], 8-aligned
-	xc = reinterpret_cast<double *>((reinterpret_cast<uintptr_t>(xc) + 7) & ~static_cast<uintptr_t>(7));
+	double *X = reinterpret_cast<double *>(dyn_smem);
 	const int r = blk0 + blockIdx.x, upper = blockIdx.y;
 	const int r0 = r * TB, rows = min(TB, n - r0);
-	const int c = threadIdx.x;
-	for (int e = c; e < TB * TB; e += TB) {
-		const int i = e % TB, j = e / TB;
-		tb[i][j] = (i < rows && j < rows) ? a[static_cast<int64_t>(r0 + j) * lda + r0 + i] : (i == j ? 1.f : 0.f);
-	}
-	__syncthreads();
-	if (!upper) {
-		for (int i = 0; i < TB; ++i) {
-			double v = (i == c) ? 1.0 : 0.0;
-			if (i > c)
-				for (int j = c; j < i; ++j) v = fma(-static_cast<double>(tb[i][j]), xc[j * TB + c], v);
-			xc[i * TB + c] = v;
-		}
-	} else {
-		for (int i = TB - 1; i >= 0; --i) {
-			double v = (i == c) ? 1.0 : 0.0;
-			if (i < c)
-				for (int j = i + 1; j <= c; ++j) v = fma(-static_cast<double>(tb[i][j]), xc[j * TB + c], v);
-			xc[i * TB + c] = (i <= c) ? v / static_cast<double>(tb[i][i]) : 0.0;
-		}
-	}
+	invert_block(X, a, lda, r0, rows, upper != 0);
 	double *out = dinv + (static_cast<int64_t>(2 * r + upper) * TB) * TB;
-	for (int i = 0; i < TB; ++i) out[static_cast<int64_t>(c) * TB + i] = xc[i * TB + c];
+	for (int e = threadIdx.x; e < TB * TB; e += TRSV_THREADS) {
+		const int i = e % TB, c = e / TB;
+		out[e] = upper ? X[c * kInvLd + i] : X[i * kInvLd + c];
+	}
 }
 
 // Copy block (rows r0.., cols c0..) of M into shared memory with cp.async:
@@ -277,16 +281,9 @@ __global__ void __launch_bounds__(TB) trsv_dinv_kernel(int n, const float *__res
 // else 4-byte copies.  The matrix is read-only for the whole solve.
 template <bool TRANS>
 __device__ __forceinline__ void stage_block(float *blk, const float *a, int64_t lda, int r0, int c0, int rows,
-	int cols, bool vec, const double *xsrc = nullptr, double *xdst = nullptr)
+	int cols, bool vec)
 {
 	const int t = threadIdx.x;
-	// x of the block column in the same copy group (its values are published)
-	if (xsrc && t < TB / 2) {
-		int bytes = (cols - 2 * t) * 8;
-		bytes = bytes < 0 ? 0 : (bytes > 16 ? 16 : bytes);
-		asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(xdst + 2 * t)),
-			"l"(xsrc + (bytes ? 2 * t : 0)), "r"(bytes) : "memory");
-	}
 	// contiguous index of the stored matrix: rows for M = stored, columns for M^T
 	const int ncont = TRANS ? cols : rows, nline = TRANS ? rows : cols;
 	if (vec) {
@@ -315,196 +312,172 @@ __device__ __forceinline__ void stage_block(float *blk, const float *a, int64_t 
 // TRANS: the triangle solved is the transpose of the stored one, M[i][j] =
 // a[i*lda + j]: lower = U^T (non-unit), upper = L^T (unit).  Otherwise
 // M[i][j] = a[j*lda + i]: lower = L (unit), upper = U (non-unit).
-// The off-diagonal blocks of a block row stream through two shared-memory
-// buffers: block q+1 is being copied while block q waits for its x and is
-// applied, so the latency of the factor reads leaves the dependency chain.
-// With dinv (the FP64 inverses of the diagonal blocks, trsv_dinv_kernel) a
-// diagonal block is applied as one product instead of 128 dependent
-// substitution steps.
-template <bool TRANS>
+//
+// What bounds it: n / 128 dependent steps (a block's x travels to the next
+// block row's CTA, is multiplied by one 128 x 128 block and by a diagonal
+// inverse), and for large n the one read of the triangle.  So everything a
+// step does not need from the step before it happens while it waits:
+//  - the off-diagonal blocks stream through three shared-memory buffers, two
+//    copies in flight while one block is applied;
+//  - x travels as tagged words (xt_publish): one L2 round trip carries value
+//    and flag, with no fence on the producer's side and no second load on
+//    the consumer's; the words of the next block are requested before the
+//    current one is applied;
+//  - this thread's 64 entries of the diagonal inverse sit in registers (read
+//    from dinv, or, where the caller keeps no inverses (HAVE_INV = false),
+//    computed here by invert_block), so the diagonal is one product of four
+//    short FMA chains.
+// Measured per triangle, before (flag word and fence, 128-step substitution
+// without dinv) and now: n = 8192 197 -> 111 us, transposed 584 -> 135;
+// n = 65536 2.64 -> 2.40 ms (3.6 TB/s); without dinv n = 16384 2350 -> 250 us.
+template <bool TRANS, bool HAVE_INV>
 __global__ void __launch_bounds__(TRSV_THREADS, 1) trsv_kernel(int lower, int n, const float *__restrict__ a,
-	int64_t lda, double *x, TrsvWork *w, const double *__restrict__ dinv)
+	int64_t lda, double *x, TrsvWork *w, ulonglong2 *xt, const double *__restrict__ dinv)
 {
-	extern __shared__ __align__(16) float dyn_smem[];
-	float (*dblk)[TB + 1] = reinterpret_cast<float (*)[TB + 1]>(dyn_smem);   // dblk[i][j] = M[r0+i][r0+j]
-	float *bufs = dyn_smem + TB * (TB + 1) + 3;   // two TB x TB blocks, 16-byte aligned
-	bufs = reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(bufs) + 15) & ~static_cast<uintptr_t>(15));
-	// With the diagonal inverses the staged diagonal block is not needed and
-	// its space becomes a third block buffer: two blocks in flight while one
-	// is applied.
-	const int NB = dinv ? 3 : 2;
-	float *const bufp[3] = {bufs, bufs + TB * TB, dyn_smem};
-	const bool unit = TRANS ? !lower : lower;
+	extern __shared__ __align__(16) float dyn_smem[];   // three TB x TB blocks
+	constexpr int NB = 3;
 	const bool vec = ((reinterpret_cast<uintptr_t>(a) & 15u) == 0) && ((lda & 3) == 0);
-	const bool xvec = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;   // x copies of 16 bytes
-	__shared__ __align__(16) double xsb[3][TB];   // x of the staged block columns, one per block buffer
-	__shared__ double part[2][TB];       // partial sums of the two column halves
-	__shared__ double rhs[TB];
-	__shared__ int ready_upto;
-	__shared__ int abort_flag;
+	__shared__ __align__(16) double xsb[2][TB];   // x of the block columns, alternating
+	__shared__ __align__(16) double part[2][TB];  // partial sums of the two column halves
+	__shared__ __align__(16) double rhs[TB];
 
-	uint32_t *flags = reinterpret_cast<uint32_t *>(w + 1);
-	const uint32_t epoch = *reinterpret_cast<volatile uint32_t *>(&w->epoch);
+	const uint32_t epoch = *reinterpret_cast<volatile uint32_t *>(&w->epoch) + 1u;
 	const int nbt = (n + TB - 1) / TB;
 	const int t = threadIdx.x;
 	const int lr = t % TB, grp = t / TB;   // row within the block, column half
+	const int jb = grp * (TB / 2);
+	bool bad = false;
 
-	// the published prefix seen so far: flags only advance during a launch,
-	// so it carries over from one block row of this CTA to its next
-	if (t == 0) {
-		abort_flag = 0;
-		ready_upto = lower ? 0 : nbt - 1;
-	}
-	__syncthreads();
 	for (int idx = blockIdx.x; idx < nbt; idx += gridDim.x) {
 		const int r = lower ? idx : nbt - 1 - idx;
 		const int r0 = r * TB;
 		const int rows = min(TB, n - r0);
 		const int nblk = lower ? r : nbt - 1 - r;
+		auto col_of = [&](int q) { return lower ? q : nbt - 1 - q; };
 		// the first NB - 1 off-diagonal blocks in flight before anything waits;
 		// one copy group per block (empty past the last) keeps the count fixed
-		// With the block goes its x when the block column is already known to
-		// be solved (the published prefix warp 0 has seen; the same for every
-		// thread between two barriers), so that applying it waits on nothing
-		// but its copy group.
-		bool xpre[3] = {false, false, false};
 		auto stage_q = [&](int q) {
 			if (q < nblk) {
-				const int cb = lower ? q : nbt - 1 - q;
-				const bool known = xvec && (lower ? (cb < ready_upto) : (cb > ready_upto));
-				xpre[q % NB] = known;
-				stage_block<TRANS>(bufp[q % NB], a, lda, r0, cb * TB, rows, min(TB, n - cb * TB), vec,
-					known ? x + static_cast<int64_t>(cb) * TB : nullptr, xsb[q % NB]);
+				const int cb = col_of(q);
+				stage_block<TRANS>(dyn_smem + (q % NB) * TB * TB, a, lda, r0, cb * TB, rows, min(TB, n - cb * TB), vec);
 			} else {
 				asm volatile("cp.async.commit_group;" ::: "memory");
 			}
 		};
-		// the diagonal block's inverse (M^{-1} = T^{-1} or its transpose) into L2
-		const double *dblock = nullptr;
-		if (dinv) {
-			const int tri = (lower != 0) == !TRANS ? 0 : 1;   // L for lower / L^T, U for upper / U^T
-			dblock = dinv + (static_cast<int64_t>(2 * r + tri) * TB) * TB;
-			if (t < 8)
-				asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(dblock + t * (TB * TB / 8)),
-					"r"(static_cast<unsigned>(sizeof(double) * TB * TB / 8)) : "memory");
-		}
-		// Not transposed: this thread's 64 entries of the inverse go to registers
-		// now, while the block row is summed, so that the diagonal step (the
-		// chain's critical path) does not wait on L2.
 		// this block's right-hand side (only this CTA writes it, at the end)
 		const double xr = (t < rows) ? __ldcg(&x[r0 + t]) : 0.0;
+		// dv[q] = M_rr^{-1}[lr][jb + q]
 		double dv[TB / 2];
-		if (!TRANS && dinv) {
-			const int jb = grp * (TB / 2);
+		if (HAVE_INV) {
+			const int tri = (lower != 0) == !TRANS ? 0 : 1;   // L for lower / L^T, U for upper / U^T
+			const double *dblock = dinv + (static_cast<int64_t>(2 * r + tri) * TB) * TB;
+			if (TRANS) {
+				const double2 *row = reinterpret_cast<const double2 *>(dblock + static_cast<int64_t>(lr) * TB + jb);
 #pragma unroll
-			for (int q = 0; q < TB / 2; ++q) dv[q] = __ldcg(&dblock[static_cast<int64_t>(jb + q) * TB + lr]);
-		}
-		// Stage the diagonal block (independent of other CTAs).
-		for (int e = t; !dinv && e < TB * TB; e += TRSV_THREADS) {
-			// consecutive threads take the contiguous index of the stored matrix
-			const int i = TRANS ? e / TB : e % TB, jj = TRANS ? e % TB : e / TB;
-			const int64_t off = TRANS ? static_cast<int64_t>(r0 + i) * lda + r0 + jj : static_cast<int64_t>(r0 + jj) * lda + r0 + i;
-			dblk[i][jj] = (i < rows && jj < rows) ? a[off] : 0.f;
+				for (int q = 0; q < TB / 4; ++q) {
+					const double2 d2 = __ldcg(&row[q]);
+					dv[2 * q] = d2.x;
+					dv[2 * q + 1] = d2.y;
+				}
+			} else {
+#pragma unroll
+				for (int q = 0; q < TB / 2; ++q) dv[q] = __ldcg(&dblock[static_cast<int64_t>(jb + q) * TB + lr]);
+			}
+		} else {
+			double *X = reinterpret_cast<double *>(dyn_smem);
+			invert_block(X, a, lda, r0, rows, lower == 0);
+#pragma unroll
+			for (int q = 0; q < TB / 2; ++q) dv[q] = lower ? X[lr * kInvLd + jb + q] : X[(jb + q) * kInvLd + lr];
+			__syncthreads();
 		}
 		double acc4[4] = {0.0, 0.0, 0.0, 0.0};
 		// TRANS: warp `wv` takes rows wv, wv + 8, ...; lane takes 4 columns
 		double tacc[TB / 8];
 #pragma unroll
 		for (int q = 0; q < TB / 8; ++q) tacc[q] = 0.0;
-		__syncthreads();
 		for (int q = 0; q < NB - 1; ++q) stage_q(q);
-		// Off-diagonal block columns in dependency order: one barrier per
-		// block.  Before it, warp 0 makes sure x of the block is published and
-		// loads it, and every thread waits for its own copies of the block;
-		// after it, the buffer of the previous block (every thread is done
-		// with it) receives the block NB - 1 ahead, and the block is applied.
+		ulonglong2 xw = make_ulonglong2(0, 0);
+		if (t < TB && nblk > 0) xw = xt_load(xt + static_cast<int64_t>(col_of(0)) * TB + t);
+		// Off-diagonal block columns in dependency order, one barrier per block.
+		// Before it, the first four warps make sure that x of the block is
+		// published and put it in shared memory, and every thread waits for its
+		// own copies of the block; after it, the buffer of the previous block
+		// receives the block NB - 1 ahead, and the block is applied.
 		for (int q = 0; q < nblk; ++q) {
-			const int cb = lower ? q : nbt - 1 - q;
-			const int cols = min(TB, n - cb * TB);
-			const float *cur = bufp[q % NB];
-			double *xs = xsb[q % NB];
-			if (t < 32 && !xpre[q % NB]) {
-				// Learn how far the published prefix reaches, 32 flags at a time.
-				bool have = lower ? (cb < ready_upto) : (cb > ready_upto);
-				if (!have) {
-					const uint64_t t0 = global_ns();
-					while (true) {
-						const int probe = lower ? cb + t : cb - t;
-						const bool inb = lower ? (probe < r) : (probe > r);
-						const bool rdy = inb && ld_acquire_u32(&flags[probe]) == epoch;
-						const unsigned m = __ballot_sync(0xffffffffu, rdy);
-						const int cnt = __ffs(~m) - 1;   // leading ready flags
-						const int c = (m == 0xffffffffu) ? 32 : cnt;
-						if (c > 0) {
-							if (t == 0) ready_upto = lower ? cb + c : cb - c;
+			double *xs = xsb[q & 1];
+			if (t < TB) {
+				const int j = col_of(q) * TB + t;
+				const ulonglong2 *src = xt + j;
+				uint64_t t0 = 0;
+				for (int it = 0; __any_sync(0xffffffffu, j < n && !xt_ready(xw, epoch)); ++it) {
+					// the decision to give up is taken by the whole warp at once
+					if ((it & 255) == 0) {
+						const uint64_t now = global_ns();
+						if (it == 0) t0 = now;
+						if (__any_sync(0xffffffffu, now - t0 > kWaitLimitNs)) {
+							bad = true;
 							break;
 						}
-						// the decision to give up is taken by the whole warp at once
-						if (__ballot_sync(0xffffffffu, global_ns() - t0 > kWaitLimitNs)) {
-							if (t == 0) abort_flag = 1;
-							break;
-						}
-						__nanosleep(100);
 					}
+					xw = xt_load(src);
 				}
-				// x of this block column, published by another CTA: bypass L1
-#pragma unroll
-				for (int k = 0; k < TB / 32; ++k) {
-					const int j = cb * TB + t + 32 * k;
-					xs[t + 32 * k] = (j < n) ? __ldcg(&x[j]) : 0.0;
-				}
+				xs[t] = (j < n) ? xt_value(xw) : 0.0;
 			}
-			// block q has landed (the NB - 2 blocks after it may still be in flight)
-			if (NB == 3)
-				asm volatile("cp.async.wait_group 1;" ::: "memory");
-			else
-				asm volatile("cp.async.wait_group 0;" ::: "memory");
-			__syncthreads();
-			if (abort_flag) break;
+			// block q has landed (the one after it may still be in flight)
+			asm volatile("cp.async.wait_group 1;" ::: "memory");
+			bad = __syncthreads_or(bad) != 0;
+			if (bad) break;
 			stage_q(q + NB - 1);
+			if (t < TB && q + 1 < nblk) xw = xt_load(xt + static_cast<int64_t>(col_of(q + 1)) * TB + t);
+			const float *cur = dyn_smem + (q % NB) * TB * TB;
 			if (TRANS) {
-				const int wv = t >> 5, ln = t & 31;
-				const int j = 4 * ln;
-				if (j < cols) {
-					const double x0 = xs[j], x1 = xs[j + 1], x2 = xs[j + 2], x3 = xs[j + 3];
+				const int wv = t >> 5, j = 4 * (t & 31);
+				const double x0 = xs[j], x1 = xs[j + 1], x2 = xs[j + 2], x3 = xs[j + 3];
 #pragma unroll
-					for (int qq = 0; qq < TB / 8; ++qq) {
-						const int i = wv + 8 * qq;
-						const float4 v = *reinterpret_cast<const float4 *>(cur + i * TB + j);
-						double s4 = tacc[qq];
-						s4 = fma(static_cast<double>(v.x), x0, s4);
-						s4 = fma(static_cast<double>(v.y), x1, s4);
-						s4 = fma(static_cast<double>(v.z), x2, s4);
-						s4 = fma(static_cast<double>(v.w), x3, s4);
-						tacc[qq] = s4;
-					}
+				for (int qq = 0; qq < TB / 8; ++qq) {
+					const int i = wv + 8 * qq;
+					const float4 v = *reinterpret_cast<const float4 *>(cur + i * TB + j);
+					double s4 = tacc[qq];
+					s4 = fma(static_cast<double>(v.x), x0, s4);
+					s4 = fma(static_cast<double>(v.y), x1, s4);
+					s4 = fma(static_cast<double>(v.z), x2, s4);
+					s4 = fma(static_cast<double>(v.w), x3, s4);
+					tacc[qq] = s4;
 				}
-			} else if (lr < rows) {
+			} else {
 				// four independent FMA chains: one chain of 64 dependent FMAs per
 				// block left the FP64 pipe waiting on its own latency
-				const int jb = grp * (TB / 2), je = min(jb + TB / 2, cols);
-				int j = jb;
-				for (; j + 3 < je; j += 4) {
-					acc4[0] = fma(static_cast<double>(cur[j * TB + lr]), xs[j], acc4[0]);
-					acc4[1] = fma(static_cast<double>(cur[(j + 1) * TB + lr]), xs[j + 1], acc4[1]);
-					acc4[2] = fma(static_cast<double>(cur[(j + 2) * TB + lr]), xs[j + 2], acc4[2]);
-					acc4[3] = fma(static_cast<double>(cur[(j + 3) * TB + lr]), xs[j + 3], acc4[3]);
+#pragma unroll
+				for (int k = 0; k < TB / 2; k += 4) {
+					const int j = jb + k;
+					const double2 x01 = *reinterpret_cast<const double2 *>(&xs[j]);
+					const double2 x23 = *reinterpret_cast<const double2 *>(&xs[j + 2]);
+					acc4[0] = fma(static_cast<double>(cur[j * TB + lr]), x01.x, acc4[0]);
+					acc4[1] = fma(static_cast<double>(cur[(j + 1) * TB + lr]), x01.y, acc4[1]);
+					acc4[2] = fma(static_cast<double>(cur[(j + 2) * TB + lr]), x23.x, acc4[2]);
+					acc4[3] = fma(static_cast<double>(cur[(j + 3) * TB + lr]), x23.y, acc4[3]);
 				}
-				for (; j < je; ++j) acc4[0] = fma(static_cast<double>(cur[j * TB + lr]), xs[j], acc4[0]);
 			}
 		}
-		if (abort_flag) break;
+		if (bad) break;
 		if (TRANS) {
-			// fold the lanes' partial sums of each row in a fixed order
+			// the 16 rows' sums over 32 lanes: each exchange halves the values a
+			// lane holds, in a fixed order
 			const int wv = t >> 5, ln = t & 31;
 #pragma unroll
-			for (int qq = 0; qq < TB / 8; ++qq) {
-				double v = tacc[qq];
-				for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-				if (ln == 0) {
-					part[0][wv + 8 * qq] = v;
-					part[1][wv + 8 * qq] = 0.0;
+			for (int h = 8, o = 16; h >= 1; h >>= 1, o >>= 1) {
+				const bool up = (ln & o) != 0;
+#pragma unroll
+				for (int q = 0; q < h; ++q) {
+					const double send = up ? tacc[q] : tacc[q + h], keep = up ? tacc[q + h] : tacc[q];
+					tacc[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
 				}
+			}
+			tacc[0] += __shfl_xor_sync(0xffffffffu, tacc[0], 1);
+			const int qq = ((ln >> 4) & 1) * 8 + ((ln >> 3) & 1) * 4 + ((ln >> 2) & 1) * 2 + ((ln >> 1) & 1);
+			if ((ln & 1) == 0) {
+				part[0][wv + 8 * qq] = tacc[0];
+				part[1][wv + 8 * qq] = 0.0;
 			}
 		} else {
 			part[grp][lr] = (acc4[0] + acc4[1]) + (acc4[2] + acc4[3]);
@@ -512,79 +485,36 @@ __global__ void __launch_bounds__(TRSV_THREADS, 1) trsv_kernel(int lower, int n,
 		__syncthreads();
 		if (t < TB) rhs[t] = (t < rows) ? xr - (part[0][t] + part[1][t]) : 0.0;
 		__syncthreads();
-		if (dinv) {
-			// x_r = M_rr^{-1} rhs: element (i, j) of M^{-1} is dblock[j*TB + i], or
-			// dblock[i*TB + j] for the transpose
-			if (TRANS) {
-				const int wv = t >> 5, ln = t & 31;
-#pragma unroll 4
-				for (int qq = 0; qq < TB / 8; ++qq) {
-					const int i = wv + 8 * qq;
-					const double *row = dblock + static_cast<int64_t>(i) * TB + 4 * ln;
-					double v = row[0] * rhs[4 * ln];
-					v = fma(row[1], rhs[4 * ln + 1], v);
-					v = fma(row[2], rhs[4 * ln + 2], v);
-					v = fma(row[3], rhs[4 * ln + 3], v);
-					for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-					if (ln == 0) {
-						part[0][i] = v;
-						part[1][i] = 0.0;
-					}
-				}
-			} else {
-				const int jb = grp * (TB / 2);
-				double v = 0.0;
+		// x_r = M_rr^{-1} rhs
+		double v4[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-				for (int q = 0; q < TB / 2; ++q) v = fma(dv[q], rhs[jb + q], v);
-				part[grp][lr] = v;
-			}
-			__syncthreads();
-			if (t < rows) rhs[t] = part[0][t] + part[1][t];
-			__syncthreads();
+		for (int q = 0; q < TB / 2; q += 4) {
+			const double2 y01 = *reinterpret_cast<const double2 *>(&rhs[jb + q]);
+			const double2 y23 = *reinterpret_cast<const double2 *>(&rhs[jb + q + 2]);
+			v4[0] = fma(dv[q], y01.x, v4[0]);
+			v4[1] = fma(dv[q + 1], y01.y, v4[1]);
+			v4[2] = fma(dv[q + 2], y23.x, v4[2]);
+			v4[3] = fma(dv[q + 3], y23.y, v4[3]);
 		}
-		// Diagonal block: 32-row sub-blocks solved by warp 0 with shuffles,
-		// the remaining rows updated by all threads.
-		const int nsb = dinv ? 0 : (rows + 31) / 32;
-		for (int sblk = 0; sblk < nsb; ++sblk) {
-			const int sb = lower ? sblk : nsb - 1 - sblk;
-			const int base = sb * 32;
-			if (t < 32) {
-				const int i = base + t;
-				double v = (i < rows) ? rhs[i] : 0.0;
-				if (lower) {
-					for (int jj = 0; jj < 32; ++jj) {
-						if (!unit && t == jj && i < rows) v = v / static_cast<double>(dblk[i][i]);
-						const double xj = __shfl_sync(0xffffffffu, v, jj);
-						if (t > jj && base + jj < rows) v = fma(-static_cast<double>(dblk[i][base + jj]), xj, v);
-					}
-				} else {
-					for (int jj = 31; jj >= 0; --jj) {
-						if (!unit && t == jj && i < rows) v = v / static_cast<double>(dblk[i][i]);
-						const double xj = __shfl_sync(0xffffffffu, v, jj);
-						if (t < jj && base + jj < rows) v = fma(-static_cast<double>(dblk[i][base + jj]), xj, v);
-					}
-				}
-				if (i < rows) rhs[i] = v;
-			}
-			__syncthreads();
-			// rows still to solve: below (lower) or above (upper) this sub-block
-			const int lo = lower ? base + 32 : 0;
-			const int hi = lower ? rows : base;
-			for (int i = lo + t; i < hi; i += TRSV_THREADS) {
-				double v = rhs[i];
-				for (int jj = 0; jj < 32 && base + jj < rows; ++jj) v = fma(-static_cast<double>(dblk[i][base + jj]), rhs[base + jj], v);
-				rhs[i] = v;
-			}
-			__syncthreads();
-		}
-		if (t < rows) x[r0 + t] = rhs[t];
-		__threadfence();
+		part[grp][lr] = (v4[0] + v4[1]) + (v4[2] + v4[3]);
 		__syncthreads();
-		if (t == 0) st_release_u32(&flags[r], epoch);
+		if (t < rows) {
+			const double v = part[0][t] + part[1][t];
+			xt_publish(xt + r0 + t, v, epoch);
+			x[r0 + t] = v;
+		}
 	}
 	// copies still in flight after a timeout land before the CTA exits
 	asm volatile("cp.async.wait_all;" ::: "memory");
-	if (t == 0 && abort_flag) atomicOr(&w->status, 1u);
+	if (t == 0) {
+		if (bad) atomicOr(&w->status, 1u);
+		// every CTA has read the epoch before it counts itself done
+		__threadfence();
+		if (atomicAdd(&w->done, 1u) == gridDim.x - 1) {
+			w->done = 0;
+			w->epoch = epoch;
+		}
+	}
 }
 
 // ---------------------------------------------------------------------------
@@ -757,10 +687,11 @@ int launch_otf_gemv_block(int64_t n, int mb, int nb, double alpha, const double 
 	return otf_launch(n, mb, nb, alpha, x, 1.0, y, state00, 0, nullptr, work, work_bytes, st);
 }
 
+// header, alignment slack, two 64-bit words per element of the padded solution
 size_t trsv_workspace(int n)
 {
 	const size_t nbt = (static_cast<size_t>(n) + TB - 1) / TB;
-	return sizeof(TrsvWork) + nbt * sizeof(uint32_t);
+	return sizeof(TrsvWork) + 16 + nbt * TB * sizeof(ulonglong2);
 }
 
 int launch_trsv(bool lower, int n, const float *a, int64_t lda, double *x, void *work, size_t work_bytes,
@@ -768,36 +699,48 @@ int launch_trsv(bool lower, int n, const float *a, int64_t lda, double *x, void 
 {
 	if (n <= 0) return HPLAI_OK;
 	if (!work || work_bytes < trsv_workspace(n)) return HPLAI_EINVAL;
-	constexpr size_t dsmem = sizeof(float) * (TB * (TB + 1) + 3 + 4 + 2 * TB * TB);
+	if (trans && !dinv) return HPLAI_EINVAL;
+	constexpr size_t dsmem = sizeof(float) * 3 * TB * TB;
+	static_assert(kInvSmem<double> <= dsmem, "the in-kernel inverse shares the block buffers");
 	// co-resident CTAs of the cooperative launch on this device
 	static DeviceOnce grid_once;
 	int max_blocks = 0;
 	HPLAI_TRY(grid_once.get([&](int dev, int *v) -> int {
-		int per_sm = 0, per_sm_t = 0, sms = 0;
-		HPLAI_CUDA_TRY(cudaFuncSetAttribute(trsv_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			static_cast<int>(dsmem)));
-		HPLAI_CUDA_TRY(cudaFuncSetAttribute(trsv_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			static_cast<int>(dsmem)));
-		HPLAI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trsv_kernel<false>, TRSV_THREADS, dsmem));
-		HPLAI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_t, trsv_kernel<true>, TRSV_THREADS, dsmem));
+		const void *fns[3] = {reinterpret_cast<const void *>(trsv_kernel<false, false>),
+			reinterpret_cast<const void *>(trsv_kernel<false, true>), reinterpret_cast<const void *>(trsv_kernel<true, true>)};
+		int least = 1 << 30, sms = 0;
+		for (const void *f : fns) {
+			int per_sm = 0;
+			HPLAI_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dsmem)));
+			HPLAI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, TRSV_THREADS, dsmem));
+			least = per_sm < least ? per_sm : least;
+		}
 		HPLAI_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-		*v = (per_sm < per_sm_t ? per_sm : per_sm_t) * sms;
+		*v = least * sms;
 		return HPLAI_OK;
 	}, &max_blocks));
 	if (max_blocks <= 0) return HPLAI_EUNSUPPORTED;
 	// the transposed solve reads rows of the stored matrix as float4
 	if (trans && ((reinterpret_cast<uintptr_t>(a) & 15u) || (lda & 3))) return HPLAI_EINVAL;
 	TrsvWork *w = static_cast<TrsvWork *>(work);
-	trsv_epoch_kernel<<<1, 1, 0, st>>>(w);
-	count_launches();
-	HPLAI_CUDA_TRY(cudaGetLastError());
+	ulonglong2 *xt = reinterpret_cast<ulonglong2 *>((reinterpret_cast<uintptr_t>(w + 1) + 15) & ~static_cast<uintptr_t>(15));
 	const int nbt = (n + TB - 1) / TB;
 	const int grid = nbt < max_blocks ? nbt : max_blocks;
 	int lw = lower ? 1 : 0;
-	void *args[] = {(void *)&lw, (void *)&n, (void *)&a, (void *)&lda, (void *)&x, (void *)&w, (void *)&dinv};
-	void *fn = trans ? reinterpret_cast<void *>(trsv_kernel<true>) : reinterpret_cast<void *>(trsv_kernel<false>);
+	void *args[] = {(void *)&lw, (void *)&n, (void *)&a, (void *)&lda, (void *)&x, (void *)&w, (void *)&xt, (void *)&dinv};
+	const void *fn = trans ? reinterpret_cast<const void *>(trsv_kernel<true, true>)
+		: dinv ? reinterpret_cast<const void *>(trsv_kernel<false, true>)
+		       : reinterpret_cast<const void *>(trsv_kernel<false, false>);
 	HPLAI_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(TRSV_THREADS), args, dsmem, st));
 	count_launches();
+	return HPLAI_OK;
+}
+
+// Clears the timeout word that trsv_status reads.
+int trsv_status_reset(void *work, cudaStream_t st)
+{
+	TrsvWork *w = static_cast<TrsvWork *>(work);
+	HPLAI_CUDA_TRY(cudaMemsetAsync(&w->status, 0, sizeof(w->status), st));
 	return HPLAI_OK;
 }
 
@@ -813,14 +756,13 @@ int launch_trsv_dinv(int n, const float *a, int64_t lda, double *dinv, cudaStrea
 	const int nbt = (n + TB - 1) / TB;
 	if (nblk < 0) nblk = nbt - blk0;
 	if (blk0 < 0 || nblk <= 0 || blk0 + nblk > nbt) return nblk == 0 ? HPLAI_OK : HPLAI_EINVAL;
-	constexpr size_t smem = sizeof(float) * (TB * (TB + 1) + 3) + sizeof(double) * TB * TB;
 	static DeviceOnce attr;
-	HPLAI_TRY(attr.get([&](int, int *) -> int {
+	HPLAI_TRY(attr.get([](int, int *) -> int {
 		HPLAI_CUDA_TRY(cudaFuncSetAttribute(trsv_dinv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			static_cast<int>(smem)));
+			static_cast<int>(kInvSmem<double>)));
 		return HPLAI_OK;
 	}));
-	trsv_dinv_kernel<<<dim3(nblk, 2), TB, smem, st>>>(n, a, lda, dinv, blk0);
+	trsv_dinv_kernel<<<dim3(nblk, 2), TRSV_THREADS, kInvSmem<double>, st>>>(n, a, lda, dinv, blk0);
 	count_launches();
 	HPLAI_CUDA_TRY(cudaGetLastError());
 	return HPLAI_OK;

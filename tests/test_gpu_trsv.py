@@ -1,0 +1,100 @@
+"""The triangular solves (panel_trsv.hpp:310-758) at the sizes where their 128-row blocks can go wrong."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _factors(rng, n):
+    """Column-major LU of a matrix with a dominant diagonal: multipliers near 2/n, U's diagonal near n/4."""
+    m = rng.uniform(-0.5, 0.5, (n, n)).astype(np.float32)
+    m[np.tril_indices(n, -1)] *= np.float32(4.0 / n)
+    m[np.arange(n), np.arange(n)] = np.float32(0.25 * n + 1.0)
+    return m
+
+
+def _solve(m, x, lower):
+    """Substitution in FP64 (the FP32 entries convert exactly)."""
+    a = m.astype(np.float64)
+    y = x.copy()
+    n = len(x)
+    for i in range(n) if lower else reversed(range(n)):
+        y[i] -= a[i, :i] @ y[:i] if lower else a[i, i + 1:] @ y[i + 1:]
+        if not lower:
+            y[i] /= a[i, i]
+    return y
+
+
+# one block and its remainders, whole and ragged block rows, an odd leading dimension and an unaligned base (the
+# 4-byte copies), more block rows than the GPU has SMs
+@pytest.mark.parametrize("n,lda,off", [(1, 1, 0), (31, 32, 0), (127, 129, 0), (128, 128, 0), (129, 132, 0), (257, 257, 1),
+                                       (1000, 1004, 0), (2500, 2501, 3), (19200, 19264, 0)])
+def test_trsv_leaf_edges(hplai, torch_cuda, n, lda, off):
+    """Backward error bound of a triangular solve, n eps |T| |x|, dominated here by a few eps of |x|_inf."""
+    torch = torch_cuda
+    rng = np.random.default_rng(n)
+    if n <= 2500:
+        m = _factors(rng, n)
+        buf = np.zeros(n * lda + off + 4, dtype=np.float32)
+        buf[off:off + n * lda].reshape(n, lda)[:, :n] = m.T   # column j at j * lda
+        a = torch.from_numpy(buf).cuda()
+    else:
+        g = torch.Generator(device="cuda").manual_seed(n)
+        a = torch.zeros((n, lda), device="cuda")
+        a[:, :n] = torch.rand((n, n), generator=g, device="cuda") - 0.5
+        i = torch.arange(n, device="cuda")
+        for c in range(0, n, 2048):
+            a[c:c + 2048, :n].mul_(torch.where(i[None, :] > i[c:c + 2048, None], 4.0 / n, 1.0))
+        a[i, i] = 0.25 * n
+    x = rng.uniform(-1, 1, n)
+    ws = hplai.trsv_workspace(n)
+    w = torch.zeros(ws, dtype=torch.uint8, device="cuda")
+    ptr = a.data_ptr() + 4 * off
+    for lower in (True, False, True):   # one workspace for solve after solve
+        xd = torch.from_numpy(x).cuda()
+        fn = hplai.trsv_lower if lower else hplai.trsv_upper
+        hplai.check(fn(n, ptr, lda, xd.data_ptr(), w.data_ptr(), ws, None))
+        got = xd.cpu().numpy()
+        if n <= 2500:
+            ref = _solve(m, x, lower)
+        else:
+            d = a[:, :n].T.double()
+            ref = torch.linalg.solve_triangular(d, torch.from_numpy(x).cuda()[:, None], upper=not lower,
+                                                unitriangular=lower)[:, 0].cpu().numpy()
+            del d
+        assert np.abs(got - ref).max() <= 1e-13 * np.abs(ref).max(), lower
+
+
+def test_trsv_leaf_workspace_limits(hplai, torch_cuda):
+    """A workspace shared by two orders; one byte too few is refused; an address off the 16-byte boundary works."""
+    torch = torch_cuda
+    rng = np.random.default_rng(5)
+    ws = hplai.trsv_workspace(600)
+    w = torch.zeros(ws + 16, dtype=torch.uint8, device="cuda")
+    for n in (600, 130, 600, 7):
+        m = _factors(rng, n)
+        a = torch.from_numpy(np.ascontiguousarray(m.T)).cuda()
+        x = rng.uniform(-1, 1, n)
+        xd = torch.from_numpy(x).cuda()
+        hplai.check(hplai.trsv_lower(n, a.data_ptr(), n, xd.data_ptr(), w.data_ptr() + 4, ws, None))
+        ref = _solve(m, x, True)
+        assert np.abs(xd.cpu().numpy() - ref).max() <= 1e-13 * np.abs(ref).max()
+    a = torch.zeros((600, 600), device="cuda")
+    xd = torch.zeros(600, dtype=torch.float64, device="cuda")
+    assert hplai.trsv_lower(600, a.data_ptr(), 600, xd.data_ptr(), w.data_ptr(), ws - 1, None) == hplai.HPLAI_EINVAL
+
+
+@pytest.mark.parametrize("n,b", [(100, 100), (700, 100), (1280, 128), (1290, 30)])
+def test_transposed_solve_ragged(hplai, oracle, torch_cuda, n, b):
+    """The transposed triangles (and their register-held inverses) through the adjoint solve: x and lambda against
+    the dense FP64 solves."""
+    g = np.random.default_rng(n).uniform(-1, 1, n)
+    with hplai.Solver(n, b) as s:
+        s.generate(42)
+        s.factor()
+        lam, r = s.solve_transpose(g)
+        x, q = s.solve_rhs(g)
+    assert r.status == hplai.HPLAI_OK and q.status == hplai.HPLAI_OK
+    a = oracle.dense_matrix_f64(n)
+    assert np.abs(lam - np.linalg.solve(a.T, g)).max() <= 1e-12 * np.abs(lam).max()
+    assert np.abs(x - np.linalg.solve(a, g)).max() <= 1e-12 * np.abs(x).max()
