@@ -135,6 +135,34 @@ __device__ __forceinline__ double state_value(uint64_t x)
 	return __dmul_rn(__ll2double_rn((long long)x), kValueScale);
 }
 
+// The LCG state as a signed integer in FP64, rounded to nearest as
+// __ll2double_rn does, for a state kept with its top bit flipped (the
+// recurrence x <- a x + c is unchanged by that: a is odd).  The halves are
+// placed in the mantissas of 2^84 and 2^52; removing 2^84 + 2^63 + 2^52 is
+// exact and the last addition rounds once.
+__device__ __forceinline__ double biased_state_value(uint64_t s)
+{
+	const double hi = __hiloint2double(0x45300000, static_cast<int>(s >> 32));
+	const double lo = __hiloint2double(0x43300000, static_cast<int>(s));
+	return __dadd_rn(__dadd_rn(hi, -0x1.00000801p+84), lo);
+}
+
+// Jump over m elements, m the same in the whole warp: lane k takes bits 2k
+// and 2k + 1, and the powers (which commute) are multiplied across the lanes.
+__device__ __forceinline__ Coeff warp_jump(const Coeff *tab, uint64_t m)
+{
+	const int lane = threadIdx.x & 31;
+	const unsigned bits = static_cast<unsigned>(m >> (2 * lane)) & 3u;
+	Coeff r{1ULL, 0ULL};
+	if (bits & 1u) r = tab[2 * lane];
+	if (bits & 2u) r = coeff_mul(r, tab[2 * lane + 1]);
+	for (int o = 16; o; o >>= 1) {
+		const Coeff q{__shfl_xor_sync(0xffffffffu, r.a, o), __shfl_xor_sync(0xffffffffu, r.c, o)};
+		r = coeff_mul(r, q);
+	}
+	return r;
+}
+
 // ---------------------------------------------------------------------------
 // Bounded waits.
 // ---------------------------------------------------------------------------

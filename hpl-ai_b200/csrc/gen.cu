@@ -46,26 +46,56 @@ __device__ __forceinline__ Coeff jump_of(const JumpTable &t, uint64_t m)
 	return r;
 }
 
-constexpr int kFillRows = 256;  // rows per CTA (one per thread)
+constexpr int kFillRows = 256;  // rows per CTA of the one-row-per-thread kernels
 constexpr int kFillCols = 32;   // columns per CTA
+constexpr int kFillRows4 = 4 * kFillRows;   // rows per CTA of fill_kernel (four per thread)
 
 // a(i, j) for i in [0,nrow), j in [0,ncol) of the sub-matrix at (i0, j0).
+// Bound by the write of the matrix: a thread takes four neighbouring rows
+// (one 16-byte store a column where a and lda allow it), the start state
+// costs one warp-wide jump, and the state's conversion to FP64 leaves the
+// conversion pipe to the rounding to FP32 (biased_state_value).  n = 32768:
+// 1380 us with a row and two jumps per thread, 601 us (7.1 TB/s written) so.
 __global__ void __launch_bounds__(kFillRows) fill_kernel(int n, int i0, int j0, int nrow, int ncol, float *a,
-	int64_t lda, uint64_t seed, JumpTable tab)
+	int64_t lda, uint64_t seed, int vec, JumpTable tab, Coeff jn)
 {
-	const int r = blockIdx.x * kFillRows + threadIdx.x;
+	__shared__ Coeff stab[64];
+	const int t = threadIdx.x, lane = t & 31;
+	if (t < 64) stab[t] = tab.p[t];
+	__syncthreads();
+	const int rw = blockIdx.x * kFillRows4 + (t - lane) * 4;   // the warp's first row
 	const int c0 = blockIdx.y * kFillCols;
-	if (r >= nrow) return;
-	const Coeff jn = jump_of(tab, static_cast<uint64_t>(n));
-	uint64_t s = coeff_apply(jump_of(tab, static_cast<uint64_t>(i0 + r) +
-	                                          static_cast<uint64_t>(n) * static_cast<uint64_t>(j0 + c0)),
+	if (rw >= nrow) return;
+	uint64_t s[4];
+	s[0] = coeff_apply(warp_jump(stab, static_cast<uint64_t>(i0 + rw) +
+	                                       static_cast<uint64_t>(n) * static_cast<uint64_t>(j0 + c0)),
 		state_initial(seed));
+#pragma unroll
+	for (int k = 0; k < 5; ++k)
+		if ((lane >> k) & 1) s[0] = coeff_apply(stab[k + 2], s[0]);
+#pragma unroll
+	for (int q = 1; q < 4; ++q) s[q] = coeff_apply(Coeff{kLcgA, kLcgC}, s[q - 1]);
+#pragma unroll
+	for (int q = 0; q < 4; ++q) s[q] ^= 1ULL << 63;
+	const int r = rw + 4 * lane;
 	const int c1 = min(c0 + kFillCols, ncol);
 	float *col = a + static_cast<int64_t>(c0) * lda + r;
+	const bool whole = vec && r + 3 < nrow;
 	for (int c = c0; c < c1; ++c) {
-		*col = __double2float_rn(state_value(s));
+		float v[4];
+#pragma unroll
+		for (int q = 0; q < 4; ++q) {
+			v[q] = __double2float_rn(__dmul_rn(biased_state_value(s[q]), kValueScale));
+			s[q] = coeff_apply(jn, s[q]);
+		}
+		if (whole) {
+			*reinterpret_cast<float4 *>(col) = make_float4(v[0], v[1], v[2], v[3]);
+		} else {
+#pragma unroll
+			for (int q = 0; q < 4; ++q)
+				if (r + q < nrow) col[q] = v[q];
+		}
 		col += lda;
-		s = coeff_apply(jn, s);
 	}
 }
 
@@ -74,36 +104,53 @@ __global__ void __launch_bounds__(kFillRows) fill_kernel(int n, int i0, int j0, 
 // sequential chain so the rounding matches hpl_rand.hpp:117-121 exactly.
 // Writes the FP64 value to d (if non-null) and/or its FP32 rounding to the
 // matrix diagonal a[(i - i0)*(lda+1)] (if non-null).
+// A warp's 32 rows meet their diagonals within 36 columns, so only those
+// columns are tested for it (n = 32768: 677 -> 499 us; the integer conversion
+// of the state, a pipe of its own, beats biased_state_value here).
 __global__ void __launch_bounds__(128) diag_kernel(int n, int i0, int count, double *d, float *adiag, int64_t lda,
-	uint64_t seed, JumpTable tab)
+	uint64_t seed, JumpTable tab, Coeff jn)
 {
 	const int k = blockIdx.x * blockDim.x + threadIdx.x;
 	if (k >= count) return;
 	const int i = i0 + k;
-	const Coeff jn = jump_of(tab, static_cast<uint64_t>(n));
 	const Coeff jn4 = coeff_mul(coeff_mul(jn, jn), coeff_mul(jn, jn));
 	uint64_t s0 = coeff_apply(jump_of(tab, static_cast<uint64_t>(i)), state_initial(seed));
 	uint64_t s1 = coeff_apply(jn, s0);
 	uint64_t s2 = coeff_apply(jn, s1);
 	uint64_t s3 = coeff_apply(jn, s2);
+	auto value = [](uint64_t s) { return fabs(state_value(s)); };
 	double sum = 0.0;
 	int j = 0;
-	for (; j + 3 < n; j += 4) {
-		const double v0 = fabs(state_value(s0));
-		const double v1 = fabs(state_value(s1));
-		const double v2 = fabs(state_value(s2));
-		const double v3 = fabs(state_value(s3));
-		if (j != i) sum = __dadd_rn(sum, v0);
-		if (j + 1 != i) sum = __dadd_rn(sum, v1);
-		if (j + 2 != i) sum = __dadd_rn(sum, v2);
-		if (j + 3 != i) sum = __dadd_rn(sum, v3);
+	auto plain = [&](int end) {
+#pragma unroll 2
+		for (; j + 3 < end; j += 4) {
+			const double v0 = value(s0), v1 = value(s1), v2 = value(s2), v3 = value(s3);
+			s0 = coeff_apply(jn4, s0);
+			s1 = coeff_apply(jn4, s1);
+			s2 = coeff_apply(jn4, s2);
+			s3 = coeff_apply(jn4, s3);
+			sum = __dadd_rn(sum, v0);
+			sum = __dadd_rn(sum, v1);
+			sum = __dadd_rn(sum, v2);
+			sum = __dadd_rn(sum, v3);
+		}
+	};
+	const int iw = i - static_cast<int>(threadIdx.x & 31);   // the warp's first row
+	plain(min(iw & ~3, n));
+	for (; j < iw + 32 && j + 3 < n; j += 4) {
+		const double v0 = value(s0), v1 = value(s1), v2 = value(s2), v3 = value(s3);
 		s0 = coeff_apply(jn4, s0);
 		s1 = coeff_apply(jn4, s1);
 		s2 = coeff_apply(jn4, s2);
 		s3 = coeff_apply(jn4, s3);
+		if (j != i) sum = __dadd_rn(sum, v0);
+		if (j + 1 != i) sum = __dadd_rn(sum, v1);
+		if (j + 2 != i) sum = __dadd_rn(sum, v2);
+		if (j + 3 != i) sum = __dadd_rn(sum, v3);
 	}
+	plain(n);
 	for (; j < n; ++j) {
-		if (j != i) sum = __dadd_rn(sum, fabs(state_value(s0)));
+		if (j != i) sum = __dadd_rn(sum, value(s0));
 		s0 = coeff_apply(jn, s0);
 	}
 	if (d) d[k] = sum;
@@ -332,12 +379,14 @@ int launch_fill(int n, int i0, int j0, int nrow, int ncol, float *a, int64_t lda
 	cudaStream_t st)
 {
 	if (nrow <= 0 || ncol <= 0) return HPLAI_OK;
-	dim3 grid((nrow + kFillRows - 1) / kFillRows, (ncol + kFillCols - 1) / kFillCols);
-	fill_kernel<<<grid, kFillRows, 0, st>>>(n, i0, j0, nrow, ncol, a, lda, seed, jump_table());
+	dim3 grid((nrow + kFillRows4 - 1) / kFillRows4, (ncol + kFillCols - 1) / kFillCols);
+	const int vec = (reinterpret_cast<uintptr_t>(a) % 16 == 0 && lda % 4 == 0) ? 1 : 0;
+	const Coeff jn = coeff_pow(static_cast<uint64_t>(n));
+	fill_kernel<<<grid, kFillRows, 0, st>>>(n, i0, j0, nrow, ncol, a, lda, seed, vec, jump_table(), jn);
 	count_launches();
 	HPLAI_CUDA_TRY(cudaGetLastError());
 	if (calc_diag && i0 == j0 && nrow == ncol) {
-		diag_kernel<<<(nrow + 127) / 128, 128, 0, st>>>(n, i0, nrow, nullptr, a, lda, seed, jump_table());
+		diag_kernel<<<(nrow + 127) / 128, 128, 0, st>>>(n, i0, nrow, nullptr, a, lda, seed, jump_table(), jn);
 		count_launches();
 		HPLAI_CUDA_TRY(cudaGetLastError());
 	}
@@ -347,7 +396,8 @@ int launch_fill(int n, int i0, int j0, int nrow, int ncol, float *a, int64_t lda
 int launch_diag(int n, int i0, int count, double *d, float *adiag, int64_t lda, uint64_t seed, cudaStream_t st)
 {
 	if (count <= 0) return HPLAI_OK;
-	diag_kernel<<<(count + 127) / 128, 128, 0, st>>>(n, i0, count, d, adiag, lda, seed, jump_table());
+	diag_kernel<<<(count + 127) / 128, 128, 0, st>>>(n, i0, count, d, adiag, lda, seed, jump_table(),
+		coeff_pow(static_cast<uint64_t>(n)));
 	count_launches();
 	HPLAI_CUDA_TRY(cudaGetLastError());
 	return HPLAI_OK;
