@@ -12,6 +12,7 @@
 #include "tri_inv.cuh"
 
 #include <mutex>
+#include <type_traits>
 
 namespace hplai {
 
@@ -38,95 +39,130 @@ const JumpTable64 &table()
 	return t;
 }
 
-__device__ __forceinline__ Coeff jump_of(const JumpTable64 &t, uint64_t m)
-{
-	Coeff r{1ULL, 0ULL};
-	for (int k = 0; m; ++k, m >>= 1)
-		if (m & 1ULL) r = coeff_mul(r, t.p[k]);
-	return r;
-}
-
 // ---------------------------------------------------------------------------
-// On-the-fly GEMV.  CTA = 256 rows x GEMV_COLS columns; each thread walks
-// its row across the column chunk with four interleaved LCG chains
-// (state jumps by n per column) and two FP64 accumulators.  Partial sums
-// go to the workspace and a second kernel folds them in a fixed order, so
-// the result does not depend on scheduling.
+// On-the-fly GEMV.  CTA = 512/SPLIT rows x GEMV_COLS columns; the columns of
+// a chunk are divided into SPLIT pieces, and each thread walks two rows (32
+// apart) across one piece with two interleaved LCG chains and two FP64
+// accumulators a row.  The pieces are folded in shared memory and the chunks
+// by a second kernel, both in a fixed order, so the result does not depend on
+// scheduling.
+//
+// Bound by the integer multiplies of the LCG (three of a 64-bit product, one
+// of them wide) together with the FP64 multiply-add, which issue to the same
+// port; hence two rows per thread, which share the reads of x, and the
+// hardware's 64-bit integer conversion, which has a pipe of its own (the
+// conversion through the mantissas of 2^84 and 2^52 costs two FP64 additions
+// and was 25 % slower here).
 // ---------------------------------------------------------------------------
+constexpr int GEMV_THREADS = 256;
 constexpr int GEMV_ROWS = 256;
 constexpr int GEMV_COLS = 2048;
 
 // TRANS: y = A^T x, output i walks column i of A (element (j, i) is state
-// j + n*i, so the chain steps by 1 instead of n).
-template <bool TRANS>
-__global__ void __launch_bounds__(GEMV_ROWS) otf_partial_kernel(int64_t n, int mb, int nb, double alpha,
+// j + n*i, so the chain steps by 1 instead of n).  jn: the jump by n.
+template <bool TRANS, int SPLIT>
+__global__ void __launch_bounds__(GEMV_THREADS) otf_partial_kernel(int64_t n, int mb, int nb, double alpha,
 	const double *__restrict__ x, uint64_t state00, int with_diag, const double *__restrict__ diag,
-	double *__restrict__ part, JumpTable64 tab)
+	double *__restrict__ part, JumpTable64 tab, Coeff jn)
 {
+	constexpr int W = GEMV_THREADS / SPLIT / 32;   // warps that share a piece, 64 rows each
+	constexpr int R = 64 * W;
+	static_assert(W >= 1, "a warp's threads share one piece");
 	__shared__ __align__(16) double xs[GEMV_COLS];
+	__shared__ Coeff stab[64];
+	__shared__ double fold[SPLIT > 1 ? SPLIT * R : 1];
+	const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
 	const int j0 = blockIdx.y * GEMV_COLS;
 	const int j1 = min(j0 + GEMV_COLS, nb);
-	for (int j = threadIdx.x; j < j1 - j0; j += GEMV_ROWS) xs[j] = x[j0 + j];
+	for (int j = t; j < j1 - j0; j += GEMV_THREADS) xs[j] = x[j0 + j];
+	if (t < 64) stab[t] = tab.p[t];
 	__syncthreads();
-	const int i = blockIdx.x * GEMV_ROWS + threadIdx.x;
-	if (i >= mb) return;
-	const Coeff jn = jump_of(tab, TRANS ? 1ULL : static_cast<uint64_t>(n));
-	const Coeff jn4 = coeff_mul(coeff_mul(jn, jn), coeff_mul(jn, jn));
-	const uint64_t idx0 = TRANS ? static_cast<uint64_t>(j0) + static_cast<uint64_t>(n) * static_cast<uint64_t>(i)
-	                            : static_cast<uint64_t>(i) + static_cast<uint64_t>(n) * j0;
-	uint64_t s0 = coeff_apply(jump_of(tab, idx0), state00);
-	uint64_t s1 = coeff_apply(jn, s0);
-	uint64_t s2 = coeff_apply(jn, s1);
-	uint64_t s3 = coeff_apply(jn, s2);
-	double a0 = 0.0, a1 = 0.0;
-	const int len = j1 - j0;
-	const int dj = (with_diag && i >= j0 && i < j1) ? i - j0 : -1;   // diagonal column inside the chunk
-	int j = 0;
-	if (dj < 0) {
-		// no diagonal in this chunk (every CTA but those on the diagonal):
-		// the same sums without the per-group test, x read two at a time
-		for (; j + 3 < len; j += 4) {
-			const double2 x01 = *reinterpret_cast<const double2 *>(&xs[j]);
-			const double2 x23 = *reinterpret_cast<const double2 *>(&xs[j + 2]);
-			a0 = fma(__ll2double_rn(static_cast<long long>(s0)), x01.x, a0);
-			a1 = fma(__ll2double_rn(static_cast<long long>(s1)), x01.y, a1);
-			a0 = fma(__ll2double_rn(static_cast<long long>(s2)), x23.x, a0);
-			a1 = fma(__ll2double_rn(static_cast<long long>(s3)), x23.y, a1);
-			s0 = coeff_apply(jn4, s0);
-			s1 = coeff_apply(jn4, s1);
-			s2 = coeff_apply(jn4, s2);
-			s3 = coeff_apply(jn4, s3);
+	const int piece = warp / W, row = (warp % W) * 64 + lane;   // and row + 32
+	const int iw = blockIdx.x * R + (warp % W) * 64;            // the warp's first row
+	const int width = ((j1 - j0 + SPLIT - 1) / SPLIT + 3) & ~3;
+	const int p0 = min(piece * width, j1 - j0), p1 = min(p0 + width, j1 - j0);
+	double r[2] = {0.0, 0.0};
+	// whole warps past the last row or without columns have nothing to do
+	if (iw < mb && p0 < p1) {
+		const uint64_t iu = static_cast<uint64_t>(iw), ju = static_cast<uint64_t>(j0 + p0);
+		uint64_t s[2][2];   // [row][column parity]
+		s[0][0] = coeff_apply(warp_jump(stab, TRANS ? ju + static_cast<uint64_t>(n) * iu
+		                                              : iu + static_cast<uint64_t>(n) * ju), state00);
+		Coeff lp = TRANS ? jn : stab[0];
+#pragma unroll
+		for (int b = 0; b < 5; ++b) {
+			if ((lane >> b) & 1) s[0][0] = coeff_apply(lp, s[0][0]);
+			lp = coeff_mul(lp, lp);
 		}
-	} else {
-		for (; j + 3 < len; j += 4) {
-			double v0 = __ll2double_rn(static_cast<long long>(s0));
-			double v1 = __ll2double_rn(static_cast<long long>(s1));
-			double v2 = __ll2double_rn(static_cast<long long>(s2));
-			double v3 = __ll2double_rn(static_cast<long long>(s3));
-			if (dj >= j && dj < j + 4) {
-				if (dj == j) v0 = 0.0;
-				if (dj == j + 1) v1 = 0.0;
-				if (dj == j + 2) v2 = 0.0;
-				if (dj == j + 3) v3 = 0.0;
+		const Coeff jc = TRANS ? stab[0] : jn;
+		const Coeff jc2 = coeff_mul(jc, jc);
+		s[1][0] = coeff_apply(lp, s[0][0]);   // 32 rows on
+		s[0][1] = coeff_apply(jc, s[0][0]);
+		s[1][1] = coeff_apply(jc, s[1][0]);
+		auto val = [](uint64_t v) { return __ll2double_rn(static_cast<long long>(v)); };
+		double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+		const int len = p1 - p0;
+		const double *xp = xs + p0;
+		// diagonal columns in the piece
+		const int dj0 = with_diag ? iw + lane - j0 - p0 : -1, dj1 = with_diag ? dj0 + 32 : -1;
+		int j = 0;
+		if (!__any_sync(0xffffffffu, (dj0 >= 0 && dj0 < len) || (dj1 >= 0 && dj1 < len))) {
+			// no diagonal in this piece for any row of the warp
+#pragma unroll 2
+			for (; j + 1 < len; j += 2) {
+				const double2 x01 = *reinterpret_cast<const double2 *>(&xp[j]);
+#pragma unroll
+				for (int q = 0; q < 2; ++q) {
+					acc[q][0] = fma(val(s[q][0]), x01.x, acc[q][0]);
+					acc[q][1] = fma(val(s[q][1]), x01.y, acc[q][1]);
+					s[q][0] = coeff_apply(jc2, s[q][0]);
+					s[q][1] = coeff_apply(jc2, s[q][1]);
+				}
 			}
-			a0 = fma(v0, xs[j], a0);
-			a1 = fma(v1, xs[j + 1], a1);
-			a0 = fma(v2, xs[j + 2], a0);
-			a1 = fma(v3, xs[j + 3], a1);
-			s0 = coeff_apply(jn4, s0);
-			s1 = coeff_apply(jn4, s1);
-			s2 = coeff_apply(jn4, s2);
-			s3 = coeff_apply(jn4, s3);
+		} else {
+			for (; j + 1 < len; j += 2) {
+				const double2 x01 = *reinterpret_cast<const double2 *>(&xp[j]);
+#pragma unroll
+				for (int q = 0; q < 2; ++q) {
+					const int dj = q ? dj1 : dj0;
+					const double v0 = j == dj ? 0.0 : val(s[q][0]), v1 = j + 1 == dj ? 0.0 : val(s[q][1]);
+					acc[q][0] = fma(v0, x01.x, acc[q][0]);
+					acc[q][1] = fma(v1, x01.y, acc[q][1]);
+					s[q][0] = coeff_apply(jc2, s[q][0]);
+					s[q][1] = coeff_apply(jc2, s[q][1]);
+				}
+			}
+		}
+		if (j < len) {
+#pragma unroll
+			for (int q = 0; q < 2; ++q) {
+				const double v = j == (q ? dj1 : dj0) ? 0.0 : val(s[q][0]);
+				acc[q][0] = fma(v, xp[j], acc[q][0]);
+			}
+		}
+#pragma unroll
+		for (int q = 0; q < 2; ++q) {
+			const int dj = q ? dj1 : dj0, i = iw + lane + 32 * q;
+			r[q] = (acc[q][0] + acc[q][1]) * (alpha * kValueScale);
+			if (dj >= 0 && dj < len && i < mb) r[q] = fma(alpha * diag[i], xp[dj], r[q]);
 		}
 	}
-	for (; j < len; ++j) {
-		const double v = (j == dj) ? 0.0 : __ll2double_rn(static_cast<long long>(s0));
-		a0 = fma(v, xs[j], a0);
-		s0 = coeff_apply(jn, s0);
+	if (SPLIT == 1) {
+#pragma unroll
+		for (int q = 0; q < 2; ++q)
+			if (iw + lane + 32 * q < mb) part[static_cast<int64_t>(blockIdx.y) * mb + iw + lane + 32 * q] = r[q];
+		return;
 	}
-	double r = (a0 + a1) * (alpha * kValueScale);
-	if (dj >= 0) r = fma(alpha * diag[i], xs[dj], r);
-	part[static_cast<int64_t>(blockIdx.y) * mb + i] = r;
+	fold[piece * R + row] = r[0];
+	fold[piece * R + row + 32] = r[1];
+	__syncthreads();
+	for (int e = t; e < R; e += GEMV_THREADS) {
+		double v = fold[e];
+#pragma unroll
+		for (int q = 1; q < SPLIT; ++q) v += fold[q * R + e];
+		const int i = blockIdx.x * R + e;
+		if (i < mb) part[static_cast<int64_t>(blockIdx.y) * mb + i] = v;
+	}
 }
 
 __global__ void otf_reduce_kernel(int mb, int nchunks, double beta, const double *__restrict__ part, double *y,
@@ -148,13 +184,26 @@ int otf_launch(int64_t n, int mb, int nb, double alpha, const double *x, double 
 	if (work_bytes < static_cast<size_t>(nchunks) * mb * sizeof(double)) return HPLAI_EINVAL;
 	double *part = static_cast<double *>(work);
 	if (nb > 0) {
-		dim3 grid((mb + GEMV_ROWS - 1) / GEMV_ROWS, nchunks);
-		if (trans)
-			otf_partial_kernel<true><<<grid, GEMV_ROWS, 0, st>>>(n, mb, nb, alpha, x, state00, with_diag, diag, part,
-				table());
+		const Coeff jn = coeff_pow(static_cast<uint64_t>(n));
+		auto launch = [&](auto split) {
+			constexpr int S = decltype(split)::value, R = 2 * GEMV_THREADS / S;
+			const dim3 grid((mb + R - 1) / R, nchunks);
+			if (trans)
+				otf_partial_kernel<true, S><<<grid, GEMV_THREADS, 0, st>>>(n, mb, nb, alpha, x, state00, with_diag, diag,
+					part, table(), jn);
+			else
+				otf_partial_kernel<false, S><<<grid, GEMV_THREADS, 0, st>>>(n, mb, nb, alpha, x, state00, with_diag, diag,
+					part, table(), jn);
+		};
+		// Short pieces spread a small order over the SMs (n = 1200: 30 us in one
+		// piece, 13 in eight) and balance the last wave of a large one (32768: 434
+		// in two, 425 in eight).  For A^T, whose set-up is longer (the lanes' jumps
+		// are by n), two pieces are faster once there is work enough (32768: 442
+		// against 483; 16384: 137 against 129).
+		if (trans && static_cast<int64_t>((mb + 255) / 256) * nchunks >= 888)
+			launch(std::integral_constant<int, 2>{});
 		else
-			otf_partial_kernel<false><<<grid, GEMV_ROWS, 0, st>>>(n, mb, nb, alpha, x, state00, with_diag, diag, part,
-				table());
+			launch(std::integral_constant<int, 8>{});
 		count_launches();
 		HPLAI_CUDA_TRY(cudaGetLastError());
 	}
