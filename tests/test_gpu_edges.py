@@ -1,0 +1,62 @@
+"""The tiled kernels at the edges of their tiles, splits and dispatch rules, against the CPU oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _put(torch, m, lda, off):
+    """Column-major m at element `off` of a device buffer with leading dimension lda."""
+    r, c = m.shape
+    buf = np.zeros(c * lda + off + 4, dtype=m.dtype)
+    buf[off:off + c * lda].reshape(c, lda)[:, :r] = m.T
+    t = torch.from_numpy(buf).cuda()
+    return t, t.data_ptr() + off * m.dtype.itemsize
+
+
+def _take(t, r, c, lda, off):
+    return t.cpu().numpy()[off:off + c * lda].reshape(c, lda)[:, :r].T
+
+
+def _dominant(rng, n):
+    m = rng.uniform(-0.5, 0.5, (n, n)).astype(np.float32)
+    m[np.arange(n), np.arange(n)] = np.abs(m).sum(1) + 1
+    return np.asfortranarray(m)
+
+
+def _same_bits(a, b):
+    return np.array_equal(np.ascontiguousarray(a).view(np.uint32), np.ascontiguousarray(b).view(np.uint32))
+
+
+@pytest.mark.parametrize("n,i0,j0,nr,nc,lda,off", [(1000, 3, 5, 1, 1, 1, 0), (1000, 0, 100, 127, 33, 127, 0),
+                                                   (4000, 1, 7, 1023, 31, 1024, 0), (4000, 9, 0, 1025, 65, 1025, 0),
+                                                   (4000, 0, 2000, 2050, 40, 2052, 1)])
+def test_fill_edges(hplai, oracle, torch_cuda, n, i0, j0, nr, nc, lda, off):
+    t, p = _put(torch_cuda, np.zeros((nr, nc), dtype=np.float32), lda, off)
+    hplai.check(hplai.fill_panel(n, i0, j0, nr, nc, p, lda, 42, 0, None))
+    assert _same_bits(_take(t, nr, nc, lda, off), oracle.fill_panel(n, i0, j0, nr, nc, calc_diag=False))
+
+
+@pytest.mark.parametrize("n,i0,count", [(1, 0, 1), (5, 0, 5), (37, 3, 30), (1000, 31, 400), (1001, 970, 31)])
+def test_diag_edges(hplai, oracle, torch_cuda, n, i0, count):
+    torch = torch_cuda
+    d = torch.empty(count, dtype=torch.float64, device="cuda")
+    hplai.check(hplai.gen_diag(n, 42, i0, count, d.data_ptr(), None))
+    assert np.array_equal(d.cpu().numpy(), np.array([oracle.calc_diag(i, n, 42) for i in range(i0, i0 + count)]))
+
+
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 127, 300, 2047, 2049, 4100])
+def test_gemv_edges(hplai, oracle, torch_cuda, n):
+    """Rows around a warp's 64 and a CTA's, columns around a chunk's 2048 and its pieces: 1e-14 of ||A|| ||x||."""
+    torch = torch_cuda
+    rng = np.random.default_rng(n)
+    a = oracle.dense_matrix_f64(n)
+    x, y0 = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    xd, dd = torch.from_numpy(x).cuda(), torch.from_numpy(np.ascontiguousarray(np.diag(a))).cuda()
+    ws = hplai.otf_gemv_workspace(n)
+    w = torch.empty(ws, dtype=torch.uint8, device="cuda")
+    for beta in (0.0, 1.0):
+        yd = torch.from_numpy(y0).cuda()
+        hplai.check(hplai.otf_gemv(n, -1.0, xd.data_ptr(), beta, yd.data_ptr(), 42, dd.data_ptr(), w.data_ptr(), ws, None))
+        ref = beta * y0 - a @ x
+        assert np.abs(yd.cpu().numpy() - ref).max() <= 1e-14 * (np.abs(a).sum(1).max() + 1)
