@@ -420,13 +420,13 @@ extern "C" int hplai_create(hplai_ctx **out, int n, int b, int precision, unsign
 	CTX_ALLOC(c->gemv_work, c->gemv_bytes);
 	c->trsv_bytes = trsv_workspace(n);
 	CTX_ALLOC(c->trsv_work, c->trsv_bytes);
-	CTX_ALLOC(c->getrf_work, getrf_workspace());
+	CTX_ALLOC(c->getrf_work, getrf_workspace(b));
 	CTX_ALLOC(c->check_work, panel_check_workspace(n) + 3 * sizeof(double));
 	CTX_ALLOC(c->dinv, sizeof(double) * trsv_dinv_doubles(n));
 	CTX_ALLOC(c->kstatus, 2 * sizeof(unsigned));
 	CTX_ALLOC(c->f16s, 4 * sizeof(unsigned));
 	if (cudaMemset(c->trsv_work, 0, c->trsv_bytes) != cudaSuccess ||
-		cudaMemset(c->getrf_work, 0, getrf_workspace()) != cudaSuccess ||
+		cudaMemset(c->getrf_work, 0, getrf_workspace(b)) != cudaSuccess ||
 		cudaMemset(c->kstatus, 0, 2 * sizeof(unsigned)) != cudaSuccess ||
 		cudaMemset(c->tcbuf, 0, sizeof(float) * tc_elems) != cudaSuccess) {
 		ctx_free(c);

@@ -7,22 +7,30 @@
 //   step r = ti = tj:      X <- LU of X                        (tile factor)
 //   step r = tj < ti:      X <- X U(r, r)^{-1}                 (L tile)
 //   step r = ti < tj:      X <- L(r, r)^{-1} X  (unit lower)   (U tile)
-// Each tile publishes a progress word, epoch * 64 + (steps applied), where a
-// tile with min(ti, tj) = r is final at r + 1; consumers wait for the value
-// they need.
+// A tile that another CTA needs travels through the workspace as tagged words
+// (64 bits: an element and the launch's number with the tile's state, handed
+// over or final), so that one load carries data and flag: no fence on the
+// producer's side, no second round trip on the consumer's.
 //
-// The diagonal is the critical chain, so one CTA (CTA 0) does nothing
-// else: at step r it takes L(r+1, r) and U(r, r+1) once their owners have
-// applied their first r updates, solves them with the factored tile (r, r)
-// it still holds (four warps each, a step per named barrier), publishes
-// them, applies the last update to tile (r+1, r+1) and factors it (all
-// eight warps).  There is no flag hop between two diagonal tiles, and its
-// code stays hot in its SM's instruction cache.  Worker warps (the other
-// CTAs) own every other tile and walk them step by step, panel tiles before
-// updates.  Every wait is on work the producer reaches
-// without waiting on the waiter, so the dataflow always completes (all
-// warps are resident: cooperative launch); every wait is bounded, and a
-// timeout sets the status word and the warp stops.
+// What bounds it is the diagonal chain, b dependent pivots.  CTA 0 does nothing
+// else, and the teams of the other CTAs own every tile that it does not need
+// next.  At step r CTA 0 holds the factored tile (r, r), solves L(r+1, r) and
+// U(r, r+1) (a team each) while its third team publishes (r, r), updates tile
+// (r+1, r+1) and factors it, while the other two publish L(r+1, r) and
+// U(r, r+1) and bring in the next step's inputs.  The chain through the
+// workers -- (r, r) published, L(r+2, r) solved, tile (r+2, r+1) updated and
+// handed back for step r+1 -- is kept to two hops through L2: one team owns
+// both (e, e-2) and (e, e-1), and tile (e, e) comes back one update early, the
+// last two being applied by CTA 0.  A worker team keeps its tiles in shared
+// memory where they fit, so a trailing update reads only its two operands and
+// writes nothing until the tile is final or handed over.
+// One block alone, before (a tile per warp, the chain on one eight-warp CTA,
+// progress words behind fences) / now: b = 60 26 / 15 us, 240 120 / 54, 512
+// 277 / 107, 1024 522 / 235.
+// Every wait is on work the producer reaches without waiting on the waiter,
+// so the dataflow always completes (all CTAs are resident: cooperative
+// launch); every wait is bounded, and a timeout sets the status word and the
+// team stops.
 //
 // Each element receives a_ij <- fmaf(-l_ik, u_kj, a_ij) in increasing k,
 // multipliers are a_ik * (1/u_kk) and the U tiles use the same unit-lower
@@ -31,6 +39,7 @@
 // unblocked kernel with any blocking (getrf_nopiv.hpp:33-44).
 #include "common.cuh"
 #include "internal.h"
+#include "tile.cuh"
 
 #include <mutex>
 
@@ -38,472 +47,326 @@ namespace hplai {
 
 namespace {
 
-constexpr int T = 32;
-constexpr int kWarps = 8;       // worker warps per CTA
+using namespace tile;
+
+constexpr int kTeams = 3;       // teams per CTA
+constexpr int kThreads = kTeams * kTeam;
 constexpr int kMaxTiles = 32;   // b <= 1024
 
-// One progress word per 128-byte line, so that polling warps and publishing
-// warps do not queue on a few L2 lines.
-constexpr int kFlagStride = 32;
+constexpr int kPairs = T * T / 2;   // two tagged elements are 16 bytes
 
-struct GetrfWork {
+struct alignas(128) GetrfWork {
 	uint32_t status;
 	uint32_t pad[31];
-	uint32_t prog[kMaxTiles * kMaxTiles * kFlagStride];
+	ulonglong2 tiles[kMaxTiles * kMaxTiles][kPairs];
 };
 
-// Wait until *f >= target (values of earlier launches are below every target
-// of this one).  Lane 0 reads the word; the whole warp stays in the loop
-// and learns the outcome through a shuffle, so the warp never diverges
-// around a wait (a warp left split after a long divergent spin runs the
-// following shuffles many times slower).
-__device__ __forceinline__ bool wait_prog(const uint32_t *f, uint32_t target)
+// Tags of one launch (epochs count from 1, so none equals the zeroed workspace's).
+constexpr uint32_t kHanded = 1, kFinal = 2;
+
+__device__ __forceinline__ void put_tile(const float *t, ulonglong2 *g, uint32_t tag, int tid)
 {
-	const bool lead = (threadIdx.x & 31) == 0;
+	const uint64_t hi = static_cast<uint64_t>(tag) << 32;
+#pragma unroll
+	for (int q = 0; q < kPairs / kTeam; ++q) {
+		const int e = tid + kTeam * q, j = e >> 4, i = (e & 15) * 2;
+		const float2 f = *reinterpret_cast<const float2 *>(t + j * kLd + i);
+		asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(g + e), "l"(hi | __float_as_uint(f.x)),
+			"l"(hi | __float_as_uint(f.y)) : "memory");
+	}
+}
+
+// One or two tiles (N words a thread) by one team, each thread until its own
+// words are there; false on a timeout.  The caller's team barrier follows.
+constexpr int kWords = kPairs / kTeam;
+
+template <int N>
+__device__ __forceinline__ bool get_words(const ulonglong2 *const (&g)[N], uint32_t tag, int tid, ulonglong2 (&v)[N][kWords])
+{
+	auto load = [](const ulonglong2 *p) {
+		ulonglong2 w;
+		asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w.x), "=l"(w.y) : "l"(p) : "memory");
+		return w;
+	};
+	auto ready = [tag](ulonglong2 w) {
+		return static_cast<uint32_t>(w.x >> 32) == tag && static_cast<uint32_t>(w.y >> 32) == tag;
+	};
+#pragma unroll
+	for (int n = 0; n < N; ++n)
+#pragma unroll
+		for (int q = 0; q < kWords; ++q) v[n][q] = load(g[n] + tid + kTeam * q);
 	uint64_t t0 = 0;
 	for (int it = 0;; ++it) {
-		int ready = lead ? (ld_acquire_u32(f) >= target) : 0;
-		ready = __shfl_sync(0xffffffffu, ready, 0);
-		if (ready) return true;
-		if (it == 0) t0 = global_ns();
-		else if (global_ns() - t0 > kWaitLimitNs) return false;
-		__nanosleep(32);
-	}
-}
-
-__device__ __forceinline__ void publish(uint32_t *f, uint32_t v)
-{
-	__syncwarp();
-	if ((threadIdx.x & 31) == 0) {
-		__threadfence();
-		st_release_u32(f, v);
-	}
-}
-
-// A staged tile: column-major, element (i, j) at t[j * kLd + i]; rows of 16
-// bytes so that cp.async can fill it.  Lane i works on row i (conflict-free
-// along a column); all lanes reading one element is a broadcast.
-constexpr int kLd = 36;
-constexpr int kTileFloats = T * kLd;
-
-// Tile (rows r0.., cols c0..) -> t, rows >= rv and columns >= cv zero.
-// vec: a, lda and r0 allow 16-byte copies (cp.async.cg, L2 only); otherwise
-// 4-byte loads through L2.  The caller waits with stage_wait().
-__device__ __forceinline__ void stage_tile(float *t, const float *a, int64_t lda, int r0, int c0, int rv, int cv,
-	bool vec, int lane)
-{
-	if (vec) {
-#pragma unroll 1
-		for (int q = 0; q < 8; ++q) {
-			const int e = lane + 32 * q, j = e >> 3, g = (e & 7) * 4;
-			int bytes = (j < cv) ? (rv - g) * 4 : 0;
-			bytes = bytes < 0 ? 0 : (bytes > 16 ? 16 : bytes);
-			const float *src = a + static_cast<int64_t>(c0 + (j < cv ? j : 0)) * lda + r0 + (bytes ? g : 0);
-			asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(t + j * kLd + g)), "l"(src),
-				"r"(bytes) : "memory");
-		}
-		asm volatile("cp.async.commit_group;" ::: "memory");
-	} else {
-#pragma unroll 4
-		for (int j = 0; j < T; ++j)
-			t[j * kLd + lane] = (lane < rv && j < cv) ? __ldcg(&a[static_cast<int64_t>(c0 + j) * lda + r0 + lane]) : 0.f;
-	}
-}
-
-__device__ __forceinline__ void stage_wait()
-{
-	asm volatile("cp.async.wait_all;" ::: "memory");
-	__syncwarp();
-}
-
-__device__ __forceinline__ void store_tile(const float *t, float *a, int64_t lda, int r0, int c0, int rv, int cv,
-	int lane)
-{
-	if (lane < rv) {
-#pragma unroll 4
-		for (int j = 0; j < cv; ++j) a[static_cast<int64_t>(c0 + j) * lda + r0 + lane] = t[j * kLd + lane];
-	}
-}
-
-// One-warp tile operations on staged tiles (the worker warps').  The solves
-// keep a row (or column) of the tile in registers, fully unrolled so that
-// every register index is static: 496 FMAs and their loads per lane, with no
-// register moves between pivots.
-
-// L tile x <- x U^{-1}, U = upper part of the factored tile d (kv x kv); row `lane`.
-__device__ __noinline__ void op_solve_l(float *x, const float *d, int kv)
-{
-	const int lane = threadIdx.x & 31;
-	float v[T];
+		bool all = true;
 #pragma unroll
-	for (int j = 0; j < T; ++j) v[j] = x[j * kLd + lane];
-	// 1/u_jj, lane j's (the staged tile is zero past kv: those lanes' values go unused)
-	const float inv = 1.0f / d[lane * kLd + lane];
+		for (int n = 0; n < N; ++n)
 #pragma unroll
-	for (int j = 0; j < T; ++j) {
-		if (j < kv) {
-			v[j] *= __shfl_sync(0xffffffffu, inv, j);
-			// U(j, t) at d[t * kLd + j]
+			for (int q = 0; q < kWords; ++q) all = all && ready(v[n][q]);
+		if (__all_sync(0xffffffffu, all)) return true;
+		// the decision to give up is taken by the whole warp at once
+		const uint64_t now = global_ns();
+		if (it == 0) t0 = now;
+		if (__any_sync(0xffffffffu, now - t0 > kWaitLimitNs)) return false;
+		__nanosleep(40);
 #pragma unroll
-			for (int t = j + 1; t < T; ++t) v[t] = fmaf(-v[j], d[t * kLd + j], v[t]);
-		}
-	}
+		for (int n = 0; n < N; ++n) {
+			// a tile's first word stands for it until it arrives
+			if (!ready(v[n][0])) {
+				v[n][0] = load(g[n] + tid);
+			} else {
 #pragma unroll
-	for (int j = 0; j < T; ++j)
-		if (j < kv) x[j * kLd + lane] = v[j];
-	__syncwarp();
-}
-
-// U tile x <- L^{-1} x, L = unit lower part of d (kv x kv); column `lane`.
-__device__ __noinline__ void op_solve_u(float *x, const float *d, int kv)
-{
-	const int lane = threadIdx.x & 31;
-	float v[T];
-	float *col = x + lane * kLd;
-#pragma unroll
-	for (int q = 0; q < T / 4; ++q) {
-		const float4 c = reinterpret_cast<const float4 *>(col)[q];
-		v[4 * q] = c.x;
-		v[4 * q + 1] = c.y;
-		v[4 * q + 2] = c.z;
-		v[4 * q + 3] = c.w;
-	}
-#pragma unroll
-	for (int k = 0; k < T; ++k) {
-		if (k < kv) {
-			// L(i, k) at d[k * kLd + i]
-#pragma unroll
-			for (int i = k + 1; i < T; ++i) v[i] = fmaf(-v[k], d[k * kLd + i], v[i]);
-		}
-	}
-#pragma unroll
-	for (int k = 0; k < T; ++k)
-		if (k < kv) col[k] = v[k];
-	__syncwarp();
-}
-
-// x -= l u (K = T); column `lane` of x in registers: per k, u_kj from the
-// lane's own column of u and column k of l as eight 16-byte broadcasts
-// (columns are 16-byte aligned: kLd * 4 = 144 bytes).
-__device__ __noinline__ void op_update(float *x, const float *l, const float *u)
-{
-	const int lane = threadIdx.x & 31;
-	float v[T];
-	float4 *xc = reinterpret_cast<float4 *>(x + lane * kLd);
-#pragma unroll
-	for (int q = 0; q < T / 4; ++q) {
-		const float4 c = xc[q];
-		v[4 * q] = c.x;
-		v[4 * q + 1] = c.y;
-		v[4 * q + 2] = c.z;
-		v[4 * q + 3] = c.w;
-	}
-	const float4 *uc = reinterpret_cast<const float4 *>(u + lane * kLd);
-#pragma unroll 1
-	for (int k4 = 0; k4 < T / 4; ++k4) {
-		const float4 u4 = uc[k4];
-		const float uk[4] = {u4.x, u4.y, u4.z, u4.w};
-#pragma unroll
-		for (int kk = 0; kk < 4; ++kk) {
-			const float4 *lc = reinterpret_cast<const float4 *>(l + (4 * k4 + kk) * kLd);
-#pragma unroll
-			for (int q = 0; q < T / 4; ++q) {
-				const float4 l4 = lc[q];
-				v[4 * q] = fmaf(-l4.x, uk[kk], v[4 * q]);
-				v[4 * q + 1] = fmaf(-l4.y, uk[kk], v[4 * q + 1]);
-				v[4 * q + 2] = fmaf(-l4.z, uk[kk], v[4 * q + 2]);
-				v[4 * q + 3] = fmaf(-l4.w, uk[kk], v[4 * q + 3]);
+				for (int q = 1; q < kWords; ++q)
+					if (!ready(v[n][q])) v[n][q] = load(g[n] + tid + kTeam * q);
 			}
 		}
 	}
-#pragma unroll
-	for (int q = 0; q < T / 4; ++q) xc[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-	__syncwarp();
 }
 
-constexpr int kDiagWarps = kWarps;
-
-// Barrier and AND-vote of the diagonal CTA's warps (named barrier 1).
-__device__ __forceinline__ void diag_sync()
+__device__ __forceinline__ void keep_words(float *t, const ulonglong2 (&v)[kWords], bool transposed, int tid)
 {
-	asm volatile("bar.sync 1, %0;" ::"n"(kDiagWarps * 32) : "memory");
-}
-
-__device__ __forceinline__ bool diag_all(bool p)
-{
-	int r;
-	asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.and.pred q, 1, %2, p;\n\t"
-	             "selp.s32 %0, 1, 0, q;\n\t}"
-	             : "=r"(r) : "r"(p ? 1 : 0), "n"(kDiagWarps * 32) : "memory");
-	return r != 0;
-}
-
-// Columns c0 .. c0 + T/kDiagWarps - 1 of x -= l u (K = T); row `lane`.
-__device__ __noinline__ void op_update_cols(float *x, const float *l, const float *u, int c0)
-{
-	constexpr int C = T / kDiagWarps;
-	const int lane = threadIdx.x & 31;
-	float v[C];
 #pragma unroll
-	for (int j = 0; j < C; ++j) v[j] = x[(c0 + j) * kLd + lane];
-#pragma unroll 4
-	for (int k = 0; k < T; ++k) {
-		const float lk = l[k * kLd + lane];
-#pragma unroll
-		for (int j = 0; j < C; ++j) v[j] = fmaf(-lk, u[(c0 + j) * kLd + k], v[j]);
-	}
-#pragma unroll
-	for (int j = 0; j < C; ++j) x[(c0 + j) * kLd + lane] = v[j];
-}
-
-// The diagonal CTA's tile operations over several warps: warp w of a group
-// owns C = T / (warps in the group) columns (rows for the U solve), lane =
-// row (column); the value each step broadcasts (a multiplier column or a
-// solved row) goes through shared memory, double-buffered, one named
-// barrier per step.  Every element receives the same operations in the same
-// order as in an unblocked one-warp factorisation and in the workers'
-// op_solve_l / op_solve_u.
-__device__ __forceinline__ void group_sync(int id, int threads)
-{
-	asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
-// Unblocked LU of the kv x kv tile x, all kDiagWarps warps (barrier 1).
-__device__ __noinline__ void coop_factor(float *x, int kv, float *mbuf, int warp)
-{
-	constexpr int C = T / kDiagWarps;
-	const int lane = threadIdx.x & 31, c0 = warp * C;
-	float v[C];
-#pragma unroll
-	for (int c = 0; c < C; ++c) v[c] = x[(c0 + c) * kLd + lane];
-#pragma unroll 1
-	for (int k = 0; k < kv; ++k) {
-		float *m = mbuf + (k & 1) * T;
-		const bool own = k >= c0 && k < c0 + C;
-		float lreg = 0.f;
-#pragma unroll
-		for (int c = 0; c < C; ++c)
-			if (k == c0 + c) {
-				const float inv = 1.0f / __shfl_sync(0xffffffffu, v[c], k);
-				const float lik = v[c] * inv;
-				if (lane > k) v[c] = lik;
-				m[lane] = lik;
-				lreg = lik;
-			}
-		group_sync(1, kDiagWarps * 32);
-		const float l = own ? lreg : m[lane];
-#pragma unroll
-		for (int c = 0; c < C; ++c) {
-			const float ukj = __shfl_sync(0xffffffffu, v[c], k);
-			if (lane > k && c0 + c > k) v[c] = fmaf(-l, ukj, v[c]);
+	for (int q = 0; q < kWords; ++q) {
+		const int e = tid + kTeam * q, j = e >> 4, i = (e & 15) * 2;
+		const float x = __uint_as_float(static_cast<uint32_t>(v[q].x)), y = __uint_as_float(static_cast<uint32_t>(v[q].y));
+		if (transposed) {
+			t[i * kLd + j] = x;
+			t[(i + 1) * kLd + j] = y;
+		} else {
+			*reinterpret_cast<float2 *>(t + j * kLd + i) = make_float2(x, y);
 		}
 	}
-#pragma unroll
-	for (int c = 0; c < C; ++c) x[(c0 + c) * kLd + lane] = v[c];
 }
 
-// L tile x <- x U^{-1} (T columns), warps w = 0 .. kSolveWarps - 1 of the
-// group on barrier `bar`; row `lane`.
-constexpr int kSolveWarps = kDiagWarps / 2;
-__device__ __noinline__ void coop_solve_l(float *x, const float *d, float *mbuf, int w, int bar)
+__device__ __forceinline__ bool get_tile(float *t, const ulonglong2 *g, uint32_t tag, int tid, bool transposed = false)
 {
-	constexpr int C = T / kSolveWarps;
-	const int lane = threadIdx.x & 31, c0 = w * C;
-	float v[C];
-#pragma unroll
-	for (int c = 0; c < C; ++c) v[c] = x[(c0 + c) * kLd + lane];
-	const float inv = 1.0f / d[lane * kLd + lane];   // lane j: 1/u_jj
-#pragma unroll 1
-	for (int j = 0; j < T; ++j) {
-		float *m = mbuf + (j & 1) * T;
-		const bool own = j >= c0 && j < c0 + C;
-		const float invj = __shfl_sync(0xffffffffu, inv, j);
-		float xreg = 0.f;
-#pragma unroll
-		for (int c = 0; c < C; ++c)
-			if (j == c0 + c) {
-				v[c] *= invj;
-				m[lane] = v[c];
-				xreg = v[c];
-			}
-		group_sync(bar, kSolveWarps * 32);
-		const float xij = own ? xreg : m[lane];
-#pragma unroll
-		for (int c = 0; c < C; ++c)
-			if (c0 + c > j) v[c] = fmaf(-xij, d[(c0 + c) * kLd + j], v[c]);
-	}
-#pragma unroll
-	for (int c = 0; c < C; ++c) x[(c0 + c) * kLd + lane] = v[c];
+	ulonglong2 v[1][kWords];
+	const ulonglong2 *const src[1] = {g};
+	const bool ok = get_words<1>(src, tag, tid, v);
+	if (ok) keep_words(t, v[0], transposed, tid);
+	return ok;
 }
 
-// U tile x <- L^{-1} x (T rows, L unit lower), warp w of its group owning
-// rows w * C ..; column `lane`.
-__device__ __noinline__ void coop_solve_u(float *x, const float *d, float *mbuf, int w, int bar)
+__device__ __forceinline__ bool get_tiles(float *t0, const ulonglong2 *g0, float *t1, const ulonglong2 *g1, uint32_t tag,
+	int tid)
 {
-	constexpr int C = T / kSolveWarps;
-	const int lane = threadIdx.x & 31, r0 = w * C;
-	float v[C];
-#pragma unroll
-	for (int r = 0; r < C; ++r) v[r] = x[lane * kLd + r0 + r];
-#pragma unroll 1
-	for (int k = 0; k < T; ++k) {
-		float *m = mbuf + (k & 1) * T;
-		const bool own = k >= r0 && k < r0 + C;
-		float xreg = 0.f;
-#pragma unroll
-		for (int r = 0; r < C; ++r)
-			if (k == r0 + r) {
-				m[lane] = v[r];
-				xreg = v[r];
-			}
-		group_sync(bar, kSolveWarps * 32);
-		const float xkj = own ? xreg : m[lane];
-#pragma unroll
-		for (int r = 0; r < C; ++r)
-			if (r0 + r > k) v[r] = fmaf(-xkj, d[k * kLd + r0 + r], v[r]);
+	ulonglong2 v[2][kWords];
+	const ulonglong2 *const src[2] = {g0, g1};
+	const bool ok = get_words<2>(src, tag, tid, v);
+	if (ok) {
+		keep_words(t0, v[0], false, tid);
+		keep_words(t1, v[1], false, tid);
 	}
-#pragma unroll
-	for (int r = 0; r < C; ++r) x[lane * kLd + r0 + r] = v[r];
+	return ok;
 }
 
-__global__ void __launch_bounds__(kWarps * 32) getrf_tiles_kernel(int b, float *a, int64_t lda, GetrfWork *w,
+// AND-vote and barrier of the whole CTA (barrier 0).
+__device__ __forceinline__ bool all_agree(bool p) { return __syncthreads_and(p) != 0; }
+
+// Tiles of a worker team's shared memory: kRes resident ones, two for a tile
+// and its neighbour that have no place there, two for operands.
+constexpr int kRes = 11;
+constexpr int kTeamTiles = kRes + 4;
+
+__global__ void __launch_bounds__(kThreads) getrf_tiles_kernel(int b, float *a, int64_t lda, GetrfWork *w,
 	uint32_t epoch)
 {
 	extern __shared__ __align__(16) float dyn[];
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	float *X = dyn + warp * 4 * kTileFloats;   // this warp's tile
-	float *D = X + kTileFloats;                // the factored diagonal tile it reads
-	float *Lt = X + 2 * kTileFloats;           // an L tile it reads
-	float *Ut = X + 3 * kTileFloats;           // a U tile it reads
+	__shared__ __align__(16) float xchs[kTeams][kXchFloats];
+	const int team = threadIdx.x / kTeam;
+	const Team tm{static_cast<int>(threadIdx.x) % kTeam, static_cast<int>(threadIdx.x) & 31,
+		static_cast<int>(threadIdx.x) % kTeam / 32, 1 + team};
+	float *const xch = xchs[team];
 	const int nt = (b + T - 1) / T, ntiles = nt * nt;
-	const uint32_t base = epoch * 64u;
-	uint32_t *prog = w->prog;
-	auto pidx = [nt](int ti, int tj) { return (ti + nt * tj) * kFlagStride; };
+	const uint32_t handed = epoch * 4u + kHanded, final_tag = epoch * 4u + kFinal;
+	auto slot_of = [w, nt](int ti, int tj) { return w->tiles[ti + nt * tj]; };
 	const bool vec = ((reinterpret_cast<uintptr_t>(a) & 15u) == 0) && ((lda & 3) == 0);
-	bool ok = true;
 
 	if (blockIdx.x == 0) {
-		// ---------------- the diagonal chain (all kDiagWarps warps) ----------------
-		// warps 0 .. 3 solve L(r+1, r) while warps 4 .. 7 solve U(r, r+1);
-		// all share the update of tile (r+1, r+1) and its factorisation.
-		// Their tiles are warp 0's four staging buffers; the broadcast rows
-		// sit in warp 1's.
-		float *Dd = dyn, *Xd = dyn + kTileFloats, *Ld = dyn + 2 * kTileFloats, *Ud = dyn + 3 * kTileFloats;
-		float *mF = dyn + 4 * kTileFloats, *mL = mF + 2 * T, *mU = mL + 2 * T;
-		const bool lgroup = warp < kSolveWarps;
-		{
-			const int kv = min(T, b);
-			if (warp == 0) stage_tile(Dd, a, lda, 0, 0, kv, kv, vec, lane);
+		// ---------------- the diagonal chain ----------------
+		float *const tile0 = dyn;
+		auto tile = [tile0](int i) { return tile0 + i * kTileFloats; };
+		float *D = tile(0), *Dt = tile(1);
+		float *const Lb[2] = {tile(2), tile(3)}, *const Ub[2] = {tile(4), tile(5)}, *const Xb[2] = {tile(6), tile(7)};
+		float *L2 = tile(8), *U2 = tile(9);   // L(r+2, r), U(r, r+2): the last update but one of tile (r+2, r+2)
+		const int v0 = min(T, b);
+		if (team == 0) {
+			stage_tile(Xb[0], a, lda, 0, 0, v0, v0, vec, tm.tid, kTeam);
 			stage_wait();
-			diag_sync();
-			coop_factor(Dd, kv, mF, warp);
-			diag_sync();
-			if (warp == 0) {
-				store_tile(Dd, a, lda, 0, 0, kv, kv, lane);
-				publish(&prog[0], base + 1);
+			tm.sync();
+			op_factor(tm, Xb[0], D, Dt, xch, v0);
+		} else if (nt > 1) {
+			// step 0's inputs are the block's own entries
+			const int v1 = min(T, b - T);
+			if (team == 1) {
+				stage_tile(Lb[0], a, lda, T, 0, v1, T, vec, tm.tid, kTeam);
+				stage_tile(Ub[0], a, lda, 0, T, T, v1, vec, tm.tid, kTeam);
+			} else {
+				stage_tile(Xb[1], a, lda, T, T, v1, v1, vec, tm.tid, kTeam);
 			}
+			stage_wait();
 		}
-		diag_sync();
-		for (int r = 0; r + 1 < nt && ok; ++r) {
+		__syncthreads();
+		bool ok = true;
+		for (int r = 0; r + 1 < nt; ++r) {
 			const int k0 = r * T, r1 = k0 + T, v1 = min(T, b - r1);
+			float *Ld = Lb[r & 1], *Ud = Ub[r & 1], *Xd = Xb[(r + 1) & 1];
+			if (team == 0) {
+				op_solve_l(tm, Ld, Dt);
+			} else if (team == 1) {
+				op_solve_u(tm, Ud, D);
+			} else {
+				put_tile(D, slot_of(r, r), final_tag, tm.tid);
+				store_tile(D, a, lda, k0, k0, T, T, tm.tid, kTeam);
+			}
+			__syncthreads();
+			// team 0: the next diagonal tile; meanwhile what is final goes out, and
+			// step r+1's inputs come in: tile (r+2, r+2) with r updates, L(r+2, r)
+			// and U(r, r+2), tiles (r+2, r+1) and (r+1, r+2) with r+1
+			const bool more = r + 2 < nt;
 			bool mine = true;
-			if (r > 0 && warp < 3) {
-				const int f = warp == 0 ? pidx(r + 1, r) : (warp == 1 ? pidx(r, r + 1) : pidx(r + 1, r + 1));
-				mine = wait_prog(&prog[f], base + r);
+			if (team == 0) {
+				op_update(tm, Xd, Ld, Ud);
+				tm.sync();
+				op_factor(tm, Xd, D, Dt, xch, v1);
+			} else if (team == 1) {
+				put_tile(Ld, slot_of(r + 1, r), final_tag, tm.tid);
+				put_tile(Ud, slot_of(r, r + 1), final_tag, tm.tid);
+				store_tile(Ld, a, lda, r1, k0, v1, T, tm.tid, kTeam);
+				store_tile(Ud, a, lda, k0, r1, T, v1, tm.tid, kTeam);
+				if (more)
+					mine = get_tiles(Lb[(r + 1) & 1], slot_of(r + 2, r + 1), Ub[(r + 1) & 1], slot_of(r + 1, r + 2), handed,
+						tm.tid);
+			} else if (more) {
+				const int r2 = r1 + T, v2 = min(T, b - r2);
+				float *const X2 = Xb[r & 1];
+				if (r > 0) {
+					mine = get_tile(X2, slot_of(r + 2, r + 2), handed, tm.tid);
+				} else {
+					stage_tile(X2, a, lda, r2, r2, v2, v2, vec, tm.tid, kTeam);
+					stage_wait();
+				}
+				mine = get_tiles(L2, slot_of(r + 2, r), U2, slot_of(r, r + 2), final_tag, tm.tid) && mine;
+				tm.sync();
+				op_update(tm, X2, L2, U2);   // its last update but one
 			}
-			ok = diag_all(mine);
+			ok = all_agree(mine);
 			if (!ok) break;
-			if (warp == 0) stage_tile(Ld, a, lda, r1, k0, v1, T, vec, lane);   // L(r+1, r) before its solve
-			if (warp == 1) stage_tile(Ud, a, lda, k0, r1, T, v1, vec, lane);   // U(r, r+1) before its solve
-			if (warp == 2) stage_tile(Xd, a, lda, r1, r1, v1, v1, vec, lane);  // tile (r+1, r+1)
-			stage_wait();
-			diag_sync();
-			if (lgroup)
-				coop_solve_l(Ld, Dd, mL, warp, 2);
-			else
-				coop_solve_u(Ud, Dd, mU, warp - kSolveWarps, 3);
-			diag_sync();
-			if (warp == 0)
-				store_tile(Ld, a, lda, r1, k0, v1, T, lane);
-			else if (warp == 1)
-				store_tile(Ud, a, lda, k0, r1, T, v1, lane);
-			__threadfence();
-			diag_sync();
-			if (warp == 0 && lane == 0) {
-				st_release_u32(&prog[pidx(r + 1, r)], base + r + 1);
-				st_release_u32(&prog[pidx(r, r + 1)], base + r + 1);
-			}
-			op_update_cols(Xd, Ld, Ud, warp * (T / kDiagWarps));
-			diag_sync();
-			coop_factor(Xd, v1, mF, warp);
-			diag_sync();
-			if (warp == 0) {
-				store_tile(Xd, a, lda, r1, r1, v1, v1, lane);
-				publish(&prog[pidx(r + 1, r + 1)], base + r + 2);
-			}
-			// the new diagonal tile is the next step's factor
-			for (int e = threadIdx.x; e < kTileFloats; e += kDiagWarps * 32) Dd[e] = Xd[e];
-			diag_sync();
 		}
-		if (!ok && threadIdx.x == 0) atomicOr(&w->status, 1u);
+		if (!ok) {
+			if (threadIdx.x == 0) atomicOr(&w->status, 1u);
+			return;
+		}
+		const int r0 = (nt - 1) * T, v = min(T, b - r0);
+		store_tile(D, a, lda, r0, r0, v, v, threadIdx.x, kThreads);
 		return;
 	}
 
-	// ---------------- worker warps ----------------
-	// worker warp w owns tiles w, w + nwarps, ... (column-major tile index);
-	// warp numbers run across the CTAs first, so that neighbouring tiles sit
-	// on different SMs (b = 1024: 0.57 ms against 0.62 with them on one SM;
-	// ordering each warp's tiles nearest-the-diagonal first was slower)
-	const int wid = warp * (gridDim.x - 1) + (blockIdx.x - 1), nwarps = (gridDim.x - 1) * kWarps;
-	for (int r = 0; r < nt && ok; ++r) {
-		const int k0 = r * T, kv = min(T, b - k0);
-		const uint32_t diag_final = base + r + 1;
-		// pass 0: panel tiles of step r; pass 1: trailing updates
-		for (int pass = 0; pass < 2 && ok; ++pass) {
-			for (int t = wid; t < ntiles && ok; t += nwarps) {
-				const int ti = t % nt, tj = t / nt;
-				const int mn = min(ti, tj);
-				if (mn < r || ti == tj && ti <= r + 1) continue;                     // done, or the diagonal CTA's
-				if ((ti == r + 1 && tj == r) || (ti == r && tj == r + 1)) continue;  // the diagonal CTA's
-				if ((mn == r ? 0 : 1) != pass) continue;
-				const int r0 = ti * T, c0 = tj * T;
-				const int rv = min(T, b - r0), cv = min(T, b - c0);
-				if (pass == 0) {
-					// L tile X <- X U(r,r)^{-1}, or U tile X <- L(r,r)^{-1} X
-					stage_tile(X, a, lda, r0, c0, rv, cv, vec, lane);
-					if (!wait_prog(&prog[pidx(r, r)], diag_final)) { ok = false; break; }
-					stage_tile(D, a, lda, k0, k0, kv, kv, vec, lane);
-					stage_wait();
-					if (tj == r)
-						op_solve_l(X, D, kv);
-					else
-						op_solve_u(X, D, kv);
-					store_tile(X, a, lda, r0, c0, rv, cv, lane);
-					publish(&prog[t * kFlagStride], base + r + 1);
-				} else {
-					// X -= L(ti, r) U(r, tj)
-					if (!wait_prog(&prog[pidx(ti, r)], base + r + 1) || !wait_prog(&prog[pidx(r, tj)], base + r + 1)) {
-						ok = false;
-						break;
-					}
-					stage_tile(X, a, lda, r0, c0, rv, cv, vec, lane);
-					stage_tile(Lt, a, lda, r0, k0, rv, T, vec, lane);
-					stage_tile(Ut, a, lda, k0, c0, T, cv, vec, lane);
-					stage_wait();
-					op_update(X, Lt, Ut);
-					store_tile(X, a, lda, r0, c0, rv, cv, lane);
-					// the next step's panel tiles, and the diagonal tile after next, announce
-					// that they hold r + 1 updates
-					if (mn == r + 1 || (ti == tj && ti == r + 2)) publish(&prog[t * kFlagStride], base + r + 1);
-				}
-				__syncwarp();   // this warp's staging tiles are free again
-			}
+	// ---------------- worker teams ----------------
+	// worker team g owns the tiles g, g + nteams, ... (column-major tile index)
+	// that are two or more off the diagonal, each with its neighbour towards
+	// the diagonal if that is one off it, and the diagonal tiles from (3, 3)
+	// on; team numbers run across the CTAs first, so that neighbouring tiles
+	// sit on different SMs
+	const int gid = team * (gridDim.x - 1) + (blockIdx.x - 1), nteams = (gridDim.x - 1) * kTeams;
+	float *const mem = dyn + team * kTeamTiles * kTileFloats;
+	float *const tmp = mem + kRes * kTileFloats, *const tmp2 = tmp + kTileFloats, *const opL = tmp2 + kTileFloats,
+	            *const opU = opL + kTileFloats;
+	bool ok = true;   // the same in the whole team
+	auto rows_of = [b](int ti) { return min(T, b - ti * T); };
+	// Calls f(ti, tj, slot) for every unit: slot of its first tile among the
+	// resident ones, -1 where they are taken.
+	auto for_units = [&](auto &&f) {
+		int used = 0;
+		for (int t = gid; t < ntiles && ok; t += nteams) {
+			const int ti = t % nt, tj = t / nt, d = ti > tj ? ti - tj : tj - ti;
+			if (d == 1 || (d == 0 && ti < 3)) continue;   // with the unit two off the diagonal, or the diagonal CTA's
+			const int need = d == 2 ? 2 : 1;
+			const int slot = used + need <= kRes ? used : -1;
+			if (slot >= 0) used += need;
+			f(ti, tj, slot);
 		}
+	};
+	auto load = [&](float *t, int ti, int tj) {
+		stage_tile(t, a, lda, ti * T, tj * T, rows_of(ti), rows_of(tj), vec, tm.tid, kTeam);
+	};
+	auto store = [&](const float *t, int ti, int tj) {
+		store_tile(t, a, lda, ti * T, tj * T, rows_of(ti), rows_of(tj), tm.tid, kTeam);
+	};
+	// every warp waits for itself; the barrier that follows makes the outcome the team's
+	auto arrived = [&](bool mine) {
+		int all;
+		asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.and.pred q, %2, %3, p;\n\t"
+		             "selp.s32 %0, 1, 0, q;\n\t}"
+		             : "=r"(all) : "r"(mine ? 1 : 0), "r"(tm.bar), "n"(kTeam) : "memory");
+		ok = all != 0;
+		return ok;
+	};
+	// X(ti, tj) -= L(ti, r) U(r, tj), an operand that the team already holds
+	// given; a resident tile stays where it is unless it is handed over
+	auto update = [&](int ti, int tj, int slot, int r, const float *haveL, const float *haveU, bool hand_over) {
+		float *x = slot >= 0 ? mem + slot * kTileFloats : tmp2;
+		bool mine;
+		if (haveL)
+			mine = get_tile(opU, slot_of(r, tj), final_tag, tm.tid);
+		else if (haveU)
+			mine = get_tile(opL, slot_of(ti, r), final_tag, tm.tid);
+		else
+			mine = get_tiles(opL, slot_of(ti, r), opU, slot_of(r, tj), final_tag, tm.tid);
+		if (slot < 0) load(x, ti, tj);
+		stage_wait();
+		if (!arrived(mine)) return;
+		op_update(tm, x, haveL ? haveL : opL, haveU ? haveU : opU);
+		tm.sync();   // the operand tiles are free again
+		if (hand_over) {
+			put_tile(x, slot_of(ti, tj), handed, tm.tid);
+		} else if (slot < 0) {
+			store(x, ti, tj);
+		}
+		if (slot < 0) tm.sync();
+	};
+	for_units([&](int ti, int tj, int slot) {
+		if (slot < 0) return;
+		load(mem + slot * kTileFloats, ti, tj);
+		if (ti - tj == 2) load(mem + (slot + 1) * kTileFloats, ti, tj + 1);
+		if (tj - ti == 2) load(mem + (slot + 1) * kTileFloats, ti + 1, tj);
+	});
+	stage_wait();
+	tm.sync();
+	for (int r = 0; r < nt && ok; ++r) {
+		// the panel tiles of step r, then the trailing updates
+		for_units([&](int ti, int tj, int slot) {
+			if (ti == tj || min(ti, tj) != r) return;
+			float *x = slot >= 0 ? mem + slot * kTileFloats : tmp;
+			const bool left = tj == r;
+			// L tile X <- X U(r,r)^{-1}, or U tile X <- L(r,r)^{-1} X (tile (r, r) is a whole one)
+			if (slot < 0) load(x, ti, tj);
+			const bool mine = get_tile(opL, slot_of(r, r), final_tag, tm.tid, left);
+			stage_wait();
+			if (!arrived(mine)) return;
+			if (left)
+				op_solve_l(tm, x, opL);
+			else
+				op_solve_u(tm, x, opL);
+			put_tile(x, slot_of(ti, tj), final_tag, tm.tid);
+			// its neighbour's last update, and on to the diagonal CTA
+			const int second = slot >= 0 ? slot + 1 : -1;
+			if (left && ti == r + 2) update(ti, r + 1, second, r, x, nullptr, true);
+			if (!left && tj == r + 2) update(r + 1, tj, second, r, nullptr, x, true);
+			store(x, ti, tj);
+			if (slot < 0) tm.sync();
+		});
+		for_units([&](int ti, int tj, int slot) {
+			if (min(ti, tj) <= r || (ti == tj && ti < r + 3)) return;
+			update(ti, tj, slot, r, nullptr, nullptr, ti == tj && ti == r + 3);
+			const int second = slot >= 0 ? slot + 1 : -1;
+			if (ok && ti - tj == 2) update(ti, tj + 1, second, r, nullptr, nullptr, false);
+			if (ok && tj - ti == 2) update(ti + 1, tj, second, r, nullptr, nullptr, false);
+		});
 	}
-	if (!ok && lane == 0) atomicOr(&w->status, 1u);
+	if (!ok && tm.tid == 0) atomicOr(&w->status, 1u);
 }
 
-constexpr size_t kSmemBytes = static_cast<size_t>(kWarps) * 4 * kTileFloats * sizeof(float);
+constexpr size_t kSmemBytes = static_cast<size_t>(kTeams) * kTeamTiles * kTileFloats * sizeof(float);
 
 std::mutex g_static_mu;
 __device__ GetrfWork g_static_work;
@@ -517,7 +380,7 @@ int max_coresident_ctas()
 		int per_sm = 0, sms = 0;
 		HPLAI_CUDA_TRY(cudaFuncSetAttribute(getrf_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
 			static_cast<int>(kSmemBytes)));
-		HPLAI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, getrf_tiles_kernel, kWarps * 32,
+		HPLAI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, getrf_tiles_kernel, kThreads,
 			kSmemBytes));
 		HPLAI_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
 		*v = per_sm * sms;
@@ -528,27 +391,33 @@ int max_coresident_ctas()
 
 } // namespace
 
-size_t getrf_workspace() { return sizeof(GetrfWork); }
+// a block of order b uses the first nt x nt tiles
+size_t getrf_workspace(int b)
+{
+	const size_t nt = (static_cast<size_t>(b) + T - 1) / T;
+	return offsetof(GetrfWork, tiles) + nt * nt * sizeof(ulonglong2) * kPairs;
+}
 
 int launch_getrf_tiles(int b, float *a, int64_t lda, void *work, uint32_t *epoch, int max_ctas, cudaStream_t st)
 {
 	if (b <= 0) return HPLAI_OK;
 	if (b > T * kMaxTiles || !a || lda < b || !work || !epoch) return HPLAI_EINVAL;
 	const int nt = (b + T - 1) / T;
-	// CTA 0: the diagonal chain; then enough worker CTAs for one tile per warp
-	int grid = 1 + (nt > 1 ? (nt * nt + kWarps - 1) / kWarps : 0);
+	// CTA 0: the diagonal chain; then enough worker CTAs for one tile per team
+	// (two tiles or fewer to a side leave them nothing to do)
+	int grid = 1 + (nt > 2 ? (nt * nt + kTeams - 1) / kTeams : 0);
 	const int cap = max_coresident_ctas();
 	if (cap < 2) return HPLAI_EUNSUPPORTED;
 	if (grid > cap) grid = cap;
 	if (max_ctas > 0 && grid > max_ctas) grid = max_ctas < 2 ? 2 : max_ctas;
-	if (nt > 1 && grid < 2) grid = 2;
+	if (nt > 2 && grid < 2) grid = 2;
 	GetrfWork *w = static_cast<GetrfWork *>(work);
-	// progress words are epoch * 64 + steps (< 64): epochs stay below 2^26
+	// tags are epoch * 4 + state: epochs stay below 2^30
 	uint32_t ep = ++*epoch;
-	if (ep >= (1u << 26)) return HPLAI_EUNSUPPORTED;
+	if (ep >= (1u << 30)) return HPLAI_EUNSUPPORTED;
 	void *args[] = {(void *)&b, (void *)&a, (void *)&lda, (void *)&w, (void *)&ep};
 	HPLAI_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(getrf_tiles_kernel), dim3(grid),
-		dim3(kWarps * 32), args, kSmemBytes, st));
+		dim3(kThreads), args, kSmemBytes, st));
 	count_launches();
 	return HPLAI_OK;
 }

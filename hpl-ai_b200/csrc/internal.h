@@ -47,11 +47,11 @@ int launch_hgemm_deck(int m, int n, int k, const uint16_t *l, int64_t ldl, const
 
 // panel.cu
 // getrf.cu: tile-parallel diagonal block LU (bit-exact with the sequential
-// order).  `work` holds getrf_workspace() bytes, zeroed once; `epoch` is
+// order).  `work` holds getrf_workspace(b) bytes, zeroed once; `epoch` is
 // the host-side launch counter that goes with it.  launch_getrf is the
 // leaf entry point's form on a library-owned workspace (it waits for the
 // result and returns the kernel's status).
-size_t getrf_workspace();
+size_t getrf_workspace(int b);
 int launch_getrf_tiles(int b, float *a, int64_t lda, void *work, uint32_t *epoch, int max_ctas, cudaStream_t st);
 int getrf_status(void *work, cudaStream_t st, int *status);
 int launch_getrf(int b, float *a, int64_t lda, cudaStream_t st);

@@ -28,6 +28,27 @@ def _same_bits(a, b):
     return np.array_equal(np.ascontiguousarray(a).view(np.uint32), np.ascontiguousarray(b).view(np.uint32))
 
 
+# one to four tiles a side and remainders, the widest block, odd leading dimensions and unaligned bases (4-byte copies)
+@pytest.mark.parametrize("b,lda,off", [(1, 1, 0), (31, 32, 0), (33, 36, 0), (64, 64, 0), (65, 65, 0), (97, 100, 1),
+                                       (130, 131, 0), (160, 160, 2), (1023, 1024, 0), (1024, 1028, 0)])
+def test_getrf_tile_edges(hplai, oracle, torch_cuda, b, lda, off):
+    m = _dominant(np.random.default_rng(b), b)
+    t, p = _put(torch_cuda, m, lda, off)
+    hplai.check(hplai.getrf_nopiv(b, p, lda, None))
+    assert _same_bits(_take(t, b, b, lda, off), oracle.getrf_nopiv(m))
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -127, 2.0 ** -140, 2.0 ** 120])
+def test_getrf_pivots_without_normal_reciprocals(hplai, oracle, torch_cuda, scale):
+    """Subnormal pivots, and pivots whose reciprocals are subnormal, take the reciprocal that keeps subnormals."""
+    m = np.asfortranarray((_dominant(np.random.default_rng(7), 100) * np.float32(scale)).astype(np.float32))
+    t, p = _put(torch_cuda, m, 100, 0)
+    hplai.check(hplai.getrf_nopiv(100, p, 100, None))
+    got, ref = _take(t, 100, 100, 100, 0), oracle.getrf_nopiv(m)
+    nan = np.isnan(ref)
+    assert np.array_equal(nan, np.isnan(got)) and _same_bits(np.where(nan, 0, got), np.where(nan, 0, ref))
+
+
 @pytest.mark.parametrize("n,i0,j0,nr,nc,lda,off", [(1000, 3, 5, 1, 1, 1, 0), (1000, 0, 100, 127, 33, 127, 0),
                                                    (4000, 1, 7, 1023, 31, 1024, 0), (4000, 9, 0, 1025, 65, 1025, 0),
                                                    (4000, 0, 2000, 2050, 40, 2052, 1)])
