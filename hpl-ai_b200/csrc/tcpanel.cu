@@ -18,6 +18,7 @@
 // TMA producer, one MMA-issuing thread, four epilogue warps; bounded waits).
 #include "common.cuh"
 #include "internal.h"
+#include "tri_inv.cuh"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -267,12 +268,13 @@ __global__ void __launch_bounds__(256) tri_f16_kernel(int b, const float *__rest
 // and padded with the identity to bp = ldp rows/columns:
 //   TRANS_T = false: T = U11, T[p][j] at lu[j*lda + p], non-unit diagonal
 //   TRANS_T = true : T = L11^T, T[p][j] = L[j][p] at lu[p*lda + j], unit diagonal
-// Level 0 inverts the 32 x 32 diagonal tiles (one warp each, back
-// substitution).  Level l joins pairs of inverted blocks of h = 32 * 2^(l-1):
+// The 128 x 128 diagonal blocks are inverted by one CTA each in shared memory
+// (invert_block).  Then level by level pairs of inverted blocks of h = 128,
+// 256, 512 are joined,
 //   [A B; 0 C]^{-1} = [A^{-1}, -A^{-1} (B C^{-1}); 0, C^{-1}]
 // as two FP32 products W = B C^{-1}, then -A^{-1} W, each an upper-triangular
 // operand whose zero blocks the tiles skip.  X (work, column-major, ld = ldp)
-// is built in place; its strictly lower part is never written and stays zero.
+// is built in place; its strictly lower part stays zero.
 // A final pass writes the hi/lo TF32 split of X for the tensor-core panels.
 // ---------------------------------------------------------------------------
 template <bool TRANS_T>
@@ -284,28 +286,34 @@ __device__ __forceinline__ float tri_t(const float *lu, int64_t lda, int b, int 
 	return lu[static_cast<int64_t>(j) * lda + p];
 }
 
-// grid (tiles, 2): blockIdx.y = 0 -> U11, 1 -> L11^T; one warp per tile.
-__global__ void __launch_bounds__(32) tri_diag_kernel(int b, const float *__restrict__ lu, int64_t lda,
-	float *__restrict__ xu, float *__restrict__ xl, int64_t ldp)
+// grid (128-blocks, 2): blockIdx.y = 0 -> U11, 1 -> L11^T.  Latency-bound: one
+// launch (TRIBLK) in place of a one-warp substitution per 32 x 32 tile and the products
+// of the h = 32 and 64 levels.  With one block in all (hi given) its TF32
+// split follows here as well.
+__global__ void __launch_bounds__(kTriThreads) tri_block_kernel(int b, int bp, const float *__restrict__ lu,
+	int64_t lda, float *__restrict__ xu, float *__restrict__ xl, int64_t ldp, float *__restrict__ uhi,
+	float *__restrict__ ulo, float *__restrict__ lhi, float *__restrict__ llo)
 {
-	__shared__ float Tb[32][33];
+	extern __shared__ __align__(16) float tri_smem[];
 	const bool lower = blockIdx.y != 0;
-	float *x = lower ? xl : xu;
-	const int o = blockIdx.x * 32, lane = threadIdx.x;
-	for (int i = 0; i < 32; ++i)
-		Tb[i][lane] = lower ? tri_t<true>(lu, lda, b, o + i, o + lane) : tri_t<false>(lu, lda, b, o + i, o + lane);
-	__syncwarp();
-	// column `lane` of the tile's inverse
-	float v[32];
-#pragma unroll
-	for (int i = 31; i >= 0; --i) {
-		float a = (i == lane) ? 1.f : 0.f;
-#pragma unroll
-		for (int p = i + 1; p < 32; ++p) a = fmaf(-Tb[i][p], v[p], a);
-		v[i] = lower ? a : a / Tb[i][i];
+	float *x = lower ? xl : xu, *hi = lower ? lhi : uhi, *lo = lower ? llo : ulo;
+	const int o = blockIdx.x * kTriBlock;
+	// the block as a lower triangle (L11, or U11^T): its inverse row by row is
+	// X column by column
+	invert_block(tri_smem, lu, lda, o, min(kTriBlock, b - o), !lower);
+	const int w = min(kTriBlock, bp - o);
+	for (int e = threadIdx.x; e < w * kTriBlock; e += kTriThreads) {
+		const int row = e % kTriBlock, col = e / kTriBlock;
+		if (row >= w) continue;
+		const float v = row <= col ? tri_smem[col * kInvLd + row] : 0.f;
+		const int64_t at = static_cast<int64_t>(o + col) * ldp + o + row;
+		x[at] = v;
+		if (hi && col < b) {
+			const float hv = tf32_hi(v);
+			hi[at] = hv;
+			lo[at] = v - hv;
+		}
 	}
-#pragma unroll
-	for (int i = 0; i < 32; ++i) x[static_cast<int64_t>(o + lane) * ldp + o + i] = v[i];
 }
 
 // One level's products for every pair and both triangles.  grid.x = 32 x 32
@@ -770,11 +778,20 @@ int launch_tri_inverses(const TcPanels &t, const float *lu, int64_t lda, cudaStr
 {
 	const int b = t.b;
 	const int bp = static_cast<int>(t.ldp);
-	const int nt = bp / 32;
-	tri_diag_kernel<<<dim3(nt, 2), 32, 0, st>>>(b, lu, lda, t.xu, t.xl, t.ldp);
+	const int nblk = (b + kTriBlock - 1) / kTriBlock;
+	const bool fused = split && nblk == 1;   // bp = ldp <= 128: one block holds it all
+	static DeviceOnce attr;
+	HPLAI_TRY(attr.get([](int, int *) -> int {
+		HPLAI_CUDA_TRY(cudaFuncSetAttribute(tri_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			static_cast<int>(kInvSmem<float>)));
+		return HPLAI_OK;
+	}));
+	tri_block_kernel<<<dim3(nblk, 2), kTriThreads, kInvSmem<float>, st>>>(b, bp, lu, lda, t.xu, t.xl, t.ldp,
+		fused ? t.uhi : nullptr, t.ulo, fused ? t.lhi : nullptr, t.llo);
 	count_launches();
 	HPLAI_CUDA_TRY(cudaGetLastError());
-	for (int h = 32; h < bp; h *= 2) {
+	if (fused) return HPLAI_OK;
+	for (int h = kTriBlock; h < bp; h *= 2) {
 		const int pairs = (bp + 2 * h - 1) / (2 * h);
 		const int tiles = ((h + 31) / 32) * ((h + 31) / 32);
 		const dim3 g(tiles, pairs, 2);
