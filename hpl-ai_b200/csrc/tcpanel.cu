@@ -609,29 +609,44 @@ __global__ void __launch_bounds__(TTHREADS, 1) tf32x3_kernel(const __grid_consta
 				tmem_ld_wait();
 				const int col0 = tn * TBN + ch * 32;
 				if (rok) {
+					float *o32 = p.out32 + row * p.s32m + col0 * p.s32n;
 					__half *o16 = p.out16 ? p.out16 + row * p.s16m + col0 * p.s16n : nullptr;
-					// a row-major FP16 copy gets this thread's 32 columns as four 16-byte stores
-					const bool vec16 = o16 && p.s16n == 1 && col0 + 32 <= p.n && (reinterpret_cast<uintptr_t>(o16) & 15u) == 0;
+					const int nc = p.n - col0;
+					if (nc >= 32) {
+						// the addresses step by a constant: no multiply or test per element
 #pragma unroll
-					for (int j = 0; j < 32; ++j) {
-						const int col = col0 + j;
-						if (col < p.n) {
-							const float v = __uint_as_float(r[j]);
-							p.out32[row * p.s32m + col * p.s32n] = v;
-							if (o16 && !vec16) p.out16[row * p.s16m + col * p.s16n] = __float2half_rn(p.scale * v);
+						for (int j = 0; j < 32; ++j) {
+							*o32 = __uint_as_float(r[j]);
+							o32 += p.s32n;
 						}
-					}
-					if (vec16) {
+						if (o16 && p.s16n == 1 && (reinterpret_cast<uintptr_t>(o16) & 15u) == 0) {
+							// a row-major FP16 copy gets this thread's 32 columns as four 16-byte stores
 #pragma unroll
-						for (int q = 0; q < 4; ++q) {
-							uint32_t w4[4];
+							for (int q = 0; q < 4; ++q) {
+								uint32_t w4[4];
 #pragma unroll
-							for (int e = 0; e < 4; ++e) {
-								const __half2 h2 = __floats2half2_rn(p.scale * __uint_as_float(r[8 * q + 2 * e]),
-									p.scale * __uint_as_float(r[8 * q + 2 * e + 1]));
-								w4[e] = *reinterpret_cast<const uint32_t *>(&h2);
+								for (int e = 0; e < 4; ++e) {
+									const __half2 h2 = __floats2half2_rn(p.scale * __uint_as_float(r[8 * q + 2 * e]),
+										p.scale * __uint_as_float(r[8 * q + 2 * e + 1]));
+									w4[e] = *reinterpret_cast<const uint32_t *>(&h2);
+								}
+								*reinterpret_cast<uint4 *>(o16 + 8 * q) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
 							}
-							*reinterpret_cast<uint4 *>(o16 + 8 * q) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+						} else if (o16) {
+#pragma unroll
+							for (int j = 0; j < 32; ++j) {
+								*o16 = __float2half_rn(p.scale * __uint_as_float(r[j]));
+								o16 += p.s16n;
+							}
+						}
+					} else {
+#pragma unroll
+						for (int j = 0; j < 32; ++j) {
+							if (j < nc) {
+								const float v = __uint_as_float(r[j]);
+								o32[j * p.s32n] = v;
+								if (o16) o16[j * p.s16n] = __float2half_rn(p.scale * v);
+							}
 						}
 					}
 				}
