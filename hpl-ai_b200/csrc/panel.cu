@@ -20,11 +20,10 @@ namespace hplai {
 // ---------------------------------------------------------------------------
 // Panel TRSM + FP16 copy, one kernel for both panels.
 //
-// X (m x b) <- X * T^{-1} with T upper triangular (b x b).  A CTA owns R rows
-// of X in shared memory (Xs[j*LDX + r]).
+// X (m x b) <- X * T^{-1} with T upper triangular (b x b).
 //   L panel (update_left_panels):  X = A_col (column-major, X[r][j] at
 //            a[j*lda + r]), T = U11 (T[p][j] at t[j*ldt + p]), non-unit.
-//   U panel (update_right_panels): L^{-1} A_row = (A_row^T L^{-T})^T, so
+//   U panel (update_right_panels, UPANEL): L^{-1} A_row = (A_row^T L^{-T})^T, so
 //            X = A_row^T (row-major, X[r][j] at a[r*lda + j]) and T = L11^T
 //            (T[p][j] = L[j][p] at t[p*ldt + j]), unit diagonal.
 // Element (r, j) receives x -= T[p][j] * x[r][p] for p = 0..j-1 in
@@ -32,150 +31,321 @@ namespace hplai {
 // both (R,U,N,N) and (L,L,N,U), so the result is bit-exact with it.
 // hc[(row0 + r)*ldh + j] = half(scale * X[r][j]) in both cases (the L copy is
 // row-major; the U copy stores column j of U as row j).
+//
+// Bound by FP32 issue.  A CTA owns 32 RL rows; a thread holds RL rows (lane,
+// lane + 32) of 16 columns (its warp's) of a 128-column block in registers.
+// Per block: the products with the columns solved before (X and T in chunks
+// of 32 p through three cp.async stages), then the block's own triangle 16
+// columns at a time -- the owning warp solves them in registers and publishes
+// them, every later warp applies them (one barrier per 16 columns).  8200 rows,
+// b = 512: 124 us a panel (270 with rows staged in shared memory and 4 x 4
+// products, two shared-memory reads per four FMAs).
 // ---------------------------------------------------------------------------
 constexpr int kTrsmThreads = 256;
+constexpr int kTB = 128;          // columns per block: 16 per warp
+constexpr int kMicro = 16;
+constexpr int kKC = 32;           // p per chunk
+constexpr int kStages = 3;
+constexpr int kLdTri = kTB + 4;
+constexpr int kLdP = kKC + 4;     // chunk rows that run along p
 
-template <int R, bool ROWX, bool TRANS_T>
-__global__ void __launch_bounds__(kTrsmThreads) trsm_kernel(int m, int b, const float *__restrict__ t,
-	int64_t ldt, float *__restrict__ a, int64_t lda, __half *__restrict__ hc, int64_t ldh, float scale)
+template <int RL, bool UPANEL>
+struct TrsmSmem {
+	static constexpr int R = 32 * RL;
+	static constexpr int LDX = UPANEL ? kLdP : R + 4;        // X chunk: [r][p] or [p][r]
+	static constexpr int LDT = UPANEL ? kLdTri : kLdP;       // T chunk: [p][c] or [c][p]
+	static constexpr int XC = (UPANEL ? R : kKC) * LDX;
+	static constexpr int TC = (UPANEL ? kKC : kTB) * LDT;
+	static constexpr size_t bytes = sizeof(float) *
+		(kTB * kLdTri + kTB + 2 * kMicro * R + kStages * static_cast<size_t>(XC + TC));
+};
+
+// lines x len floats, line l at src + l * lds, to dst + l * ldd; lines from
+// nl on and elements from ne on are zero.
+__device__ __forceinline__ void stage_lines(float *dst, int ldd, const float *src, int64_t lds, int lines, int len,
+	int nl, int ne, bool vec)
 {
-	constexpr int CW = 4 * 4 * kTrsmThreads / R;   // update chunk width (4x4 tiles, one per thread)
-	constexpr int LDX = R + 4;                     // padded so row-wise reads spread over banks
-	constexpr int LDU = CW + 1;
-	constexpr bool UNIT = TRANS_T;                 // L11^T has a unit diagonal
-	extern __shared__ float sm[];
-	float *Xs = sm;                                  // b x LDX
-	float *Us = Xs + static_cast<size_t>(b) * LDX;   // 32 x LDU, Us[p*LDU + cc] = T[jb+p][c0+cc]
-	float *Ud = Us + 32 * LDU;                       // 32 x 33,  Ud[p*33 + j]  = T[jb+p][jb+j]
-	float *inv = Ud + 32 * 33;                       // 32 reciprocals
-	const int tid = threadIdx.x;
-	const int row0 = blockIdx.x * R;
-	const int rows = min(R, m - row0);
-	auto tval = [&](int p, int j) -> float {
-		return TRANS_T ? t[static_cast<int64_t>(p) * ldt + j] : t[static_cast<int64_t>(j) * ldt + p];
-	};
-
-	if (ROWX) {
-		for (int idx = tid; idx < R * b; idx += kTrsmThreads) {
-			const int r = idx / b, j = idx - r * b;
-			Xs[j * LDX + r] = (r < rows) ? a[static_cast<int64_t>(row0 + r) * lda + j] : 0.f;
+	if (vec) {
+		const int g4 = len / 4;
+		for (int e = threadIdx.x; e < lines * g4; e += kTrsmThreads) {
+			const int l = e / g4, g = (e % g4) * 4;
+			int bytes = l < nl ? (ne - g) * 4 : 0;
+			bytes = bytes < 0 ? 0 : (bytes > 16 ? 16 : bytes);
+			const float *p = src + (bytes ? static_cast<int64_t>(l) * lds + g : 0);
+			asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + l * ldd + g)), "l"(p),
+				"r"(bytes) : "memory");
 		}
 	} else {
-		for (int idx = tid; idx < R * b; idx += kTrsmThreads) {
-			const int r = idx % R, j = idx / R;
-			Xs[j * LDX + r] = (r < rows) ? a[static_cast<int64_t>(j) * lda + row0 + r] : 0.f;
-		}
-	}
-
-	for (int jb = 0; jb < b; jb += 32) {
-		const int jw = min(32, b - jb);
-		for (int idx = tid; idx < 32 * 32; idx += kTrsmThreads) {
-			const int p = TRANS_T ? (idx >> 5) : (idx & 31), j = TRANS_T ? (idx & 31) : (idx >> 5);
-			Ud[p * 33 + j] = (p < jw && j < jw) ? tval(jb + p, jb + j) : 0.f;
-		}
-		if (!UNIT && tid < jw) inv[tid] = 1.0f / tval(jb + tid, jb + tid);
-		__syncthreads();
-		// Triangular 32-column block: one row per thread.
-		if (tid < R) {
-			float x[32];
-#pragma unroll
-			for (int j = 0; j < 32; ++j) x[j] = (j < jw) ? Xs[(jb + j) * LDX + tid] : 0.f;
-#pragma unroll
-			for (int j = 0; j < 32; ++j) {
-				if (j < jw) {
-#pragma unroll
-					for (int p = 0; p < j; ++p) x[j] = fmaf(-Ud[p * 33 + j], x[p], x[j]);
-					if (!UNIT) x[j] *= inv[j];
-				}
-			}
-#pragma unroll
-			for (int j = 0; j < 32; ++j)
-				if (j < jw) Xs[(jb + j) * LDX + tid] = x[j];
-		}
-		__syncthreads();
-		// Update the columns right of the block, CW at a time.
-		for (int c0 = jb + jw; c0 < b; c0 += CW) {
-			const int cw = min(CW, b - c0);
-			for (int idx = tid; idx < 32 * CW; idx += kTrsmThreads) {
-				// coalesced along the contiguous index of T's storage
-				const int p = TRANS_T ? (idx / CW) : (idx & 31), cc = TRANS_T ? (idx % CW) : (idx >> 5);
-				Us[p * LDU + cc] = (p < jw && cc < cw) ? tval(jb + p, c0 + cc) : 0.f;
-			}
-			__syncthreads();
-			const int rt = tid % (R / 4), ct = tid / (R / 4);
-			const int r0 = rt * 4, cc0 = ct * 4;
-			if (cc0 < cw) {
-				float acc[4][4];
-#pragma unroll
-				for (int i = 0; i < 4; ++i)
-#pragma unroll
-					for (int j = 0; j < 4; ++j)
-						acc[i][j] = (cc0 + j < cw) ? Xs[(c0 + cc0 + j) * LDX + r0 + i] : 0.f;
-				for (int p = 0; p < jw; ++p) {
-					const float4 xv = *reinterpret_cast<const float4 *>(&Xs[(jb + p) * LDX + r0]);
-					const float xr[4] = {xv.x, xv.y, xv.z, xv.w};
-					float ur[4];
-#pragma unroll
-					for (int j = 0; j < 4; ++j) ur[j] = Us[p * LDU + cc0 + j];
-#pragma unroll
-					for (int i = 0; i < 4; ++i)
-#pragma unroll
-						for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(-ur[j], xr[i], acc[i][j]);
-				}
-#pragma unroll
-				for (int i = 0; i < 4; ++i)
-#pragma unroll
-					for (int j = 0; j < 4; ++j)
-						if (cc0 + j < cw) Xs[(c0 + cc0 + j) * LDX + r0 + i] = acc[i][j];
-			}
-			__syncthreads();
-		}
-	}
-
-	if (ROWX) {
-		for (int idx = tid; idx < R * b; idx += kTrsmThreads) {
-			const int r = idx / b, j = idx - r * b;
-			if (r < rows) a[static_cast<int64_t>(row0 + r) * lda + j] = Xs[j * LDX + r];
-		}
-	} else {
-		for (int idx = tid; idx < R * b; idx += kTrsmThreads) {
-			const int r = idx % R, j = idx / R;
-			if (r < rows) a[static_cast<int64_t>(j) * lda + row0 + r] = Xs[j * LDX + r];
-		}
-	}
-	if (hc) {
-		// 8 consecutive halves per thread (16-byte store), rows across lanes.
-		const int b8 = b / 8;
-		for (int idx = tid; idx < R * b8; idx += kTrsmThreads) {
-			const int r = idx % R, q = idx / R;
-			if (r < rows) {
-				__align__(16) __half h[8];
-#pragma unroll
-				for (int e = 0; e < 8; ++e) h[e] = __float2half_rn(scale * Xs[(8 * q + e) * LDX + r]);
-				*reinterpret_cast<uint4 *>(hc + static_cast<int64_t>(row0 + r) * ldh + 8 * q) =
-					*reinterpret_cast<const uint4 *>(h);
-			}
-		}
-		for (int idx = tid; idx < R * (b - 8 * b8); idx += kTrsmThreads) {
-			const int r = idx % R, j = 8 * b8 + idx / R;
-			if (r < rows) hc[static_cast<int64_t>(row0 + r) * ldh + j] = __float2half_rn(scale * Xs[j * LDX + r]);
+		for (int e = threadIdx.x; e < lines * len; e += kTrsmThreads) {
+			const int l = e / len, g = e % len;
+			if (l < nl && g < ne)
+				dst[l * ldd + g] = __ldcg(src + static_cast<int64_t>(l) * lds + g);
+			else
+				dst[l * ldd + g] = 0.f;
 		}
 	}
 }
 
-template <int R, bool ROWX, bool TRANS_T>
+template <int RL, bool UPANEL>
+__device__ __forceinline__ void trsm_rows(float *sm, int m, int b, const float *__restrict__ t, int64_t ldt, float *a,
+	int64_t lda, __half *__restrict__ hc, int64_t ldh, float scale, int vec_x, int vec_t)
+{
+	using S = TrsmSmem<RL, UPANEL>;
+	constexpr int R = S::R;
+	constexpr bool UNIT = UPANEL;   // L11^T has a unit diagonal
+	float *tri = sm;                      // tri[i * kLdTri + j] = T[j0 + i][j0 + j]
+	float *inv = tri + kTB * kLdTri;
+	float *pub = inv + kTB;               // [2][16][R]
+	float *chunks = pub + 2 * kMicro * R; // kStages x (X chunk, T chunk)
+	const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+	const int row0 = blockIdx.x * R, rows = min(R, m - row0);
+	const int e0 = kMicro * wp;
+	for (int j0 = 0; j0 < b; j0 += kTB) {
+		const int jw = min(kTB, b - j0), nc = j0 / kKC;
+		auto stage = [&](int q) {
+			if (q < nc) {
+				float *xc = chunks + (q % kStages) * (S::XC + S::TC), *tc = xc + S::XC;
+				const int p0 = q * kKC;
+				if (UPANEL) {
+					stage_lines(xc, S::LDX, a + static_cast<int64_t>(row0) * lda + p0, lda, R, kKC, rows, kKC, vec_x != 0);
+					stage_lines(tc, S::LDT, t + static_cast<int64_t>(p0) * ldt + j0, ldt, kKC, kTB, kKC, jw, vec_t != 0);
+				} else {
+					stage_lines(xc, S::LDX, a + static_cast<int64_t>(p0) * lda + row0, lda, kKC, R, kKC, rows, vec_x != 0);
+					stage_lines(tc, S::LDT, t + static_cast<int64_t>(j0) * ldt + p0, ldt, kTB, kKC, jw, kKC, vec_t != 0);
+				}
+			}
+			asm volatile("cp.async.commit_group;" ::: "memory");
+		};
+		for (int q = 0; q < kStages - 1; ++q) stage(q);
+		// this block's triangle (rows and columns past jw zero) and columns; the
+		// loads of each are all in flight together
+		if (UPANEL) {
+			stage_lines(tri, kLdTri, t + static_cast<int64_t>(j0) * ldt + j0, ldt, kTB, kTB, jw, jw, vec_t != 0);
+			asm volatile("cp.async.commit_group;" ::: "memory");
+		} else if (vec_t && jw % 4 == 0) {
+			const int c = tid % 32, r4 = (tid / 32) * 4;   // lanes along the columns: rows of T without bank conflicts
+			float4 f[16];
+#pragma unroll
+			for (int q = 0; q < 16; ++q) {
+				const int cc = c + 32 * (q & 3), rr = r4 + 32 * (q >> 2);
+				f[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+				if (cc < jw && rr < jw)
+					f[q] = __ldcg(reinterpret_cast<const float4 *>(t + static_cast<int64_t>(j0 + cc) * ldt + j0 + rr));
+			}
+#pragma unroll
+			for (int q = 0; q < 16; ++q) {
+				const int cc = c + 32 * (q & 3), rr = r4 + 32 * (q >> 2);
+				tri[rr * kLdTri + cc] = f[q].x;
+				tri[(rr + 1) * kLdTri + cc] = f[q].y;
+				tri[(rr + 2) * kLdTri + cc] = f[q].z;
+				tri[(rr + 3) * kLdTri + cc] = f[q].w;
+			}
+		} else {
+#pragma unroll 16
+			for (int e = tid; e < kTB * kTB; e += kTrsmThreads) {
+				const int p = e % kTB, j = e / kTB;
+				tri[p * kLdTri + j] = (p < jw && j < jw) ? __ldcg(t + static_cast<int64_t>(j0 + j) * ldt + j0 + p) : 0.f;
+			}
+		}
+		float x[RL][kMicro];
+		const bool wide = UPANEL && vec_x && e0 + kMicro <= jw;   // this thread's 16 elements as four float4
+#pragma unroll
+		for (int r = 0; r < RL; ++r) {
+			const int row = lane + 32 * r;
+			const float *src = UPANEL ? a + static_cast<int64_t>(row0 + row) * lda + j0 + e0
+			                          : a + static_cast<int64_t>(j0 + e0) * lda + row0 + row;
+			if (wide) {
+#pragma unroll
+				for (int g = 0; g < kMicro / 4; ++g) {
+					float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+					if (row < rows) v = __ldcg(reinterpret_cast<const float4 *>(src + 4 * g));
+					x[r][4 * g] = v.x;
+					x[r][4 * g + 1] = v.y;
+					x[r][4 * g + 2] = v.z;
+					x[r][4 * g + 3] = v.w;
+				}
+			} else {
+#pragma unroll
+				for (int c = 0; c < kMicro; ++c)
+					x[r][c] = (row < rows && e0 + c < jw) ? __ldcg(src + (UPANEL ? c : static_cast<int64_t>(c) * lda)) : 0.f;
+			}
+		}
+		for (int q = 0; q < nc; ++q) {
+			asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+			__syncthreads();   // chunk q is here; everyone is done with the one before it
+			stage(q + kStages - 1);
+			const float *xc = chunks + (q % kStages) * (S::XC + S::TC), *tc = xc + S::XC;
+#pragma unroll 2
+			for (int p = 0; p < kKC; p += 4) {
+				float xp[RL][4];
+#pragma unroll
+				for (int r = 0; r < RL; ++r) {
+					if (UPANEL) {
+						const float4 v = *reinterpret_cast<const float4 *>(xc + (lane + 32 * r) * S::LDX + p);
+						xp[r][0] = v.x;
+						xp[r][1] = v.y;
+						xp[r][2] = v.z;
+						xp[r][3] = v.w;
+					} else {
+#pragma unroll
+						for (int k = 0; k < 4; ++k) xp[r][k] = xc[(p + k) * S::LDX + lane + 32 * r];
+					}
+				}
+				if (UPANEL) {
+#pragma unroll
+					for (int k = 0; k < 4; ++k)
+#pragma unroll
+						for (int g = 0; g < kMicro / 4; ++g) {
+							const float4 v = *reinterpret_cast<const float4 *>(tc + (p + k) * S::LDT + e0 + 4 * g);
+#pragma unroll
+							for (int r = 0; r < RL; ++r) {
+								x[r][4 * g] = fmaf(-v.x, xp[r][k], x[r][4 * g]);
+								x[r][4 * g + 1] = fmaf(-v.y, xp[r][k], x[r][4 * g + 1]);
+								x[r][4 * g + 2] = fmaf(-v.z, xp[r][k], x[r][4 * g + 2]);
+								x[r][4 * g + 3] = fmaf(-v.w, xp[r][k], x[r][4 * g + 3]);
+							}
+						}
+				} else {
+#pragma unroll
+					for (int c = 0; c < kMicro; ++c) {
+						const float4 v = *reinterpret_cast<const float4 *>(tc + (e0 + c) * S::LDT + p);
+#pragma unroll
+						for (int r = 0; r < RL; ++r) {
+							x[r][c] = fmaf(-v.x, xp[r][0], x[r][c]);
+							x[r][c] = fmaf(-v.y, xp[r][1], x[r][c]);
+							x[r][c] = fmaf(-v.z, xp[r][2], x[r][c]);
+							x[r][c] = fmaf(-v.w, xp[r][3], x[r][c]);
+						}
+					}
+				}
+			}
+		}
+		asm volatile("cp.async.wait_all;" ::: "memory");
+		__syncthreads();   // the triangle is here
+		if (!UNIT && tid < kTB) inv[tid] = tid < jw ? 1.0f / tri[tid * kLdTri + tid] : 0.f;
+		if (!UNIT) __syncthreads();
+		const int nmicro = (jw + kMicro - 1) / kMicro;
+		for (int oi = 0; oi < nmicro; ++oi) {
+			float *const pb = pub + (oi & 1) * kMicro * R + lane;
+			if (wp == oi) {
+#pragma unroll
+				for (int li = 0; li < kMicro; ++li) {
+					const int i = kMicro * oi + li;
+#pragma unroll
+					for (int r = 0; r < RL; ++r) {
+						if (!UNIT) x[r][li] *= inv[i];
+						pb[li * R + 32 * r] = x[r][li];
+					}
+					const float4 *row = reinterpret_cast<const float4 *>(tri + i * kLdTri + e0);
+#pragma unroll
+					for (int g = (li + 1) / 4; g < kMicro / 4; ++g) {
+						const float4 v = row[g];
+						const float tv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+						for (int h = 0; h < 4; ++h) {
+							const int c = 4 * g + h;
+							if (c <= li) continue;
+#pragma unroll
+							for (int r = 0; r < RL; ++r) x[r][c] = fmaf(-tv[h], x[r][li], x[r][c]);
+						}
+					}
+				}
+			}
+			__syncthreads();
+			if (wp > oi) {
+#pragma unroll 4
+				for (int li = 0; li < kMicro; ++li) {
+					float xi[RL];
+#pragma unroll
+					for (int r = 0; r < RL; ++r) xi[r] = pb[li * R + 32 * r];
+					const float4 *row = reinterpret_cast<const float4 *>(tri + (kMicro * oi + li) * kLdTri + e0);
+#pragma unroll
+					for (int g = 0; g < kMicro / 4; ++g) {
+						const float4 v = row[g];
+#pragma unroll
+						for (int r = 0; r < RL; ++r) {
+							x[r][4 * g] = fmaf(-v.x, xi[r], x[r][4 * g]);
+							x[r][4 * g + 1] = fmaf(-v.y, xi[r], x[r][4 * g + 1]);
+							x[r][4 * g + 2] = fmaf(-v.z, xi[r], x[r][4 * g + 2]);
+							x[r][4 * g + 3] = fmaf(-v.w, xi[r], x[r][4 * g + 3]);
+						}
+					}
+				}
+			}
+		}
+#pragma unroll
+		for (int r = 0; r < RL; ++r) {
+			const int row = lane + 32 * r;
+			if (row >= rows) continue;
+			float *dst = UPANEL ? a + static_cast<int64_t>(row0 + row) * lda + j0 + e0
+			                    : a + static_cast<int64_t>(j0 + e0) * lda + row0 + row;
+			if (wide) {
+#pragma unroll
+				for (int g = 0; g < kMicro / 4; ++g)
+					*reinterpret_cast<float4 *>(dst + 4 * g) =
+						make_float4(x[r][4 * g], x[r][4 * g + 1], x[r][4 * g + 2], x[r][4 * g + 3]);
+			} else {
+#pragma unroll
+				for (int c = 0; c < kMicro; ++c)
+					if (e0 + c < jw) dst[UPANEL ? c : static_cast<int64_t>(c) * lda] = x[r][c];
+			}
+			if (hc) {
+				__half *o = hc + static_cast<int64_t>(row0 + row) * ldh + j0 + e0;
+#pragma unroll
+				for (int q = 0; q < kMicro / 8; ++q) {
+					if (e0 + 8 * q + 8 <= jw) {
+						// 8 halves, 16-byte aligned: hc is, ldh and the offset are multiples of 8
+						__align__(16) __half h[8];
+#pragma unroll
+						for (int e = 0; e < 8; ++e) h[e] = __float2half_rn(scale * x[r][8 * q + e]);
+						*reinterpret_cast<uint4 *>(o + 8 * q) = *reinterpret_cast<const uint4 *>(h);
+					} else {
+#pragma unroll
+						for (int e = 0; e < 8; ++e)
+							if (e0 + 8 * q + e < jw) o[8 * q + e] = __float2half_rn(scale * x[r][8 * q + e]);
+					}
+				}
+			}
+		}
+		__syncthreads();   // X is in memory for the next block; the triangle is free
+	}
+}
+
+template <int RL, bool UPANEL>
+__global__ void __launch_bounds__(kTrsmThreads) trsm_kernel(int m, int b, const float *__restrict__ t, int64_t ldt,
+	float *a, int64_t lda, __half *__restrict__ hc, int64_t ldh, float scale, int vec_x, int vec_t)
+{
+	extern __shared__ __align__(16) float sm[];
+	trsm_rows<RL, UPANEL>(sm, m, b, t, ldt, a, lda, hc, ldh, scale, vec_x, vec_t);
+}
+
+template <int RL, bool UPANEL>
 static int trsm_launch(int m, int b, const float *t, int64_t ldt, float *a, int64_t lda, uint16_t *hc, int64_t ldh,
 	float scale, cudaStream_t st)
 {
-	constexpr int CW = 4 * 4 * kTrsmThreads / R;
-	const size_t smem = (static_cast<size_t>(b) * (R + 4) + 32 * (CW + 1) + 32 * 33 + 32) * sizeof(float);
-	HPLAI_CUDA_TRY(cudaFuncSetAttribute(trsm_kernel<R, ROWX, TRANS_T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		static_cast<int>(smem)));
-	trsm_kernel<R, ROWX, TRANS_T><<<(m + R - 1) / R, kTrsmThreads, smem, st>>>(m, b, t, ldt, a, lda,
-		reinterpret_cast<__half *>(hc), ldh, scale);
+	constexpr size_t smem = TrsmSmem<RL, UPANEL>::bytes;
+	static DeviceOnce attr;
+	HPLAI_TRY(attr.get([](int, int *) -> int {
+		HPLAI_CUDA_TRY(cudaFuncSetAttribute(trsm_kernel<RL, UPANEL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			static_cast<int>(smem)));
+		return HPLAI_OK;
+	}));
+	auto vec = [](const float *p, int64_t ld) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0 && ld % 4 == 0 ? 1 : 0; };
+	trsm_kernel<RL, UPANEL><<<(m + 32 * RL - 1) / (32 * RL), kTrsmThreads, smem, st>>>(m, b, t, ldt, a, lda,
+		reinterpret_cast<__half *>(hc), ldh, scale, vec(a, lda), vec(t, ldt));
 	count_launches();
 	HPLAI_CUDA_TRY(cudaGetLastError());
 	return HPLAI_OK;
+}
+
+// 64 rows per CTA reuse each triangle read twice; below 74 such CTAs half the
+// GPU would idle, and 32 rows per CTA are faster.
+template <bool UPANEL>
+static int trsm_pick(int m, int b, const float *t, int64_t ldt, float *a, int64_t lda, uint16_t *hc, int64_t ldh,
+	float scale, cudaStream_t st)
+{
+	if (m > 64 * 74) return trsm_launch<2, UPANEL>(m, b, t, ldt, a, lda, hc, ldh, scale, st);
+	return trsm_launch<1, UPANEL>(m, b, t, ldt, a, lda, hc, ldh, scale, st);
 }
 
 static bool vec_ok(const uint16_t *hc, int64_t ldh)
@@ -188,8 +358,7 @@ int launch_trsm_right_upper(int m, int b, const float *u, int64_t ldu, float *a,
 {
 	if (m <= 0) return HPLAI_OK;
 	if (b <= 0 || b > 1024 || !vec_ok(lh, ldh)) return HPLAI_EINVAL;
-	if (b <= 512) return trsm_launch<64, false, false>(m, b, u, ldu, a, lda, lh, ldh, scale, st);
-	return trsm_launch<32, false, false>(m, b, u, ldu, a, lda, lh, ldh, scale, st);
+	return trsm_pick<false>(m, b, u, ldu, a, lda, lh, ldh, scale, st);
 }
 
 int launch_trsm_left_lower(int b, int ncols, const float *l, int64_t ldl, float *a, int64_t lda, uint16_t *uh,
@@ -197,8 +366,7 @@ int launch_trsm_left_lower(int b, int ncols, const float *l, int64_t ldl, float 
 {
 	if (ncols <= 0) return HPLAI_OK;
 	if (b <= 0 || b > 1024 || !vec_ok(uh, ldh)) return HPLAI_EINVAL;
-	if (b <= 512) return trsm_launch<64, true, true>(ncols, b, l, ldl, a, lda, uh, ldh, scale, st);
-	return trsm_launch<32, true, true>(ncols, b, l, ldl, a, lda, uh, ldh, scale, st);
+	return trsm_pick<true>(ncols, b, l, ldl, a, lda, uh, ldh, scale, st);
 }
 
 } // namespace hplai

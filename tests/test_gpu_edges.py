@@ -49,6 +49,31 @@ def test_getrf_pivots_without_normal_reciprocals(hplai, oracle, torch_cuda, scal
     assert np.array_equal(nan, np.isnan(got)) and _same_bits(np.where(nan, 0, got), np.where(nan, 0, ref))
 
 
+# rows around a CTA's 32 or 64 and the rule's 4736, widths around the 16-column steps and 128-column blocks
+@pytest.mark.parametrize("m,b,off", [(1, 1, 0), (31, 15, 0), (33, 16, 1), (65, 17, 0), (100, 127, 0), (64, 128, 0),
+                                     (70, 129, 0), (200, 260, 3), (40, 1000, 0), (4736, 48, 0), (4737, 50, 0)])
+def test_panel_solve_edges(hplai, oracle, torch_cuda, m, b, off):
+    torch = torch_cuda
+    rng = np.random.default_rng(m + b)
+    lu = _dominant(rng, b)
+    lu[np.tril_indices(b, -1)] *= np.float32(4.0 / max(b, 4))
+    d, dp = _put(torch, lu, b, off)
+    ldh = (b + 7) // 8 * 8
+    x = np.asfortranarray(rng.uniform(-0.5, 0.5, (m, b)).astype(np.float32))
+    t, p = _put(torch, x, m, off)
+    h = torch.zeros((m, ldh), dtype=torch.float16, device="cuda")
+    hplai.check(hplai.trsm_right_upper(m, b, dp, b, p, m, h.data_ptr(), ldh, 2.0, None))
+    ref = oracle.trsm_right_upper(np.triu(lu), x)
+    assert _same_bits(_take(t, m, b, m, off), ref)
+    assert np.array_equal(h.cpu().numpy()[:, :b], (np.float32(2.0) * ref).astype(np.float16))
+    y = np.asfortranarray(rng.uniform(-0.5, 0.5, (b, m)).astype(np.float32))
+    t, p = _put(torch, y, b, off)
+    hplai.check(hplai.trsm_left_lower(b, m, dp, b, p, b, h.data_ptr(), ldh, 1.0, None))
+    ref = oracle.trsm_left_lower_unit(np.tril(lu, -1) + np.eye(b, dtype=np.float32), y)
+    assert _same_bits(_take(t, b, m, b, off), ref)
+    assert np.array_equal(h.cpu().numpy()[:, :b], ref.T.astype(np.float16))
+
+
 @pytest.mark.parametrize("n,i0,j0,nr,nc,lda,off", [(1000, 3, 5, 1, 1, 1, 0), (1000, 0, 100, 127, 33, 127, 0),
                                                    (4000, 1, 7, 1023, 31, 1024, 0), (4000, 9, 0, 1025, 65, 1025, 0),
                                                    (4000, 0, 2000, 2050, 40, 2052, 1)])
