@@ -538,6 +538,17 @@ bool f16_panel_form(const hplai_ctx *c, bool simt)
 	return !simt && c->precision == HPLAI_F32_F8 && c->b % 4 == 0;
 }
 
+// The plain form's panels by substitution on the CUDA cores, both in one
+// launch, while they are small: the tensor-core path's inverses, splits and
+// products are seven or more dependent launches that a small panel does not
+// fill.  Measured (tensor cores / one launch): b = 60, 600 rows 42 / 11 us,
+// 9600 43 / 31, 39960 69 / 86; b = 128, 9600 48 / 45, 19968 56 / 76; b = 256,
+// 2304 71 / 36, 9472 79 / 83; b = 512, 2048 109 / 94, 4608 118 / 189.
+bool pair_panel_form(const hplai_ctx *c, int rem)
+{
+	return c->precision == HPLAI_F32_F16 && static_cast<int64_t>(rem) * c->b <= 1200000;
+}
+
 // Factor the diagonal block of step k and form its two panels with their
 // FP16 copies in slot `slot` of group buffer `buf` (getrf_nopiv +
 // update_left/right_panels + convert_left/right_panels,
@@ -602,6 +613,11 @@ int panel_step(hplai_ctx *c, int k, int buf, int slot, bool simt, int side_ctas,
 		}
 		HPLAI_TRY(launch_lpanel_f16(c->tc, c->maps[buf][slot], static_cast<int>(kb), rem, c->A, lda, lslot, uslot, ldg,
 			deck, c->deck_ld, inv_dscale, side_ctas, st, src, n, &al));
+	} else if (pair_panel_form(c, rem)) {
+		// both panels and their FP16 copies, timed as TRSM_L
+		HPLAI_TRY(launch_trsm_pair(rem, b, diag, diag + b, diag + static_cast<int64_t>(b) * lda, lda, lslot + (kb + b) * ldg,
+			uslot + (kb + b) * ldg, ldg, st));
+		return pe.end(st);
 	} else {
 		HPLAI_TRY(launch_tri_inverses(c->tc, diag, lda, st));
 		// the precision form's Schur update reads the e4m3 copies only: no FP16 copy

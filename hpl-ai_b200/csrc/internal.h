@@ -59,6 +59,10 @@ int launch_trsm_right_upper(int m, int b, const float *u, int64_t ldu, float *a,
 	int64_t ldh, float scale, cudaStream_t st);
 int launch_trsm_left_lower(int b, int ncols, const float *l, int64_t ldl, float *a, int64_t lda, uint16_t *uh,
 	int64_t ldh, float scale, cudaStream_t st);
+// Both panels of a step in one launch: acol (rem x b) <- acol U^{-1}, arow (b x rem) <- L^{-1} arow with the factored
+// block diag, all in one matrix (lda), and their FP16 copies.
+int launch_trsm_pair(int rem, int b, const float *diag, float *acol, float *arow, int64_t lda, uint16_t *lh,
+	uint16_t *uh, int64_t ldh, cudaStream_t st);
 
 // schur.cu
 // Tensor maps for the FP16 panel buffers are built once per buffer and

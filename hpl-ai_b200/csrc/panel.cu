@@ -319,6 +319,19 @@ __global__ void __launch_bounds__(kTrsmThreads) trsm_kernel(int m, int b, const 
 	trsm_rows<RL, UPANEL>(sm, m, b, t, ldt, a, lda, hc, ldh, scale, vec_x, vec_t);
 }
 
+// Both panels of a step in one launch (blockIdx.y = 0: L, 1: U), the
+// triangles and panels in one matrix.
+template <int RL>
+__global__ void __launch_bounds__(kTrsmThreads) trsm_pair_kernel(int rem, int b, const float *__restrict__ lu, float *acol,
+	float *arow, int64_t lda, __half *__restrict__ lh, __half *__restrict__ uh, int64_t ldh, int vec)
+{
+	extern __shared__ __align__(16) float sm[];
+	if (blockIdx.y == 0)
+		trsm_rows<RL, false>(sm, rem, b, lu, lda, acol, lda, lh, ldh, 1.0f, vec, vec);
+	else
+		trsm_rows<RL, true>(sm, rem, b, lu, lda, arow, lda, uh, ldh, 1.0f, vec, vec);
+}
+
 template <int RL, bool UPANEL>
 static int trsm_launch(int m, int b, const float *t, int64_t ldt, float *a, int64_t lda, uint16_t *hc, int64_t ldh,
 	float scale, cudaStream_t st)
@@ -367,6 +380,34 @@ int launch_trsm_left_lower(int b, int ncols, const float *l, int64_t ldl, float 
 	if (ncols <= 0) return HPLAI_OK;
 	if (b <= 0 || b > 1024 || !vec_ok(uh, ldh)) return HPLAI_EINVAL;
 	return trsm_pick<true>(ncols, b, l, ldl, a, lda, uh, ldh, scale, st);
+}
+
+template <int RL>
+static int pair_launch(int rem, int b, const float *diag, float *acol, float *arow, int64_t lda, uint16_t *lh,
+	uint16_t *uh, int64_t ldh, cudaStream_t st)
+{
+	constexpr size_t sl = TrsmSmem<RL, false>::bytes, su = TrsmSmem<RL, true>::bytes, smem = sl > su ? sl : su;
+	static DeviceOnce attr;
+	HPLAI_TRY(attr.get([](int, int *) -> int {
+		HPLAI_CUDA_TRY(cudaFuncSetAttribute(trsm_pair_kernel<RL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			static_cast<int>(smem)));
+		return HPLAI_OK;
+	}));
+	const int vec = (reinterpret_cast<uintptr_t>(diag) & 15u) == 0 && lda % 4 == 0 && b % 4 == 0 ? 1 : 0;
+	trsm_pair_kernel<RL><<<dim3((rem + 32 * RL - 1) / (32 * RL), 2), kTrsmThreads, smem, st>>>(rem, b, diag, acol, arow,
+		lda, reinterpret_cast<__half *>(lh), reinterpret_cast<__half *>(uh), ldh, vec);
+	count_launches();
+	HPLAI_CUDA_TRY(cudaGetLastError());
+	return HPLAI_OK;
+}
+
+int launch_trsm_pair(int rem, int b, const float *diag, float *acol, float *arow, int64_t lda, uint16_t *lh,
+	uint16_t *uh, int64_t ldh, cudaStream_t st)
+{
+	if (rem <= 0) return HPLAI_OK;
+	if (b <= 0 || b > 1024 || !vec_ok(lh, ldh) || !vec_ok(uh, ldh)) return HPLAI_EINVAL;
+	if (rem > 64 * 74) return pair_launch<2>(rem, b, diag, acol, arow, lda, lh, uh, ldh, st);
+	return pair_launch<1>(rem, b, diag, acol, arow, lda, lh, uh, ldh, st);
 }
 
 } // namespace hplai

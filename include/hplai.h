@@ -82,7 +82,9 @@ typedef enum hplai_phase {
 /* hplai_create flags. */
 /* Panel TRSMs on CUDA cores in netlib strsm order -- bit-exact with the
  * reference's substitution -- instead of the default tensor-core path
- * (triangular inverses of the diagonal block applied in 3xTF32). */
+ * (triangular inverses of the diagonal block applied in 3xTF32).  The plain
+ * form takes the substitution for its small panels by default, both panels of
+ * a step in one launch, which is timed as HPLAI_PH_TRSM_L. */
 #define HPLAI_FLAG_SIMT_PANELS 1u
 /* One-step look-ahead on two streams: the next diagonal block and panels are
  * formed on a high-priority side stream while the main stream applies the

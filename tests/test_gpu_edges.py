@@ -74,6 +74,19 @@ def test_panel_solve_edges(hplai, oracle, torch_cuda, m, b, off):
     assert np.array_equal(h.cpu().numpy()[:, :b], ref.T.astype(np.float16))
 
 
+@pytest.mark.parametrize("n,b,flags", [(1200, 60, 0), (770, 70, 0), (1000, 125, 0), (1280, 128, 0), (2048, 512, 2),
+                                       (1200, 50, 2)])
+def test_small_panels_are_the_substitution_panels(hplai, torch_cuda, n, b, flags):
+    """Below the size rule the default panels are the bit-exact substitution (HPLAI_FLAG_SIMT_PANELS), both panels in
+    one launch: the same factors bit for bit, on one stream and with look-ahead."""
+    def lu(f):
+        with hplai.Solver(n, b, flags=f) as s:
+            s.generate(42)
+            s.factor()
+            return s.lu()
+    assert _same_bits(lu(flags), lu(flags | hplai.FLAG_SIMT_PANELS))
+
+
 @pytest.mark.parametrize("n,i0,j0,nr,nc,lda,off", [(1000, 3, 5, 1, 1, 1, 0), (1000, 0, 100, 127, 33, 127, 0),
                                                    (4000, 1, 7, 1023, 31, 1024, 0), (4000, 9, 0, 1025, 65, 1025, 0),
                                                    (4000, 0, 2000, 2050, 40, 2052, 1)])
