@@ -215,12 +215,14 @@ def run_reference(args):
     return 0
 
 
-def schur_algorithmic(n, b, panel_bytes=2, c_bytes=8, group=1):
+def schur_algorithmic(n, b, panel_bytes=2, c_bytes=8, group=1, side=None):
     """Flops, bytes and launches of all Schur updates of one factorisation,
     in the order hplai_factor issues them.  The update by a group of `group`
     panels (K = group * b) of the trailing matrix from block e on is split
-    into the next group's block columns, its block rows and the rest; with
-    panel groups a group's block e + j first receives the updates of the
+    into the next group's block columns, its block rows and the rest where the
+    next group's panels overlap it, else one launch (side: the schedule's SMs of
+    the side stream as hplai_set_schedule takes them, 0 for one stream; None:
+    every group split); with panel groups a group's block e + j first receives the updates of the
     group's panels e .. e + j - 1, each alone (K = b).  A region of m x n C
     elements with panel width K
     does 2 m n K flops and moves c_bytes per C element (8: FP32 read +
@@ -241,6 +243,12 @@ def schur_algorithmic(n, b, panel_bytes=2, c_bytes=8, group=1):
             region(n - j * b, b, b)
             region(b, n - (j + 1) * b, b)
 
+    def overlaps(e):
+        if side is None or side > 0:
+            return side is None or 2 * side <= 148
+        share = max(8, round(148 * -side / ((n - e * b) / b - side)))
+        return side < 0 and 2 * share <= 148
+
     for j in range(1, min(group, nb)):
         panel_updates(j, 0)
     s = 0
@@ -248,16 +256,21 @@ def schur_algorithmic(n, b, panel_bytes=2, c_bytes=8, group=1):
         e = s + group
         ne = min(group, nb - e)
         r1, r2, k = e * b, (e + ne) * b, group * b
-        region(n - r1, r2 - r1, k)
-        region(r2 - r1, n - r2, k)
+        whole = not overlaps(e) and b % 4 == 0
+        if whole:
+            region(n - r1, n - r1, k)
+        else:
+            region(n - r1, r2 - r1, k)
+            region(r2 - r1, n - r2, k)
         for j in range(e + 1, e + ne):
             panel_updates(j, e)
-        region(n - r2, n - r2, k)
+        if not whole:
+            region(n - r2, n - r2, k)
         s += group
     return acc["flops"], acc["bytes"], acc["launches"]
 
 
-def schur_traffic_per_launch(n, b, group=1, kind="fp16_fp32c"):
+def schur_traffic_per_launch(n, b, group=1, kind="fp16_fp32c", side=None):
     """DRAM bytes per average launch from the committed ncu summaries (DRAM
     bytes per updated C element of the kernel at the group's K: 2048 or 4096),
     times the C elements of one factorisation's launches (traffic grows with
@@ -270,7 +283,7 @@ def schur_traffic_per_launch(n, b, group=1, kind="fp16_fp32c"):
     d = d or kernels.get(kind)
     if not d:
         return None
-    _, byts, launches = schur_algorithmic(n, b, 0, 1, group)   # bytes = C elements
+    _, byts, launches = schur_algorithmic(n, b, 0, 1, group, side)   # bytes = C elements
     return d["dram_bytes_per_c_element"] * byts / launches
 
 
@@ -286,7 +299,7 @@ FORMS = {
 }
 
 
-def schur_roofline(hplai, n, b, fp8, deck, gemm_ms, group=1):
+def schur_roofline(hplai, n, b, fp8, deck, gemm_ms, group=1, side=None):
     """Roofline of the Schur GEMM over one factorisation: algorithmic flops
     and bytes per launch (schur_algorithmic) over the average launch time
     (CUDA events around each launch on its stream, summed by the library)."""
@@ -300,7 +313,7 @@ def schur_roofline(hplai, n, b, fp8, deck, gemm_ms, group=1):
         else:
             tc_sus *= 2.0
             peak_note += " x 2 for e4m3 (nominal e4m3:bf16 ratio; no measured e4m3 peak)"
-    sflops, sbytes, slaunch = schur_algorithmic(n, b, 1 if fp8 else 2, 4 if deck else 8, group)
+    sflops, sbytes, slaunch = schur_algorithmic(n, b, 1 if fp8 else 2, 4 if deck else 8, group, side)
     avg_launch_s = gemm_ms * 1e-3 / slaunch
     ach_gbs = sbytes / slaunch / avg_launch_s / 1e9
     ach_tf = sflops / slaunch / avg_launch_s / 1e12
@@ -314,7 +327,7 @@ def schur_roofline(hplai, n, b, fp8, deck, gemm_ms, group=1):
     cdesc = "FP16 deck, deck -= s*L*U" if deck else "FP32 C, C -= L*U"
     kname = f"schur_kernel (tcgen05 {'e4m3 x e4m3' if fp8 else 'FP16 x FP16'} -> FP32 accumulator; {cdesc})"
     kind = "e4m3_deck" if (fp8 and deck) else ("fp16_fp32c" if (not fp8 and not deck) else None)
-    traffic = schur_traffic_per_launch(n, b, group, kind) if kind else None
+    traffic = schur_traffic_per_launch(n, b, group, kind, side) if kind else None
     roof.update({"traffic": traffic, "kernel": kname,
                  "launches_per_step": slaunch, "avg_launch_ms": avg_launch_s * 1e3,
                  "algorithmic_bytes_per_launch": sbytes / slaunch, "algorithmic_flops_per_launch": sflops / slaunch,
@@ -386,6 +399,7 @@ class FormRun:
             return 4 if (f & hplai.FLAG_GROUP4) else 2 if (f & hplai.FLAG_GROUP2) else 1
         self.group = group_of(flags)
         sched_bits = hplai.FLAG_LOOKAHEAD | hplai.FLAG_GROUP2 | hplai.FLAG_GROUP4
+        self.side = side_sms if flags & hplai.FLAG_LOOKAHEAD else 0
         if lookahead:
             self.s.set_schedule(flags & sched_bits, side_sms)
         self.schedule = {"lookahead": bool(lookahead), "side_sms": side_sms if lookahead else None,
@@ -395,6 +409,7 @@ class FormRun:
             tflags, tside, tms = self.s.autotune(seed)
             la = bool(tflags & hplai.FLAG_LOOKAHEAD)
             self.group = group_of(tflags)
+            self.side = tside if la else 0
             def side_desc(f, sd):
                 if not (f & hplai.FLAG_LOOKAHEAD):
                     return None
@@ -440,7 +455,7 @@ class FormRun:
         steps = len(self.results)
         value, max_ms = replica_value(total_ms, steps * hpl_flops(self.n), world, device="cuda")
         phases = {k: statistics.mean(r[2][k] for r in self.results) for k in self.results[0][2]}
-        roof = schur_roofline(hplai, self.n, self.b, self.fp8, self.deck, phases["GEMM_UPDATE"], self.group)
+        roof = schur_roofline(hplai, self.n, self.b, self.fp8, self.deck, phases["GEMM_UPDATE"], self.group, self.side)
         last = self.results[-1]
         return {
             "form": self.form["label"], "value": value, "unit": UNIT, "steps": steps,

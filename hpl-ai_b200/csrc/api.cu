@@ -881,7 +881,9 @@ int factor_impl(hplai_ctx *c, int kend, const float *host_a = nullptr, int64_t h
 	// the group's second block first receiving its first panel's update.
 	// With HPLAI_FLAG_LOOKAHEAD they are formed on the side stream while the
 	// main stream applies the rest, which then leaves side_sms SMs to the
-	// side stream; otherwise everything runs in the same order on one stream.
+	// side stream.  Where nothing overlaps (one stream, or a share above one
+	// half) the update is one launch, ahead of the panels: the thin regions
+	// fill a fraction of the 128 x 256 tiles.
 	cudaStream_t st = c->st, sd = serial ? c->st : c->st2;
 	int sms = 148;
 	{
@@ -946,9 +948,17 @@ int factor_impl(hplai_ctx *c, int kend, const float *host_a = nullptr, int64_t h
 		const int side_ctas = side, main_ctas = side ? sms - side : 0;
 		HPLAI_CUDA_TRY(cudaEventRecord(c->ev_panel, sd));
 		HPLAI_CUDA_TRY(cudaStreamWaitEvent(st, c->ev_panel, 0));
-		// the next group's block columns (rows r1..n) and block rows (columns r2..n)
-		HPLAI_TRY(schur_region(c, op, r1, n, r1, r2, 0, st, pe));
-		HPLAI_TRY(schur_region(c, op, r1, r2, r2, n, 0, st, pe));
+		const bool whole = side == 0 && b % 4 == 0;
+		if (whole) {
+			// nothing to overlap with: the whole trailing matrix in one launch
+			// (rows of every region on 16-byte boundaries, so that its elements
+			// see the same epilogue as in the split update)
+			HPLAI_TRY(schur_region(c, op, r1, n, r1, n, 0, st, pe));
+		} else {
+			// the next group's block columns (rows r1..n) and block rows (columns r2..n)
+			HPLAI_TRY(schur_region(c, op, r1, n, r1, r2, 0, st, pe));
+			HPLAI_TRY(schur_region(c, op, r1, r2, r2, n, 0, st, pe));
+		}
 		HPLAI_CUDA_TRY(cudaEventRecord(c->ev_next, st));
 		HPLAI_CUDA_TRY(cudaStreamWaitEvent(sd, c->ev_next, 0));
 		for (int j = e; j < e + ne && j < kend; ++j) {
@@ -956,13 +966,13 @@ int factor_impl(hplai_ctx *c, int kend, const float *host_a = nullptr, int64_t h
 			HPLAI_TRY(prepare_block(c, j, e, q ^ 1, simt, side_ctas, sd, pe));
 			HPLAI_TRY(panel_step(c, j, q ^ 1, j - e, simt, side_ctas, sd, pe));
 		}
-		if (!serial && side == 0) {
+		if (!whole && !serial && side == 0) {
 			// no overlap for this group: its panels first, on the whole GPU
 			HPLAI_CUDA_TRY(cudaEventRecord(c->ev_panel, sd));
 			HPLAI_CUDA_TRY(cudaStreamWaitEvent(st, c->ev_panel, 0));
 		}
 		// the rest of the trailing matrix
-		HPLAI_TRY(schur_region(c, op, r2, n, r2, n, main_ctas, st, pe));
+		if (!whole) HPLAI_TRY(schur_region(c, op, r2, n, r2, n, main_ctas, st, pe));
 	}
 	HPLAI_CUDA_TRY(cudaEventRecord(c->ev_panel, sd));
 	HPLAI_CUDA_TRY(cudaStreamWaitEvent(st, c->ev_panel, 0));
