@@ -125,6 +125,7 @@ struct hplai_ctx {
 	cudaStream_t st = nullptr;    // main stream: Schur updates, refinement, everything else
 	cudaStream_t st2 = nullptr;   // side stream (high priority): diagonal block + panels
 	cudaEvent_t ev_panel = nullptr, ev_next = nullptr;
+	std::vector<cudaEvent_t> phase_events;   // PhaseEvents' pool
 	// host -> device copies of the matrix streamed behind the factorisation
 	// (hplai_solve_host with the FP16 deck): one event per panel's block
 	// column and row, created on first use
@@ -212,6 +213,7 @@ int ctx_free(hplai_ctx *c)
 	if (c->ev_panel) cudaEventDestroy(c->ev_panel);
 	if (c->ev_next) cudaEventDestroy(c->ev_next);
 	for (cudaEvent_t e : c->ev_copy) cudaEventDestroy(e);
+	for (cudaEvent_t e : c->phase_events) cudaEventDestroy(e);
 	if (c->st3) cudaStreamDestroy(c->st3);
 	if (c->st) cudaStreamDestroy(c->st);
 	if (c->st2) cudaStreamDestroy(c->st2);
@@ -230,32 +232,60 @@ int ctx_free(hplai_ctx *c)
 		}                                                                             \
 	} while (0)
 
-// Elapsed milliseconds between event pairs recorded around each phase.
+// Elapsed milliseconds between event pairs recorded around each phase.  The
+// events belong to the context and are reused by its next call: an event costs
+// the host as much as a launch, and a small solve is bound by its launches.
 struct PhaseEvents {
-	std::vector<cudaEvent_t> ev;
-	std::vector<int> phase;
-	int record(cudaStream_t st, int ph)
+	struct Span {
+		int phase;
+		cudaEvent_t begin, end;
+	};
+	std::vector<cudaEvent_t> &pool;
+	size_t used = 0;
+	std::vector<Span> spans;
+	// everything of this call runs on one stream, phase after phase: a phase
+	// begins where the last one ended
+	bool chained;
+	explicit PhaseEvents(std::vector<cudaEvent_t> &p, bool one_stream = false) : pool(p), chained(one_stream) {}
+	int take(cudaEvent_t *e)
 	{
-		cudaEvent_t a, b;
-		HPLAI_CUDA_TRY(cudaEventCreate(&a));
-		HPLAI_CUDA_TRY(cudaEventCreate(&b));
-		HPLAI_CUDA_TRY(cudaEventRecord(a, st));
-		ev.push_back(a);
-		ev.push_back(b);
-		phase.push_back(ph);
+		if (used == pool.size()) {
+			cudaEvent_t n;
+			HPLAI_CUDA_TRY(cudaEventCreate(&n));
+			pool.push_back(n);
+		}
+		*e = pool[used++];
 		return HPLAI_OK;
 	}
-	int end(cudaStream_t st) { return cudaEventRecord(ev.back(), st) == cudaSuccess ? HPLAI_OK : HPLAI_ECUDA; }
+	int record(cudaStream_t st, int ph)
+	{
+		Span sp{ph, nullptr, nullptr};
+		if (chained && !spans.empty()) {
+			sp.begin = spans.back().end;
+		} else {
+			HPLAI_TRY(take(&sp.begin));
+			HPLAI_CUDA_TRY(cudaEventRecord(sp.begin, st));
+		}
+		HPLAI_TRY(take(&sp.end));
+		spans.push_back(sp);
+		return HPLAI_OK;
+	}
+	int end(cudaStream_t st) { return cudaEventRecord(spans.back().end, st) == cudaSuccess ? HPLAI_OK : HPLAI_ECUDA; }
+	// ends the phase and begins the next one on the same stream, nothing between them
+	int next(cudaStream_t st, int ph)
+	{
+		HPLAI_TRY(end(st));
+		Span sp{ph, spans.back().end, nullptr};
+		HPLAI_TRY(take(&sp.end));
+		spans.push_back(sp);
+		return HPLAI_OK;
+	}
 	void collect(double *ms)
 	{
-		for (size_t i = 0; i < phase.size(); ++i) {
+		for (const Span &sp : spans) {
 			float t = 0.f;
-			if (cudaEventElapsedTime(&t, ev[2 * i], ev[2 * i + 1]) == cudaSuccess) ms[phase[i]] += t;
+			if (cudaEventElapsedTime(&t, sp.begin, sp.end) == cudaSuccess) ms[sp.phase] += t;
 		}
-	}
-	~PhaseEvents()
-	{
-		for (auto e : ev) cudaEventDestroy(e);
 	}
 };
 
@@ -565,8 +595,8 @@ int panel_step(hplai_ctx *c, int k, int buf, int slot, bool simt, int side_ctas,
 	float *diag = c->A + kb + kb * lda;
 	HPLAI_TRY(pe.record(st, HPLAI_PH_DIAG_LU));
 	HPLAI_TRY(launch_getrf_tiles(b, diag, lda, c->getrf_work, &c->getrf_epoch, side_ctas, st));
-	HPLAI_TRY(pe.end(st));
-	if (k == c->nb - 1) return HPLAI_OK;
+	if (k == c->nb - 1) return pe.end(st);
+	HPLAI_TRY(pe.next(st, HPLAI_PH_TRSM_L));
 	const int rem = n - static_cast<int>(kb) - b;
 	const bool f16_panels = f16_panel_form(c, simt);
 	const uint16_t *deck = f16_panels ? c->deck : nullptr;   // folded into the FP16 panel copies
@@ -598,7 +628,6 @@ int panel_step(hplai_ctx *c, int k, int buf, int slot, bool simt, int side_ctas,
 			al.base[1] = au.base[1] = (G - 1 - slot) * b;
 		}
 	}
-	HPLAI_TRY(pe.record(st, HPLAI_PH_TRSM_L));
 	if (simt) {
 		HPLAI_TRY(launch_trsm_right_upper(rem, b, diag, lda, diag + b, lda, lslot + (kb + b) * ldg, ldg, 1.0f, st));
 	} else if (f16_panels) {
@@ -624,8 +653,7 @@ int panel_step(hplai_ctx *c, int k, int buf, int slot, bool simt, int side_ctas,
 		uint16_t *lh = c->precision == HPLAI_F32_F8 ? nullptr : lslot + (kb + b) * ldg;
 		HPLAI_TRY(launch_lpanel_tc(c->tc, rem, diag + b, lda, lh, ldg, 1.0f, side_ctas, st));
 	}
-	HPLAI_TRY(pe.end(st));
-	HPLAI_TRY(pe.record(st, HPLAI_PH_TRSM_R));
+	HPLAI_TRY(pe.next(st, HPLAI_PH_TRSM_R));
 	if (simt) {
 		HPLAI_TRY(launch_trsm_left_lower(b, rem, diag, lda, diag + static_cast<int64_t>(b) * lda, lda,
 			uslot + (kb + b) * ldg, ldg, 1.0f, st));
@@ -792,7 +820,7 @@ int factor_refdeck(hplai_ctx *c, int kend)
 	const int64_t lda = c->lda, ldg = c->ldg;
 	cudaStream_t st = c->st;
 	for (double &v : c->phase_ms) v = 0.0;
-	PhaseEvents pe;
+	PhaseEvents pe(c->phase_events);
 	HPLAI_CUDA_TRY(cudaMemsetAsync(c->rdeck, 0, sizeof(uint16_t) * static_cast<size_t>(lda) * n, st));
 	if (c->rback) HPLAI_CUDA_TRY(cudaMemsetAsync(c->rback, 0, sizeof(uint16_t) * static_cast<size_t>(lda) * n, st));
 	HPLAI_CUDA_TRY(cudaMemsetAsync(c->getrf_work, 0, sizeof(uint32_t), st));   // its status word
@@ -871,7 +899,7 @@ int factor_impl(hplai_ctx *c, int kend, const float *host_a = nullptr, int64_t h
 	const bool simt = (c->flags & HPLAI_FLAG_SIMT_PANELS) != 0;
 	const bool serial = (c->flags & HPLAI_FLAG_LOOKAHEAD) == 0;
 	for (double &v : c->phase_ms) v = 0.0;
-	PhaseEvents pe;
+	PhaseEvents pe(c->phase_events, serial);
 	// Right-looking blocked LU without pivoting with look-ahead
 	// (panel_lu_async / RDMAPanelLU::run, panel_trf.hpp:434-858), by groups
 	// of G panels.  The update by group [s, s+G) of the trailing matrix
@@ -1207,7 +1235,7 @@ int refine_core(hplai_ctx *c, int mode, bool trans, const double *rhs, double no
 	if (iters) *iters = 0;
 	if (mode == HPLAI_GMRES) HPLAI_TRY(ensure_gmres_buffers(c));
 	HPLAI_TRY(trsv_status_reset(c->trsv_work, st));
-	PhaseEvents pe;
+	PhaseEvents pe(c->phase_events);
 	// x_0 = b ./ diag(A)   (iterative_refinement.hpp:31-34)
 	HPLAI_TRY(launch_div(n, rhs, c->d, x, st));
 	int rc = HPLAI_ENOTCONV;
