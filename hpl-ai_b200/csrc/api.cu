@@ -306,12 +306,16 @@ int compute_norms(hplai_ctx *c)
 
 // y <- beta y + alpha A x (A^T x with trans), A regenerated in FP64
 // (panel_gemv with Matgen<double> or HMGen<double>, panel_gemv.hpp:57-132)
-int matvec(hplai_ctx *c, double alpha, const double *x, double beta, double *y, cudaStream_t st, bool trans)
+// With y0, beta y0 instead of beta y; with norms, max |x_i|, max |y_i| and the
+// triangular solves' timeout word.
+int matvec(hplai_ctx *c, double alpha, const double *x, double beta, double *y, cudaStream_t st, bool trans,
+	const double *y0 = nullptr, double *norms = nullptr)
 {
 	if (c->matrix == HPLAI_MATRIX_HIGHAM)
 		return launch_higham_gemv(c->n, alpha, x, beta, y, c->h_alpha, c->h_beta, c->d, c->gemv_work, c->gemv_bytes, st,
-			trans);
-	return launch_otf_gemv(c->n, alpha, x, beta, y, c->seed, c->d, c->gemv_work, c->gemv_bytes, st, trans);
+			trans, y0, norms, trsv_status_word(c->trsv_work));
+	return launch_otf_gemv(c->n, alpha, x, beta, y, c->seed, c->d, c->gemv_work, c->gemv_bytes, st, trans, y0, norms,
+		trsv_status_word(c->trsv_work));
 }
 
 } // namespace
@@ -1239,17 +1243,18 @@ int refine_core(hplai_ctx *c, int mode, bool trans, const double *rhs, double no
 	// x_0 = b ./ diag(A)   (iterative_refinement.hpp:31-34)
 	HPLAI_TRY(launch_div(n, rhs, c->d, x, st));
 	int rc = HPLAI_ENOTCONV;
+	bool checked = true;   // the last correction's solves are known to have finished
 	for (int it = 0; it < maxit; ++it) {
-		HPLAI_CUDA_TRY(cudaMemcpyAsync(c->r, rhs, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-		HPLAI_TRY(launch_infnorm(n, x, c->scal + 2, st));
-		// r = b - A x with A regenerated in FP64 (panel_gemv(-1, ..., 1, r))
+		// r = b - A x with A regenerated in FP64 (panel_gemv(-1, ..., 1, r)), and
+		// ||x||_inf and ||r||_inf from the same pass
 		HPLAI_TRY(pe.record(st, HPLAI_PH_IR_GEMV));
-		HPLAI_TRY(matvec(c, -1.0, x, 1.0, c->r, st, trans));
+		HPLAI_TRY(matvec(c, -1.0, x, 1.0, c->r, st, trans, rhs, c->scal + 2));
 		HPLAI_TRY(pe.end(st));
-		HPLAI_TRY(launch_infnorm(n, c->r, c->scal + 3, st));
-		double h[2];
+		double h[3];
 		HPLAI_CUDA_TRY(cudaMemcpyAsync(h, c->scal + 2, sizeof h, cudaMemcpyDeviceToHost, st));
 		HPLAI_CUDA_TRY(cudaStreamSynchronize(st));
+		checked = true;
+		if (h[2] != 0.0) return HPLAI_ETIMEOUT;   // of the correction before
 		const double normx = h[0], normr = h[1];
 		// iterative_refinement.hpp:43
 		const double hpl = normr / std::fma(c->norma, normx, normb) * 1. / (n * DBL_EPSILON / 2);
@@ -1262,6 +1267,7 @@ int refine_core(hplai_ctx *c, int mode, bool trans, const double *rhs, double no
 			break;
 		}
 		if (!std::isfinite(hpl)) break;
+		checked = false;
 		if (mode == HPLAI_IR) {
 			HPLAI_TRY(correct_ir(c, x, pe, trans));
 		} else {
@@ -1270,11 +1276,12 @@ int refine_core(hplai_ctx *c, int mode, bool trans, const double *rhs, double no
 			c->gm_inner += in;
 			if (gr != HPLAI_OK) break;
 		}
-		int ts = HPLAI_OK;
-		HPLAI_TRY(trsv_status(c->trsv_work, st, &ts));
-		if (ts != HPLAI_OK) return ts;
 	}
+	uint32_t late = 0;
+	if (!checked)
+		HPLAI_CUDA_TRY(cudaMemcpyAsync(&late, trsv_status_word(c->trsv_work), sizeof late, cudaMemcpyDeviceToHost, st));
 	HPLAI_CUDA_TRY(cudaStreamSynchronize(st));
+	if (late) return HPLAI_ETIMEOUT;
 	double tmp[HPLAI_PH_COUNT] = {};
 	pe.collect(tmp);
 	c->phase_ms[HPLAI_PH_IR_GEMV] = tmp[HPLAI_PH_IR_GEMV];

@@ -217,11 +217,13 @@ int launch_deck_apply(int r0, int r1, int c0, int c1, float *a, int64_t lda, con
 size_t otf_gemv_workspace(int n);
 // trans: y <- beta*y + alpha*A^T x
 int launch_otf_gemv(int n, double alpha, const double *x, double beta, double *y, uint64_t seed,
-	const double *diag, void *work, size_t work_bytes, cudaStream_t st, bool trans = false);
+	const double *diag, void *work, size_t work_bytes, cudaStream_t st, bool trans = false, const double *y0 = nullptr,
+	double *norms = nullptr, const uint32_t *status = nullptr);
 // y <- beta y + alpha A x (A^T x with trans) over Higham's matrix with
 // parameters (halpha, hbeta), entries computed on the fly in FP64.
 int launch_higham_gemv(int n, double alpha, const double *x, double beta, double *y, double halpha, double hbeta,
-	const double *diag, void *work, size_t work_bytes, cudaStream_t st, bool trans);
+	const double *diag, void *work, size_t work_bytes, cudaStream_t st, bool trans, const double *y0 = nullptr,
+	double *norms = nullptr, const uint32_t *status = nullptr);
 int launch_otf_gemv_block(int64_t n, int mb, int nb, double alpha, const double *x, double *y, uint64_t state00,
 	void *work, size_t work_bytes, cudaStream_t st);
 size_t trsv_workspace(int n);
@@ -234,8 +236,9 @@ int launch_trsv(bool lower, int n, const float *a, int64_t lda, double *x, void 
 size_t trsv_dinv_doubles(int n);
 // blocks blk0 .. blk0 + nblk - 1 of 128 rows (nblk < 0: to the last)
 int launch_trsv_dinv(int n, const float *a, int64_t lda, double *dinv, cudaStream_t st, int blk0 = 0, int nblk = -1);
-int trsv_status(void *work, cudaStream_t st, int *status);
-// Clears the timeout word trsv_status reads.
+// The solves' timeout word (device address).
+const uint32_t *trsv_status_word(const void *work);
+// Clears it.
 int trsv_status_reset(void *work, cudaStream_t st);
 int launch_infnorm(int n, const double *x, double *out, cudaStream_t st);
 // panel_check: sigs (device, 3 doubles) = FP64 sums of |a_ij| over the

@@ -39,6 +39,26 @@ const JumpTable64 &table()
 	return t;
 }
 
+// max that propagates NaN, so a diverged vector cannot report a finite norm
+__device__ __forceinline__ double nan_max(double p, double q) { return (q != q || q > p) ? q : p; }
+
+// *out <- max(*out, the block's largest m); every thread calls it, at most 32
+// warps.  Non-negative doubles (and NaN above them) order like their bits.
+__device__ __forceinline__ void block_max(double m, double *out)
+{
+	__shared__ double wm[32];
+	for (int o = 16; o; o >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, o));
+	if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
+	__syncthreads();
+	if (threadIdx.x < 32) {
+		m = (threadIdx.x < (blockDim.x + 31) / 32) ? wm[threadIdx.x] : 0.0;
+		for (int o = 16; o; o >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, o));
+		if (threadIdx.x == 0)
+			atomicMax(reinterpret_cast<unsigned long long *>(out), static_cast<unsigned long long>(__double_as_longlong(m)));
+	}
+	__syncthreads();
+}
+
 // ---------------------------------------------------------------------------
 // On-the-fly GEMV.  CTA = 512/SPLIT rows x GEMV_COLS columns; the columns of
 // a chunk are divided into SPLIT pieces, and each thread walks two rows (32
@@ -63,7 +83,7 @@ constexpr int GEMV_COLS = 2048;
 template <bool TRANS, int SPLIT>
 __global__ void __launch_bounds__(GEMV_THREADS) otf_partial_kernel(int64_t n, int mb, int nb, double alpha,
 	const double *__restrict__ x, uint64_t state00, int with_diag, const double *__restrict__ diag,
-	double *__restrict__ part, JumpTable64 tab, Coeff jn)
+	double *__restrict__ part, JumpTable64 tab, Coeff jn, double *norms)
 {
 	constexpr int W = GEMV_THREADS / SPLIT / 32;   // warps that share a piece, 64 rows each
 	constexpr int R = 64 * W;
@@ -72,6 +92,7 @@ __global__ void __launch_bounds__(GEMV_THREADS) otf_partial_kernel(int64_t n, in
 	__shared__ Coeff stab[64];
 	__shared__ double fold[SPLIT > 1 ? SPLIT * R : 1];
 	const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+	if (norms && blockIdx.x == 0 && blockIdx.y == 0 && t < 2) norms[t] = 0.0;   // for otf_reduce_kernel
 	const int j0 = blockIdx.y * GEMV_COLS;
 	const int j1 = min(j0 + GEMV_COLS, nb);
 	for (int j = t; j < j1 - j0; j += GEMV_THREADS) xs[j] = x[j0 + j];
@@ -165,19 +186,33 @@ __global__ void __launch_bounds__(GEMV_THREADS) otf_partial_kernel(int64_t n, in
 	}
 }
 
-__global__ void otf_reduce_kernel(int mb, int nchunks, double beta, const double *__restrict__ part, double *y,
-	int overwrite)
+// y <- beta y0 + the chunks' sum (y0 may be y).  With `norms` (three doubles,
+// the first two zeroed by the kernel before), also max |x_i| and max |y_i|
+// into them and *status into the third, for the host to fetch in one copy.
+__global__ void __launch_bounds__(256) otf_reduce_kernel(int mb, int nchunks, double beta,
+	const double *__restrict__ part, const double *y0, double *y, int overwrite, const double *__restrict__ x,
+	double *norms, const uint32_t *status)
 {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= mb) return;
-	double s = 0.0;
-	for (int c = 0; c < nchunks; ++c) s += part[static_cast<int64_t>(c) * mb + i];
-	y[i] = overwrite ? s : fma(beta, y[i], s);
+	double r = 0.0, xv = 0.0;
+	if (i < mb) {
+		double s = 0.0;
+		for (int c = 0; c < nchunks; ++c) s += part[static_cast<int64_t>(c) * mb + i];
+		r = overwrite ? s : fma(beta, y0[i], s);
+		y[i] = r;
+		if (norms) xv = x[i];
+	}
+	if (norms) {
+		block_max(fabs(xv), norms);
+		block_max(fabs(r), norms + 1);
+		if (i == 0) norms[2] = status ? static_cast<double>(*status) : 0.0;
+	}
 }
 
 int otf_launch(int64_t n, int mb, int nb, double alpha, const double *x, double beta, double *y,
 	uint64_t state00, int with_diag, const double *diag, void *work, size_t work_bytes, cudaStream_t st,
-	bool trans = false)
+	bool trans = false, const double *y0 = nullptr, double *norms = nullptr,
+	const uint32_t *status = nullptr)
 {
 	if (mb <= 0) return HPLAI_OK;
 	const int nchunks = (nb + GEMV_COLS - 1) / GEMV_COLS;
@@ -190,10 +225,10 @@ int otf_launch(int64_t n, int mb, int nb, double alpha, const double *x, double 
 			const dim3 grid((mb + R - 1) / R, nchunks);
 			if (trans)
 				otf_partial_kernel<true, S><<<grid, GEMV_THREADS, 0, st>>>(n, mb, nb, alpha, x, state00, with_diag, diag,
-					part, table(), jn);
+					part, table(), jn, norms);
 			else
 				otf_partial_kernel<false, S><<<grid, GEMV_THREADS, 0, st>>>(n, mb, nb, alpha, x, state00, with_diag, diag,
-					part, table(), jn);
+					part, table(), jn, norms);
 		};
 		// Short pieces spread a small order over the SMs (n = 1200: 30 us in one
 		// piece, 13 in eight) and balance the last wave of a large one (32768: 434
@@ -207,8 +242,8 @@ int otf_launch(int64_t n, int mb, int nb, double alpha, const double *x, double 
 		count_launches();
 		HPLAI_CUDA_TRY(cudaGetLastError());
 	}
-	otf_reduce_kernel<<<(mb + 255) / 256, 256, 0, st>>>(mb, nb > 0 ? nchunks : 0, beta, part, y,
-		beta == 0.0 ? 1 : 0);
+	otf_reduce_kernel<<<(mb + 255) / 256, 256, 0, st>>>(mb, nb > 0 ? nchunks : 0, beta, part, y0 ? y0 : y, y,
+		beta == 0.0 ? 1 : 0, x, norms, status);
 	count_launches();
 	HPLAI_CUDA_TRY(cudaGetLastError());
 	return HPLAI_OK;
@@ -222,8 +257,9 @@ int otf_launch(int64_t n, int mb, int nb, double alpha, const double *x, double 
 // CTA shape, accumulators and fixed-order fold as the LCG GEMV.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(GEMV_ROWS) higham_partial_kernel(int n, double alpha, const double *__restrict__ x,
-	double ab, double cu, double cl, const double *__restrict__ diag, double *__restrict__ part)
+	double ab, double cu, double cl, const double *__restrict__ diag, double *__restrict__ part, double *norms)
 {
+	if (norms && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) norms[threadIdx.x] = 0.0;   // for otf_reduce_kernel
 	__shared__ double xs[GEMV_COLS];
 	__shared__ double ls[GEMV_COLS];
 	const int j0 = blockIdx.y * GEMV_COLS;
@@ -569,22 +605,11 @@ __global__ void __launch_bounds__(TRSV_THREADS, 1) trsv_kernel(int lower, int n,
 // ---------------------------------------------------------------------------
 // Vector helpers.
 // ---------------------------------------------------------------------------
-__global__ void infnorm_kernel(int n, const double *__restrict__ x, unsigned long long *out)
+__global__ void infnorm_kernel(int n, const double *__restrict__ x, double *out)
 {
-	// max that propagates NaN, so a diverged vector cannot report a finite norm
-	auto vmax = [](double p, double q) { return (q != q || q > p) ? q : p; };
 	double m = 0.0;
-	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = vmax(m, fabs(x[i]));
-	for (int o = 16; o; o >>= 1) m = vmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-	__shared__ double wm[32];
-	if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
-	__syncthreads();
-	if (threadIdx.x < 32) {
-		m = (threadIdx.x < (blockDim.x + 31) / 32) ? wm[threadIdx.x] : 0.0;
-		for (int o = 16; o; o >>= 1) m = vmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-		// non-negative doubles order like their bit patterns
-		if (threadIdx.x == 0) atomicMax(out, static_cast<unsigned long long>(__double_as_longlong(m)));
-	}
+	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = nan_max(m, fabs(x[i]));
+	block_max(m, out);
 }
 
 // Checksum of the factored matrix (panel_check.hpp:9-65): FP64 sums of
@@ -705,13 +730,16 @@ size_t otf_gemv_workspace(int n)
 }
 
 int launch_otf_gemv(int n, double alpha, const double *x, double beta, double *y, uint64_t seed, const double *diag,
-	void *work, size_t work_bytes, cudaStream_t st, bool trans)
+	void *work, size_t work_bytes, cudaStream_t st, bool trans, const double *y0, double *norms,
+	const uint32_t *status)
 {
-	return otf_launch(n, n, n, alpha, x, beta, y, state_initial(seed), 1, diag, work, work_bytes, st, trans);
+	return otf_launch(n, n, n, alpha, x, beta, y, state_initial(seed), 1, diag, work, work_bytes, st, trans, y0, norms,
+		status);
 }
 
 int launch_higham_gemv(int n, double alpha, const double *x, double beta, double *y, double halpha, double hbeta,
-	const double *diag, void *work, size_t work_bytes, cudaStream_t st, bool trans)
+	const double *diag, void *work, size_t work_bytes, cudaStream_t st, bool trans, const double *y0, double *norms,
+	const uint32_t *status)
 {
 	if (n <= 0) return HPLAI_OK;
 	const int nchunks = (n + GEMV_COLS - 1) / GEMV_COLS;
@@ -721,10 +749,11 @@ int launch_higham_gemv(int n, double alpha, const double *x, double beta, double
 	// A: upper constants -beta + ab i, lower -alpha + ab j; A^T the other way round
 	const double cu = trans ? -halpha : -hbeta, cl = trans ? -hbeta : -halpha;
 	higham_partial_kernel<<<dim3((n + GEMV_ROWS - 1) / GEMV_ROWS, nchunks), GEMV_ROWS, 0, st>>>(n, alpha, x, ab, cu, cl,
-		diag, part);
+		diag, part, norms);
 	count_launches();
 	HPLAI_CUDA_TRY(cudaGetLastError());
-	otf_reduce_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, nchunks, beta, part, y, beta == 0.0 ? 1 : 0);
+	otf_reduce_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, nchunks, beta, part, y0 ? y0 : y, y, beta == 0.0 ? 1 : 0, x,
+		norms, status);
 	count_launches();
 	HPLAI_CUDA_TRY(cudaGetLastError());
 	return HPLAI_OK;
@@ -785,7 +814,7 @@ int launch_trsv(bool lower, int n, const float *a, int64_t lda, double *x, void 
 	return HPLAI_OK;
 }
 
-// Clears the timeout word that trsv_status reads.
+// Clears the solves' timeout word.
 int trsv_status_reset(void *work, cudaStream_t st)
 {
 	TrsvWork *w = static_cast<TrsvWork *>(work);
@@ -817,15 +846,7 @@ int launch_trsv_dinv(int n, const float *a, int64_t lda, double *dinv, cudaStrea
 	return HPLAI_OK;
 }
 
-int trsv_status(void *work, cudaStream_t st, int *status)
-{
-	uint32_t v = 0;
-	TrsvWork *w = static_cast<TrsvWork *>(work);
-	HPLAI_CUDA_TRY(cudaMemcpyAsync(&v, &w->status, sizeof(v), cudaMemcpyDeviceToHost, st));
-	HPLAI_CUDA_TRY(cudaStreamSynchronize(st));
-	*status = v ? HPLAI_ETIMEOUT : HPLAI_OK;
-	return HPLAI_OK;
-}
+const uint32_t *trsv_status_word(const void *work) { return &static_cast<const TrsvWork *>(work)->status; }
 
 int launch_infnorm(int n, const double *x, double *out, cudaStream_t st)
 {
@@ -833,7 +854,7 @@ int launch_infnorm(int n, const double *x, double *out, cudaStream_t st)
 	if (n <= 0) return HPLAI_OK;
 	int blocks = (n + 255) / 256;
 	if (blocks > 1184) blocks = 1184;
-	infnorm_kernel<<<blocks, 256, 0, st>>>(n, x, reinterpret_cast<unsigned long long *>(out));
+	infnorm_kernel<<<blocks, 256, 0, st>>>(n, x, out);
 	count_launches();
 	HPLAI_CUDA_TRY(cudaGetLastError());
 	return HPLAI_OK;
