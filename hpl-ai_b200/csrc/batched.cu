@@ -25,9 +25,8 @@
 //
 // Step k (128-wide panels):
 //   getrf   one CTA per system, the 128 x 128 diagonal block in shared
-//           memory, unblocked right-looking LU with fmaf(-l_ik, u_kj, a_ij)
-//           and multipliers a_ik * (1 / u_kk): the operation sequence of
-//           getrf_nopiv (getrf_nopiv.hpp:30-46, 124-160), bit for bit;
+//           memory as 32 x 32 tiles, each element's operations in the order
+//           of getrf_nopiv (getrf_nopiv.hpp:30-46, 124-160), bit for bit;
 //   trsm    one CTA per 128-row (128-column) chunk of every system's L (U)
 //           panel, netlib strsm order (panel_trf.hpp:143-171), writing the
 //           FP32 panel and its FP16 copy;
@@ -39,6 +38,7 @@
 // one counter per step.
 #include "common.cuh"
 #include "internal.h"
+#include "tile.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -185,34 +185,58 @@ __global__ void __launch_bounds__(128) brhs_kernel(const BSys *__restrict__ sys,
 constexpr int kLdS = kBB + 1;   // shared-memory column pitch (bank-conflict free)
 constexpr int kLdT = kBB + 4;   // pitch of the TRSM triangle: rows of 16-byte aligned float4
 
-// The diagonal block (k, k) of system blockIdx.x (the active prefix).
-__global__ void __launch_bounds__(512) bgetrf_kernel(const BSys *__restrict__ sys, float *__restrict__ A, int64_t lda,
-	int k)
+// The diagonal block (k, k) of system blockIdx.x (the active prefix): 4 x 4
+// tiles of 32 x 32 in shared memory, two teams of four warps (tile.cuh).  The
+// chain is 128 pivots: after the panel tiles of step r are solved, one team
+// updates and factors the next diagonal tile while the other applies the
+// remaining updates.  512 systems' first blocks: 49 us (217 us as a rank-1
+// update of the whole block per pivot by 512 threads).
+constexpr int kGetrfThreads = 2 * tile::kTeam;
+constexpr int kNT = kBB / tile::T;
+__global__ void __launch_bounds__(kGetrfThreads) bgetrf_kernel(const BSys *__restrict__ sys, float *__restrict__ A,
+	int64_t lda, int k)
 {
-	extern __shared__ float sm[];
+	using namespace tile;
+	extern __shared__ __align__(16) float sm[];
+	__shared__ __align__(16) float xchs[2][kXchFloats];
 	const BSys S = sys[blockIdx.x];
 	float *blk = A + static_cast<int64_t>(k) * kBB + (S.C + static_cast<int64_t>(k) * kBB) * lda;
-	for (int e = threadIdx.x; e < kBB * kBB; e += 512) {
-		const int r = e % kBB, c = e / kBB;
-		sm[c * kLdS + r] = blk[r + static_cast<int64_t>(c) * lda];
-	}
+	const int team = threadIdx.x / kTeam;
+	const Team tm{static_cast<int>(threadIdx.x) % kTeam, static_cast<int>(threadIdx.x) & 31,
+		static_cast<int>(threadIdx.x) % kTeam / 32, 1 + team};
+	float *const xch = xchs[team];
+	float *Dt = sm, *D = sm + kTileFloats;   // the factored diagonal tile, row by row and column by column
+	float *const tiles = sm + 2 * kTileFloats;
+	auto at = [tiles](int ti, int tj) { return tiles + (ti + kNT * tj) * kTileFloats; };
+	for (int t = 0; t < kNT * kNT; ++t)
+		stage_tile(at(t % kNT, t / kNT), blk, lda, (t % kNT) * T, (t / kNT) * T, T, T, true, threadIdx.x, kGetrfThreads);
+	stage_wait();
 	__syncthreads();
-	for (int p = 0; p < kBB; ++p) {
-		// multipliers a_ip * (1 / u_pp), then the rank-1 update of the trailing block
-		const float inv = 1.0f / sm[p * kLdS + p];
-		for (int i = p + 1 + threadIdx.x; i < kBB; i += 512) sm[p * kLdS + i] *= inv;
+	if (team == 0) op_factor(tm, at(0, 0), D, Dt, xch, T);
+	__syncthreads();
+	for (int r = 0; r + 1 < kNT; ++r) {
+		const int w = kNT - 1 - r;
+		for (int t = 0; t < w; ++t) {
+			if (team == 0) op_solve_l(tm, at(r + 1 + t, r), Dt);
+			else op_solve_u(tm, at(r, r + 1 + t), D);
+		}
+		for (int e = threadIdx.x; e < kTileFloats; e += kGetrfThreads) at(r, r)[e] = D[e];
 		__syncthreads();
-		const int w = kBB - 1 - p;
-		for (int e = threadIdx.x; e < w * w; e += 512) {
-			const int i = p + 1 + e % w, j = p + 1 + e / w;
-			sm[j * kLdS + i] = fmaf(-sm[p * kLdS + i], sm[j * kLdS + p], sm[j * kLdS + i]);
+		if (team == 0) {
+			op_update(tm, at(r + 1, r + 1), at(r + 1, r), at(r, r + 1));
+			tm.sync();
+			op_factor(tm, at(r + 1, r + 1), D, Dt, xch, T);
+		} else {
+			for (int t = 1; t < w * w; ++t) {
+				const int ti = r + 1 + t % w, tj = r + 1 + t / w;
+				op_update(tm, at(ti, tj), at(ti, r), at(r, tj));
+			}
 		}
 		__syncthreads();
 	}
-	for (int e = threadIdx.x; e < kBB * kBB; e += 512) {
-		const int r = e % kBB, c = e / kBB;
-		blk[r + static_cast<int64_t>(c) * lda] = sm[c * kLdS + r];
-	}
+	for (int t = 0; t < kNT * kNT; ++t)
+		store_tile(t == kNT * kNT - 1 ? D : at(t % kNT, t / kNT), blk, lda, (t % kNT) * T, (t / kNT) * T, T, T,
+			threadIdx.x, kGetrfThreads);
 }
 
 // One 128-row chunk of a system's L panel below the diagonal block (side 0:
@@ -671,7 +695,7 @@ int upload(T **dst, const std::vector<T> &v)
 	return HPLAI_OK;
 }
 
-constexpr size_t kGetrfSmem = sizeof(float) * kBB * kLdS;
+constexpr size_t kGetrfSmem = sizeof(float) * (2 + kNT * kNT) * tile::kTileFloats;
 constexpr size_t kTrsmSmem = sizeof(float) * (kBB * kLdT + 2 * kBB);
 constexpr size_t kTrsvSmem = sizeof(float) * kBB * kLdS;
 
@@ -688,7 +712,7 @@ int enqueue_factor(BatchEngine *e)
 	for (int k = 0; k < e->nsteps; ++k) {
 		const int m = e->active[k];
 		if (m <= 0) break;
-		bgetrf_kernel<<<m, 512, kGetrfSmem, st>>>(e->dsys, e->A, e->lda, k);
+		bgetrf_kernel<<<m, kGetrfThreads, kGetrfSmem, st>>>(e->dsys, e->A, e->lda, k);
 		HPLAI_CUDA_TRY(cudaGetLastError());
 		++launches;
 		if (e->trsm_cnt[k] <= 0) continue;

@@ -119,3 +119,15 @@ def test_gemv_edges(hplai, oracle, torch_cuda, n):
         hplai.check(hplai.otf_gemv(n, -1.0, xd.data_ptr(), beta, yd.data_ptr(), 42, dd.data_ptr(), w.data_ptr(), ws, None))
         ref = beta * y0 - a @ x
         assert np.abs(yd.cpu().numpy() - ref).max() <= 1e-14 * (np.abs(a).sum(1).max() + 1)
+
+
+@pytest.mark.parametrize("n", [[2], [127, 129, 128], [640, 100, 36], [1500, 1536]])
+def test_batch_edges(hplai, oracle, torch_cuda, n):
+    """Orders around the 128-wide steps, one to eight right-hand sides."""
+    nrhs = [(3 * i + 8 - len(n)) % 8 + 1 for i in range(len(n))]
+    with hplai.Batch(n, nrhs, list(range(5, 5 + len(n)))) as bt:
+        assert bt.solve() == hplai.HPLAI_OK
+        for s, m in enumerate(n):
+            a = oracle.dense_matrix_f64(m, 5 + s)
+            ref = np.linalg.solve(a, oracle.rhs_cols(m, 5 + s, 0, nrhs[s]))
+            assert np.abs(bt.x(s) - ref).max() <= 1e-12 * np.abs(ref).max()
