@@ -250,50 +250,77 @@ __global__ void __launch_bounds__(kGetrfThreads) bgetrf_kernel(const BSys *__res
 // element sees the same updates in the same order as the netlib loops.
 // 256 threads; thread (lane, warp) holds 4 panel rows (side 0; columns for
 // side 1) 4 lane .. 4 lane + 3 times 16 elements 16 warp .. 16 warp + 15 in
-// registers, so the owner of step i is one warp and every other thread
-// updates 64 elements per step from two 16-byte shared-memory reads.
-// The 128 steps of one panel chunk.  Warp oi owns steps 16 oi .. 16 oi + 15
-// (its elements); within a warp's 16 steps the step index is a
-// compile-time constant, so the owner reads and scales its element directly
-// and a thread of a later warp updates all 16 of its elements unpredicated.
+// registers.
+// Bound by FP32 issue, so the 128 steps run 16 at a time: warp oi solves its
+// own 16 elements against the triangle alone, in registers, and publishes
+// them; after one barrier every later warp applies the 16 updates, 64 FMAs a
+// step from two 16-byte shared-memory reads, warp oi + 1 first of all going on
+// to its own solve.  512 systems' first panels: 343 us (661 with a barrier and
+// a publication per step, a quarter of the FP32 rate).  Within a warp's 16 steps every index is a compile-time
+// constant.
+constexpr int kMicro = 16;
+
 template <bool UPPER>
-__device__ __forceinline__ void trsm_steps(float (&b)[4][16], const float *tri, float *pub, int p0, int e0, int wp)
+__device__ __forceinline__ void trsm_steps(float (&b)[4][kMicro], const float *tri, const float *inv, float *pub,
+	int p0, int e0, int wp)
 {
-	for (int oi = 0; oi < 8; ++oi) {
+#pragma unroll 1
+	for (int oi = 0; oi < kBB / kMicro; ++oi) {
+		float *const pb = pub + (oi & 1) * kMicro * kBB + p0;
+		if (wp == oi) {
 #pragma unroll
-		for (int li = 0; li < 16; ++li) {
-			const int i = 16 * oi + li;
-			float *pb = pub + (li & 1) * kBB;
-			if (wp == oi) {
+			for (int li = 0; li < kMicro; ++li) {
+				const int i = kMicro * oi + li;
+				__syncwarp();   // keeps later steps' loads from being hoisted into too many registers
 				if (!UPPER) {
-					const float inv = 1.0f / tri[i * kLdT + i];
+					const float iv = inv[i];
 #pragma unroll
-					for (int r = 0; r < 4; ++r) b[r][li] = inv * b[r][li];
+					for (int r = 0; r < 4; ++r) b[r][li] = iv * b[r][li];
 				}
-				*reinterpret_cast<float4 *>(pb + p0) = make_float4(b[0][li], b[1][li], b[2][li], b[3][li]);
+				*reinterpret_cast<float4 *>(pb + li * kBB) = make_float4(b[0][li], b[1][li], b[2][li], b[3][li]);
+				const float4 *row = reinterpret_cast<const float4 *>(tri + i * kLdT + e0);
+#pragma unroll
+				for (int g = (li + 1) / 4; g < kMicro / 4; ++g) {
+					const float4 m4 = row[g];
+					const float mg[4] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+					for (int h = 0; h < 4; ++h) {
+						const int c = 4 * g + h;
+						if (c <= li) continue;
+						if (UPPER) {
+#pragma unroll
+							for (int r = 0; r < 4; ++r)
+								if (b[r][li] != 0.0f) b[r][c] = fmaf(-b[r][li], mg[h], b[r][c]);
+						} else if (mg[h] != 0.0f) {
+#pragma unroll
+							for (int r = 0; r < 4; ++r) b[r][c] = fmaf(-mg[h], b[r][li], b[r][c]);
+						}
+					}
+				}
 			}
-			__syncthreads();
-			if (wp < oi) continue;
-			const float4 b4 = *reinterpret_cast<const float4 *>(pb + p0);
-			const float bi[4] = {b4.x, b4.y, b4.z, b4.w};
-			const float4 *row = reinterpret_cast<const float4 *>(tri + i * kLdT + e0);
-			const int cfirst = (wp > oi) ? 0 : li + 1;   // a later warp: all 16; the owner: after li
+		}
+		__syncthreads();
+		if (wp > oi) {
+#pragma unroll 1
+			for (int li = 0; li < kMicro; ++li) {
+				const float4 b4 = *reinterpret_cast<const float4 *>(pb + li * kBB);
+				const float bi[4] = {b4.x, b4.y, b4.z, b4.w};
+				const float4 *row = reinterpret_cast<const float4 *>(tri + (kMicro * oi + li) * kLdT + e0);
 #pragma unroll
-			for (int g = 0; g < 4; ++g) {
-				if (wp == oi && 4 * g + 3 <= li) continue;
-				const float4 m4 = row[g];
-				const float mg[4] = {m4.x, m4.y, m4.z, m4.w};
+				for (int g = 0; g < kMicro / 4; ++g) {
+					const float4 m4 = row[g];
+					const float mg[4] = {m4.x, m4.y, m4.z, m4.w};
 #pragma unroll
-				for (int h = 0; h < 4; ++h) {
-					const int c = 4 * g + h;
-					if (c < cfirst) continue;
-					if (UPPER) {
+					for (int h = 0; h < 4; ++h) {
+						const int c = 4 * g + h;
+						if (UPPER) {
 #pragma unroll
-						for (int r = 0; r < 4; ++r)
-							if (bi[r] != 0.0f) b[r][c] = fmaf(-bi[r], mg[h], b[r][c]);
-					} else if (mg[h] != 0.0f) {
+							for (int r = 0; r < 4; ++r)
+								if (bi[r] != 0.0f) b[r][c] = fmaf(-bi[r], mg[h], b[r][c]);
+						} else if (mg[h] != 0.0f) {
 #pragma unroll
-						for (int r = 0; r < 4; ++r) b[r][c] = fmaf(-mg[h], bi[r], b[r][c]);
+							for (int r = 0; r < 4; ++r) b[r][c] = fmaf(-mg[h], bi[r], b[r][c]);
+						}
 					}
 				}
 			}
@@ -309,36 +336,82 @@ __global__ void __launch_bounds__(kTrsmThreads, 2) btrsm_kernel(const BSys *__re
 	extern __shared__ __align__(16) float sm[];
 	// side 0: tri[i * kLdT + j] = U(i, j) (rows of U); side 1: tri[i * kLdT + r] = L(r, i) (columns of L)
 	float *tri = sm;
-	float *pub = sm + kBB * kLdT;    // pub[2][128]: step i's final element of each panel row (column)
+	float *pub = sm + kBB * kLdT;    // pub[2][16][128]: 16 steps' final elements of each panel row (column)
+	float *inv = pub + 2 * kMicro * kBB;   // 1 / U(i, i)
 	const int4 it = items[blockIdx.x];
 	const BSys S = sys[it.x];
 	const bool upper = it.z != 0;
 	const int64_t kb = static_cast<int64_t>(k) * kBB;
 	const int64_t off = kb + kBB + static_cast<int64_t>(it.y) * kBB;   // first panel row / column
 	const float *diag = A + kb + (S.C + kb) * lda;
-	for (int e = threadIdx.x; e < kBB * kBB; e += kTrsmThreads) {
-		const int r = e % kBB, c = e / kBB;   // diag(r, c)
-		tri[upper ? c * kLdT + r : r * kLdT + c] = diag[r + static_cast<int64_t>(c) * lda];
+	// the triangle: each thread four rows of eight columns (side 0: transposed
+	// into rows of U, lanes along the columns), all loads in flight at once
+	{
+		float4 f[16];
+		const int t = threadIdx.x, c = upper ? t / 32 : t % 32, r4 = upper ? (t % 32) * 4 : (t / 32) * 4;
+#pragma unroll
+		for (int q = 0; q < 16; ++q) {
+			const int cc = upper ? c + 8 * q : c + 32 * (q & 3), rr = upper ? r4 : r4 + 32 * (q >> 2);
+			f[q] = *reinterpret_cast<const float4 *>(diag + rr + static_cast<int64_t>(cc) * lda);
+		}
+#pragma unroll
+		for (int q = 0; q < 16; ++q) {
+			const int cc = upper ? c + 8 * q : c + 32 * (q & 3), rr = upper ? r4 : r4 + 32 * (q >> 2);
+			if (upper) {
+				*reinterpret_cast<float4 *>(tri + cc * kLdT + rr) = f[q];
+			} else {
+				tri[rr * kLdT + cc] = f[q].x;
+				tri[(rr + 1) * kLdT + cc] = f[q].y;
+				tri[(rr + 2) * kLdT + cc] = f[q].z;
+				tri[(rr + 3) * kLdT + cc] = f[q].w;
+			}
+		}
 	}
 	const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
 	const int p0 = 4 * lane, e0 = 16 * wp;   // panel rows (columns) p0..p0+3, elements e0..e0+15
 	float b[4][16];
 	// element e of panel row p: side 0 A(off + p, kb + e); side 1 A(kb + e, off + p)
+	if (upper) {
 #pragma unroll
-	for (int r = 0; r < 4; ++r)
+		for (int r = 0; r < 4; ++r)
 #pragma unroll
-		for (int c = 0; c < 16; ++c)
-			b[r][c] = upper ? A[kb + e0 + c + (S.C + off + p0 + r) * lda] : A[off + p0 + r + (S.C + kb + e0 + c) * lda];
-	__syncthreads();
-	if (upper) trsm_steps<true>(b, tri, pub, p0, e0, wp);
-	else trsm_steps<false>(b, tri, pub, p0, e0, wp);
-#pragma unroll
-	for (int r = 0; r < 4; ++r) {
+			for (int q = 0; q < 4; ++q) {
+				const float4 v = *reinterpret_cast<const float4 *>(A + kb + e0 + 4 * q + (S.C + off + p0 + r) * lda);
+				b[r][4 * q] = v.x;
+				b[r][4 * q + 1] = v.y;
+				b[r][4 * q + 2] = v.z;
+				b[r][4 * q + 3] = v.w;
+			}
+	} else {
 #pragma unroll
 		for (int c = 0; c < 16; ++c) {
-			if (upper) A[kb + e0 + c + (S.C + off + p0 + r) * lda] = b[r][c];
-			else A[off + p0 + r + (S.C + kb + e0 + c) * lda] = b[r][c];
+			const float4 v = *reinterpret_cast<const float4 *>(A + off + p0 + (S.C + kb + e0 + c) * lda);
+			b[0][c] = v.x;
+			b[1][c] = v.y;
+			b[2][c] = v.z;
+			b[3][c] = v.w;
 		}
+	}
+	__syncthreads();
+	if (threadIdx.x < kBB) inv[threadIdx.x] = 1.0f / tri[threadIdx.x * kLdT + threadIdx.x];
+	__syncthreads();
+	if (upper) trsm_steps<true>(b, tri, inv, pub, p0, e0, wp);
+	else trsm_steps<false>(b, tri, inv, pub, p0, e0, wp);
+	if (upper) {
+#pragma unroll
+		for (int r = 0; r < 4; ++r)
+#pragma unroll
+			for (int q = 0; q < 4; ++q)
+				*reinterpret_cast<float4 *>(A + kb + e0 + 4 * q + (S.C + off + p0 + r) * lda) =
+					make_float4(b[r][4 * q], b[r][4 * q + 1], b[r][4 * q + 2], b[r][4 * q + 3]);
+	} else {
+#pragma unroll
+		for (int c = 0; c < 16; ++c)
+			*reinterpret_cast<float4 *>(A + off + p0 + (S.C + kb + e0 + c) * lda) =
+				make_float4(b[0][c], b[1][c], b[2][c], b[3][c]);
+	}
+#pragma unroll
+	for (int r = 0; r < 4; ++r) {
 		__half *o = (upper ? U16 : L16) + (S.R + off + p0 + r) * kBB + e0;
 #pragma unroll
 		for (int q = 0; q < 2; ++q) {
@@ -696,7 +769,7 @@ int upload(T **dst, const std::vector<T> &v)
 }
 
 constexpr size_t kGetrfSmem = sizeof(float) * (2 + kNT * kNT) * tile::kTileFloats;
-constexpr size_t kTrsmSmem = sizeof(float) * (kBB * kLdT + 2 * kBB);
+constexpr size_t kTrsmSmem = sizeof(float) * (kBB * kLdT + 2 * kMicro * kBB + kBB);
 constexpr size_t kTrsvSmem = sizeof(float) * kBB * kLdS;
 
 // Generation and factorisation of every system, in stream order.
