@@ -39,6 +39,7 @@
 #include "common.cuh"
 #include "internal.h"
 #include "tile.cuh"
+#include "tri_inv.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -182,7 +183,6 @@ __global__ void __launch_bounds__(128) brhs_kernel(const BSys *__restrict__ sys,
 // ---------------------------------------------------------------------------
 // Factorisation step k.
 // ---------------------------------------------------------------------------
-constexpr int kLdS = kBB + 1;   // shared-memory column pitch (bank-conflict free)
 constexpr int kLdT = kBB + 4;   // pitch of the TRSM triangle: rows of 16-byte aligned float4
 
 // The diagonal block (k, k) of system blockIdx.x (the active prefix): 4 x 4
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(256) bnorm_kernel(const BSys *__restrict__ sys
 // 128-row chunk below it is updated in parallel with that block column
 // (btrsv_off_kernel); the U pass does the same from each system's last block
 // up.  The steps of one correction are a CUDA graph.
-constexpr int kTrsvThreads = 256;   // 8 warps: one per right-hand side
+constexpr int kTrsvThreads = kTriThreads;
 
 __device__ __forceinline__ bool any_live(const BSys &S, const int *__restrict__ state)
 {
@@ -574,76 +574,75 @@ __device__ __forceinline__ bool any_live(const BSys &S, const int *__restrict__ 
 }
 
 // One CTA per system: its diagonal block (L pass: block t; U pass: block
-// nbk-1-t) staged in shared memory and solved by one warp per right-hand
-// side, the solved entry broadcast by shuffle (no block barrier inside).
+// nbk-1-t) inverted in FP64 in shared memory (invert_block: short chains over
+// all threads instead of 128 dependent steps of one warp) and applied as one
+// product, thread (row, half) taking every other right-hand side.  512
+// systems' blocks: 41 us (75 as a substitution, a warp per right-hand side).
 __global__ void __launch_bounds__(kTrsvThreads) btrsv_diag_kernel(const BSys *__restrict__ sys,
 	const float *__restrict__ A, int64_t lda, const int *__restrict__ state, double *__restrict__ r, int t, int up)
 {
-	extern __shared__ __align__(16) float blk[];   // blk[j * kLdS + i] = T(j0 + i, j0 + j)
+	extern __shared__ __align__(16) double inv[];
+	__shared__ double y[kMaxRhs][kBB];
 	const BSys S = sys[blockIdx.x];
 	const int n = S.n, nbk = (n + kBB - 1) / kBB;
 	if (t >= nbk || !any_live(S, state)) return;
 	const int jb = up ? nbk - 1 - t : t;
 	const int j0 = jb * kBB, w = min(kBB, n - j0);
-	const float *a = A + S.C * lda;
-	for (int e = threadIdx.x; e < kBB * kBB; e += kTrsvThreads) {
-		const int i = e % kBB, j = e / kBB;
-		blk[j * kLdS + i] = (i < w && j < w) ? a[j0 + i + static_cast<int64_t>(j0 + j) * lda] : 0.f;
+	double *rv = r + S.voff + j0;
+	for (int e = threadIdx.x; e < S.nrhs * kBB; e += kTrsvThreads) {
+		const int q = e / kBB, j = e % kBB;
+		y[q][j] = j < w ? rv[static_cast<int64_t>(q) * n + j] : 0.0;
 	}
-	__syncthreads();
-	const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	if (q >= S.nrhs || state[S.pair0 + q] != 0) return;
-	double *rv = r + S.voff + static_cast<int64_t>(q) * n + j0;
-	double v[4];
+	invert_block(inv, A + S.C * lda, lda, j0, w, up != 0);   // ends with a barrier
+	const int i = threadIdx.x % kBB, half = threadIdx.x / kBB;
+	double acc[kMaxRhs / 2] = {0.0, 0.0, 0.0, 0.0};
+	// row i of T^{-1}: X is T^{-1} for L, its transpose for U
+	const double *row = up ? inv + i : inv + i * kInvLd;
+	const int step = up ? kInvLd : 1;
+#pragma unroll 4
+	for (int j = 0; j < kBB; ++j) {
+		const double m = row[j * step];
 #pragma unroll
-	for (int m = 0; m < 4; ++m) {
-		const int i = lane + 32 * m;
-		v[m] = i < w ? rv[i] : 0.0;
+		for (int h = 0; h < kMaxRhs / 2; ++h)
+			if (2 * h < S.nrhs) acc[h] = fma(m, y[2 * h + half][j], acc[h]);
 	}
-	if (!up) {
-		// unit lower: y_j final in order, then y_i -= L(i, j) y_j for i > j
-		for (int j = 0; j < w; ++j) {
-			double vj = 0.0;
+	if (i >= w) return;
 #pragma unroll
-			for (int m = 0; m < 4; ++m)
-				if (m == (j >> 5)) vj = __shfl_sync(0xffffffffu, v[m], j & 31);
-#pragma unroll
-			for (int m = 0; m < 4; ++m) {
-				const int i = lane + 32 * m;
-				if (i > j && i < w) v[m] = fma(-static_cast<double>(blk[j * kLdS + i]), vj, v[m]);
-			}
-		}
-	} else {
-		// upper: y_j = v_j / U(j, j) from the last row up, then y_i -= U(i, j) y_j for i < j
-		for (int j = w - 1; j >= 0; --j) {
-#pragma unroll
-			for (int m = 0; m < 4; ++m)
-				if (m == (j >> 5) && lane == (j & 31)) v[m] = v[m] / static_cast<double>(blk[j * kLdS + j]);
-			double vj = 0.0;
-#pragma unroll
-			for (int m = 0; m < 4; ++m)
-				if (m == (j >> 5)) vj = __shfl_sync(0xffffffffu, v[m], j & 31);
-#pragma unroll
-			for (int m = 0; m < 4; ++m) {
-				const int i = lane + 32 * m;
-				if (i < j) v[m] = fma(-static_cast<double>(blk[j * kLdS + i]), vj, v[m]);
-			}
-		}
-	}
-#pragma unroll
-	for (int m = 0; m < 4; ++m) {
-		const int i = lane + 32 * m;
-		if (i < w) rv[i] = v[m];
+	for (int h = 0; h < kMaxRhs / 2; ++h) {
+		const int q = 2 * h + half;
+		if (q < S.nrhs && state[S.pair0 + q] == 0) rv[static_cast<int64_t>(q) * n + i] = acc[h];
 	}
 }
 
 // item = (system, chunk): 128 rows below (L pass) or above (U pass) the
-// block solved at step t take its update, r_i -= sum_j T(i, j0 + j) y_j,
-// one thread per row, every refining right-hand side at once.
-__global__ void __launch_bounds__(kBB) btrsv_off_kernel(const BSys *__restrict__ sys, const int2 *__restrict__ items,
-	const float *__restrict__ A, int64_t lda, const int *__restrict__ state, double *__restrict__ r, int t, int up)
+// block solved at step t take their update, r_i -= sum_j T(i, j0 + j) y_j,
+// every refining right-hand side at once.  Bound by the read of the factor:
+// thread (row, half) takes 64 of the 128 columns, eight loads in flight (52 us
+// against 57 with a thread per row and one load at a time).
+template <int NQ>
+__device__ __forceinline__ void off_row(const float *arow, int64_t lda, const double (*y)[kBB], int jb,
+	double (&acc)[kMaxRhs])
+{
+#pragma unroll 1
+	for (int j = 0; j < kBB / 2; j += 8) {
+		float l[8];
+#pragma unroll
+		for (int g = 0; g < 8; ++g) l[g] = __ldg(arow + static_cast<int64_t>(j + g) * lda);
+#pragma unroll
+		for (int g = 0; g < 8; ++g) {
+			const double v = l[g];
+#pragma unroll
+			for (int q = 0; q < NQ; ++q) acc[q] = fma(v, y[q][jb + j + g], acc[q]);
+		}
+	}
+}
+
+__global__ void __launch_bounds__(kTrsvThreads) btrsv_off_kernel(const BSys *__restrict__ sys,
+	const int2 *__restrict__ items, const float *__restrict__ A, int64_t lda, const int *__restrict__ state,
+	double *__restrict__ r, int t, int up)
 {
 	__shared__ double y[kMaxRhs][kBB];
+	__shared__ double fold[kMaxRhs][kBB];
 	const int2 it = items[blockIdx.x];
 	const BSys S = sys[it.x];
 	const int n = S.n, nq = S.nrhs, nbk = (n + kBB - 1) / kBB;
@@ -652,25 +651,41 @@ __global__ void __launch_bounds__(kBB) btrsv_off_kernel(const BSys *__restrict__
 	const int j0 = jb * kBB, w = min(kBB, n - j0);
 	const int rbase = up ? it.y * kBB : j0 + kBB + it.y * kBB;
 	double *rv = r + S.voff;
-	for (int e = threadIdx.x; e < kMaxRhs * kBB; e += kBB) {
+	// columns past n (the padding's identity) meet zeros
+	for (int e = threadIdx.x; e < nq * kBB; e += kTrsvThreads) {
 		const int q = e / kBB, j = e % kBB;
-		y[q][j] = (q < nq && j < w) ? rv[static_cast<int64_t>(q) * n + j0 + j] : 0.0;
+		y[q][j] = j < w ? rv[static_cast<int64_t>(q) * n + j0 + j] : 0.0;
 	}
 	__syncthreads();
-	const int i = rbase + threadIdx.x;
-	if (i >= (up ? j0 : n)) return;
-	const float *arow = A + i + (S.C + j0) * lda;
+	const int row = threadIdx.x % kBB, half = threadIdx.x / kBB;
+	const int i = rbase + row, c0 = half * (kBB / 2);
+	const bool in = i < (up ? j0 : n);
 	double acc[kMaxRhs];
 #pragma unroll
 	for (int q = 0; q < kMaxRhs; ++q) acc[q] = 0.0;
-	for (int j = 0; j < w; ++j) {
-		const double l = arow[static_cast<int64_t>(j) * lda];
+	if (in) {
+		const float *arow = A + i + (S.C + j0 + c0) * lda;
+		switch (nq) {
+		case 1: off_row<1>(arow, lda, y, c0, acc); break;
+		case 2: off_row<2>(arow, lda, y, c0, acc); break;
+		case 3: off_row<3>(arow, lda, y, c0, acc); break;
+		case 4: off_row<4>(arow, lda, y, c0, acc); break;
+		case 5: off_row<5>(arow, lda, y, c0, acc); break;
+		case 6: off_row<6>(arow, lda, y, c0, acc); break;
+		case 7: off_row<7>(arow, lda, y, c0, acc); break;
+		default: off_row<8>(arow, lda, y, c0, acc); break;
+		}
+	}
+	if (half == 1) {
 #pragma unroll
 		for (int q = 0; q < kMaxRhs; ++q)
-			if (q < nq) acc[q] = fma(l, y[q][j], acc[q]);
+			if (q < nq) fold[q][row] = acc[q];
 	}
-	for (int q = 0; q < nq; ++q)
-		if (state[S.pair0 + q] == 0) rv[static_cast<int64_t>(q) * n + i] -= acc[q];
+	__syncthreads();
+	if (half != 0 || !in) return;
+#pragma unroll
+	for (int q = 0; q < kMaxRhs; ++q)
+		if (q < nq && state[S.pair0 + q] == 0) rv[static_cast<int64_t>(q) * n + i] -= acc[q] + fold[q][row];
 }
 
 // x += r for the pairs still refining; item = (system, first row)
@@ -770,7 +785,7 @@ int upload(T **dst, const std::vector<T> &v)
 
 constexpr size_t kGetrfSmem = sizeof(float) * (2 + kNT * kNT) * tile::kTileFloats;
 constexpr size_t kTrsmSmem = sizeof(float) * (kBB * kLdT + 2 * kMicro * kBB + kBB);
-constexpr size_t kTrsvSmem = sizeof(float) * kBB * kLdS;
+constexpr size_t kTrsvSmem = kInvSmem<double>;
 
 // Generation and factorisation of every system, in stream order.
 int enqueue_factor(BatchEngine *e)
@@ -815,7 +830,7 @@ int enqueue_correction(BatchEngine *e, unsigned long long *launches)
 			HPLAI_CUDA_TRY(cudaGetLastError());
 			++nl;
 			if (e->off_cnt[t] > 0) {
-				btrsv_off_kernel<<<e->off_cnt[t], kBB, 0, st>>>(e->dsys, e->off_items + e->off_off[t], e->A, e->lda,
+				btrsv_off_kernel<<<e->off_cnt[t], kTrsvThreads, 0, st>>>(e->dsys, e->off_items + e->off_off[t], e->A, e->lda,
 					e->state, e->r, t, up);
 				HPLAI_CUDA_TRY(cudaGetLastError());
 				++nl;
