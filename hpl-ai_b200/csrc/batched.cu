@@ -106,20 +106,37 @@ namespace {
 __global__ void __launch_bounds__(256) bfill_kernel(const BSys *__restrict__ sys, const int2 *__restrict__ items,
 	float *__restrict__ A, int64_t lda, JumpT tab)
 {
+	__shared__ Coeff stab[64];
 	const int2 it = items[blockIdx.x];
 	const BSys S = sys[it.x];
 	const int c0 = it.y, c1 = min(c0 + 32, S.P);
-	const Coeff jn = jump(tab, static_cast<uint64_t>(S.n));
-	for (int i = threadIdx.x; i < S.P; i += 256) {
-		float *col = A + i + (S.C + c0) * lda;
-		if (i < S.n) {
-			uint64_t s = coeff_apply(jump(tab, static_cast<uint64_t>(i) + static_cast<uint64_t>(S.n) * c0), S.state0);
-			for (int c = c0; c < c1; ++c, col += lda) {
-				*col = c < S.n ? __double2float_rn(state_value(s)) : 0.f;
-				s = coeff_apply(jn, s);
+	const int t = threadIdx.x, lane = t & 31;
+	if (t < 64) stab[t] = tab.p[t];
+	__syncthreads();
+	const Coeff jn = warp_jump(stab, static_cast<uint64_t>(S.n));
+	// four neighbouring rows per thread (as fill_kernel), 16-byte stores
+	for (int rw = 4 * (t - lane); rw < S.P; rw += 4 * 256) {
+		const int r = rw + 4 * lane;
+		uint64_t s[4];
+		s[0] = coeff_apply(warp_jump(stab, static_cast<uint64_t>(rw) + static_cast<uint64_t>(S.n) * c0), S.state0);
+#pragma unroll
+		for (int k = 0; k < 5; ++k)
+			if ((lane >> k) & 1) s[0] = coeff_apply(stab[k + 2], s[0]);
+#pragma unroll
+		for (int q = 1; q < 4; ++q) s[q] = coeff_apply(Coeff{kLcgA, kLcgC}, s[q - 1]);
+#pragma unroll
+		for (int q = 0; q < 4; ++q) s[q] ^= 1ULL << 63;
+		if (r >= S.P) continue;   // P is a multiple of 4
+		float *col = A + r + (S.C + c0) * lda;
+		for (int c = c0; c < c1; ++c, col += lda) {
+			float v[4];
+#pragma unroll
+			for (int q = 0; q < 4; ++q) {
+				v[q] = r + q < S.n && c < S.n ? __double2float_rn(__dmul_rn(biased_state_value(s[q]), kValueScale))
+				     : r + q == c            ? 1.f : 0.f;
+				s[q] = coeff_apply(jn, s[q]);
 			}
-		} else {
-			for (int c = c0; c < c1; ++c, col += lda) *col = (c == i) ? 1.f : 0.f;
+			*reinterpret_cast<float4 *>(col) = make_float4(v[0], v[1], v[2], v[3]);
 		}
 	}
 }
@@ -140,24 +157,22 @@ __global__ void __launch_bounds__(128) bdiag_kernel(const BSys *__restrict__ sys
 	uint64_t s1 = coeff_apply(jn, s0);
 	uint64_t s2 = coeff_apply(jn, s1);
 	uint64_t s3 = coeff_apply(jn, s2);
+	auto value = [](uint64_t s) { return fabs(state_value(s)); };
 	double sum = 0.0;
 	int j = 0;
 	for (; j + 3 < n; j += 4) {
-		const double v0 = fabs(state_value(s0));
-		const double v1 = fabs(state_value(s1));
-		const double v2 = fabs(state_value(s2));
-		const double v3 = fabs(state_value(s3));
-		if (j != i) sum = __dadd_rn(sum, v0);
-		if (j + 1 != i) sum = __dadd_rn(sum, v1);
-		if (j + 2 != i) sum = __dadd_rn(sum, v2);
-		if (j + 3 != i) sum = __dadd_rn(sum, v3);
+		const double v0 = value(s0), v1 = value(s1), v2 = value(s2), v3 = value(s3);
 		s0 = coeff_apply(jn4, s0);
 		s1 = coeff_apply(jn4, s1);
 		s2 = coeff_apply(jn4, s2);
 		s3 = coeff_apply(jn4, s3);
+		if (j != i) sum = __dadd_rn(sum, v0);
+		if (j + 1 != i) sum = __dadd_rn(sum, v1);
+		if (j + 2 != i) sum = __dadd_rn(sum, v2);
+		if (j + 3 != i) sum = __dadd_rn(sum, v3);
 	}
 	for (; j < n; ++j) {
-		if (j != i) sum = __dadd_rn(sum, fabs(state_value(s0)));
+		if (j != i) sum = __dadd_rn(sum, value(s0));
 		s0 = coeff_apply(jn, s0);
 	}
 	d[S.doff + i] = sum;
@@ -450,10 +465,39 @@ __global__ void __launch_bounds__(128) bdiv_kernel(const BSys *__restrict__ sys,
 // columns times the generator scale, plus d_i x_i on the diagonal (the
 // on-the-fly GEMV of otf_gemv.cpp:5-131 / panel_gemv.hpp:16-180).  item =
 // (system, row block, column chunk).
+// Bound by the generator and FP64 issue: two LCG chains per row, and the loop
+// compiled for each number of right-hand sides (512 systems: 1163 us against
+// 1750 with one chain and a test per right-hand side).
+template <int NQ>
+__device__ __forceinline__ void gemv_row(const double (*xs)[kGemvCols], Coeff jn, uint64_t s0, int len, int dj,
+	double (&acc)[kMaxRhs])
+{
+	uint64_t s1 = coeff_apply(jn, s0);
+	const Coeff jn2 = coeff_mul(jn, jn);
+	int j = 0;
+	for (; j + 1 < len; j += 2) {
+		const double v0 = (j == dj) ? 0.0 : __ll2double_rn(static_cast<long long>(s0));
+		const double v1 = (j + 1 == dj) ? 0.0 : __ll2double_rn(static_cast<long long>(s1));
+#pragma unroll
+		for (int q = 0; q < NQ; ++q) {
+			const double2 x01 = *reinterpret_cast<const double2 *>(&xs[q][j]);
+			acc[q] = fma(v0, x01.x, acc[q]);
+			acc[q] = fma(v1, x01.y, acc[q]);
+		}
+		s0 = coeff_apply(jn2, s0);
+		s1 = coeff_apply(jn2, s1);
+	}
+	if (j < len) {
+		const double v0 = (j == dj) ? 0.0 : __ll2double_rn(static_cast<long long>(s0));
+#pragma unroll
+		for (int q = 0; q < NQ; ++q) acc[q] = fma(v0, xs[q][j], acc[q]);
+	}
+}
+
 __global__ void __launch_bounds__(kGemvRows) bgemv_kernel(const BSys *__restrict__ sys, const int4 *__restrict__ items,
 	const double *__restrict__ x, const double *__restrict__ d, double *__restrict__ part, JumpT tab)
 {
-	__shared__ double xs[kMaxRhs][kGemvCols];
+	__shared__ __align__(16) double xs[kMaxRhs][kGemvCols];
 	const int4 it = items[blockIdx.x];
 	const BSys S = sys[it.x];
 	const int i = it.y + threadIdx.x, c = it.z;
@@ -463,21 +507,26 @@ __global__ void __launch_bounds__(kGemvRows) bgemv_kernel(const BSys *__restrict
 	__syncthreads();
 	if (i >= S.n) return;
 	const Coeff jn = jump(tab, static_cast<uint64_t>(S.n));
-	uint64_t s = coeff_apply(jump(tab, static_cast<uint64_t>(i) + static_cast<uint64_t>(S.n) * j0), S.state0);
+	const uint64_t s = coeff_apply(jump(tab, static_cast<uint64_t>(i) + static_cast<uint64_t>(S.n) * j0), S.state0);
 	double acc[kMaxRhs];
 #pragma unroll
 	for (int q = 0; q < kMaxRhs; ++q) acc[q] = 0.0;
-	for (int j = 0; j < j1 - j0; ++j) {
-		const double v = (j0 + j == i) ? 0.0 : __ll2double_rn(static_cast<long long>(s));
-#pragma unroll
-		for (int q = 0; q < kMaxRhs; ++q)
-			if (q < S.nrhs) acc[q] = fma(v, xs[q][j], acc[q]);
-		s = coeff_apply(jn, s);
+	const int len = j1 - j0, dj = i >= j0 && i < j1 ? i - j0 : -1;
+	switch (S.nrhs) {
+	case 1: gemv_row<1>(xs, jn, s, len, dj, acc); break;
+	case 2: gemv_row<2>(xs, jn, s, len, dj, acc); break;
+	case 3: gemv_row<3>(xs, jn, s, len, dj, acc); break;
+	case 4: gemv_row<4>(xs, jn, s, len, dj, acc); break;
+	case 5: gemv_row<5>(xs, jn, s, len, dj, acc); break;
+	case 6: gemv_row<6>(xs, jn, s, len, dj, acc); break;
+	case 7: gemv_row<7>(xs, jn, s, len, dj, acc); break;
+	default: gemv_row<8>(xs, jn, s, len, dj, acc); break;
 	}
-	const bool dg = i >= j0 && i < j1;
-	for (int q = 0; q < S.nrhs; ++q) {
+#pragma unroll
+	for (int q = 0; q < kMaxRhs; ++q) {
+		if (q >= S.nrhs) break;
 		double r = acc[q] * kValueScale;
-		if (dg) r = fma(d[S.doff + i], xs[q][i - j0], r);
+		if (dj >= 0) r = fma(d[S.doff + i], xs[q][dj], r);
 		part[S.poff + (static_cast<int64_t>(c) * S.nrhs + q) * S.n + i] = r;
 	}
 }
