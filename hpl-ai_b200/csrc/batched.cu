@@ -18,9 +18,9 @@
 // row i, column C_s + j, with 128 unused columns after each system (the
 // last 256-column Schur tile of a step may reach past a system's columns).
 // A system's columns are contiguous in memory, so a 128-column block spans a
-// few pages.  Its L and U panels of step k are FP16 copies in two stacked
-// K-major buffers (row R_s + i of L16 = row i of L, row R_s + j of U16 =
-// column j of U).  Systems are ordered by decreasing P_s, so the systems
+// few pages.  Its L and U panels of a group of steps are FP16 copies in two
+// stacked K-major buffers (row R_s + i of L16 = row i of L, row R_s + j of U16
+// = column j of U).  Systems are ordered by decreasing P_s, so the systems
 // still factoring at step k are a prefix.
 //
 // Step k (128-wide panels):
@@ -31,7 +31,9 @@
 //           panel, netlib strsm order (panel_trf.hpp:143-171), writing the
 //           FP32 panel and its FP16 copy;
 //   schur   one persistent tcgen05 launch over the tiles of every system's
-//           trailing update (a tile table; TMA reduce-add into A).
+//           update (a tile table; TMA reduce-add into A): after a group's
+//           last panel the trailing matrix by the whole group, before that
+//           the next step's block column and row by the group's panels so far.
 // Refinement, per (system, right-hand side): x_0 = b ./ d, then residuals
 // with the matrix regenerated in FP64, the hpl-harness on the device, and
 // corrections x += U^-1 L^-1 r for the pairs still above 16; the host reads
@@ -51,6 +53,13 @@ namespace hplai {
 namespace {
 
 constexpr int kBB = 128;          // panel width
+// Panels per group: the trailing matrices are updated once per group, and a
+// block row and column inside the group, before its own step, by the group's
+// panels so far (still one update launch per step).  An update of K = 128 is
+// bound by the traffic of C: 512 systems' updates 16.5 ms one panel at a time,
+// 5.9 ms in groups of four.
+constexpr int kGroup = 4;
+constexpr int kLdK = kGroup * kBB;   // a panel row's FP16 copies: one slot of kBB per panel of the group
 constexpr int kGemvRows = 256;    // GEMV rows per CTA
 constexpr int kGemvCols = 512;    // GEMV columns per CTA (one partial-sum chunk)
 constexpr int kMaxRhs = 8;
@@ -427,7 +436,7 @@ __global__ void __launch_bounds__(kTrsmThreads, 2) btrsm_kernel(const BSys *__re
 	}
 #pragma unroll
 	for (int r = 0; r < 4; ++r) {
-		__half *o = (upper ? U16 : L16) + (S.R + off + p0 + r) * kBB + e0;
+		__half *o = (upper ? U16 : L16) + (S.R + off + p0 + r) * kLdK + (k % kGroup) * kBB + e0;
 #pragma unroll
 		for (int q = 0; q < 2; ++q) {
 			uint4 w;
@@ -858,7 +867,7 @@ int enqueue_factor(BatchEngine *e)
 		HPLAI_CUDA_TRY(cudaGetLastError());
 		++launches;
 		if (e->tile_cnt[k] > 0) {
-			HPLAI_TRY(launch_schur_tiles(e->maps, e->tiles + e->tile_off[k], e->tile_cnt[k], 0, st));
+			HPLAI_TRY(launch_schur_tiles(e->maps, e->tiles + e->tile_off[k], e->tile_cnt[k], (k % kGroup + 1) * kBB, 0, st));
 			++launches;
 		}
 	}
@@ -988,17 +997,25 @@ int batched_create(BatchEngine **out, int count, const int *n, const int *nrhs, 
 		}
 		e->trsm_cnt.push_back(static_cast<int>(trsm.size()) - e->trsm_off.back());
 	}
-	// tiles of step k: the trailing rows and columns from (k + 1) * 128 of every
-	// system still factoring, 128-row x 256-column tiles
+	// tiles after step k, 128 rows x 256 columns, of every system still
+	// factoring: with the group's last panel the trailing rows and columns from
+	// (k + 1) * 128, before that only the next step's block column and row
 	for (int k = 0; k < e->nsteps; ++k) {
 		e->tile_off.push_back(static_cast<int>(tiles.size()));
 		for (int i = 0; i < e->active[k]; ++i) {
 			const BSys &S = e->sys[i];
-			const int t0 = (k + 1) * kBB;
-			for (int c = t0; c < S.P; c += 256)
-				for (int rr = t0; rr < S.P; rr += kBB)
-					tiles.push_back(make_int4(static_cast<int>(S.R + rr), static_cast<int>(S.R + c), rr,
-						static_cast<int>(S.C + c)));
+			const int t0 = (k + 1) * kBB, t1 = t0 + kBB;
+			auto tile = [&](int rr, int c, bool half) {
+				const int col = static_cast<int>(S.C + c);
+				tiles.push_back(make_int4(static_cast<int>(S.R + rr), static_cast<int>(S.R + c), rr, half ? ~col : col));
+			};
+			if ((k + 1) % kGroup == 0) {
+				for (int c = t0; c < S.P; c += 256)
+					for (int rr = t0; rr < S.P; rr += kBB) tile(rr, c, c + kBB == S.P);
+			} else {
+				for (int rr = t0; rr < S.P; rr += kBB) tile(rr, t0, true);
+				for (int c = t1; c < S.P; c += 256) tile(t0, c, c + kBB == S.P);
+			}
 		}
 		e->tile_cnt.push_back(static_cast<int>(tiles.size()) - e->tile_off.back());
 	}
@@ -1015,8 +1032,8 @@ int batched_create(BatchEngine **out, int count, const int *n, const int *nrhs, 
 	};
 	if (rows > (int64_t(1) << 31) - 1 || cols > (int64_t(1) << 31) - 1) rc = HPLAI_EUNSUPPORTED;   // int tile coordinates
 	alloc(reinterpret_cast<void **>(&e->A), sizeof(float) * static_cast<size_t>(e->lda) * e->cols);
-	alloc(reinterpret_cast<void **>(&e->L16), sizeof(__half) * static_cast<size_t>(rows) * kBB);
-	alloc(reinterpret_cast<void **>(&e->U16), sizeof(__half) * static_cast<size_t>(rows) * kBB);
+	alloc(reinterpret_cast<void **>(&e->L16), sizeof(__half) * static_cast<size_t>(rows) * kLdK);
+	alloc(reinterpret_cast<void **>(&e->U16), sizeof(__half) * static_cast<size_t>(rows) * kLdK);
 	alloc(reinterpret_cast<void **>(&e->d), sizeof(double) * static_cast<size_t>(doff));
 	alloc(reinterpret_cast<void **>(&e->rhs), sizeof(double) * static_cast<size_t>(voff));
 	alloc(reinterpret_cast<void **>(&e->x), sizeof(double) * static_cast<size_t>(voff));
@@ -1044,7 +1061,7 @@ int batched_create(BatchEngine **out, int count, const int *n, const int *nrhs, 
 		rc = HPLAI_ECUDA;
 	if (rc == HPLAI_OK && cudaMemset(e->status, 0, sizeof(unsigned)) != cudaSuccess) rc = HPLAI_ECUDA;
 	if (rc == HPLAI_OK) rc = schur_make_maps(&e->maps, reinterpret_cast<const uint16_t *>(e->L16),
-		static_cast<int>(rows), kBB, reinterpret_cast<const uint16_t *>(e->U16), static_cast<int>(rows), kBB, kBB);
+		static_cast<int>(rows), kLdK, reinterpret_cast<const uint16_t *>(e->U16), static_cast<int>(rows), kLdK, kLdK);
 	if (rc == HPLAI_OK) rc = schur_set_cmap(&e->maps, e->A, e->pmax, static_cast<int>(e->cols), e->lda);
 	if (rc == HPLAI_OK && !e->maps.has_cmap) rc = HPLAI_EINVAL;
 	e->maps.status = e->status;

@@ -137,7 +137,7 @@ int launch_schur_deck(const SchurMaps &maps, bool fp8, const float *sl, int sl0,
 // schur_set_cmap with L rows tiles[t].x.. and U rows tiles[t].y.. (FP16
 // maps); a tile may reach past the columns of its system into columns nobody
 // reads (or past the matrix, where it is clipped).
-int launch_schur_tiles(const SchurMaps &maps, const int4 *tiles, int ntiles, int max_ctas, cudaStream_t st);
+int launch_schur_tiles(const SchurMaps &maps, const int4 *tiles, int ntiles, int k, int max_ctas, cudaStream_t st);
 int schur_status();          // the library's word: HPLAI_ETIMEOUT if a device wait ran out since the last reset
 void schur_status_reset();
 

@@ -136,6 +136,7 @@ struct Params {
 	// Batched form (FP16 operands, reduce epilogue): `ntiles` tiles whose L
 	// row, U row, C row and C column come from this table instead of the
 	// region's tile grid -- the tiles of many systems' updates in one launch.
+	// A column c given as ~c: only the tile's first 128 columns go to C.
 	const int4 *tiles;
 	int ntiles;
 	int group_m;        // tile rows per group of the tile order (tile_coords)
@@ -462,11 +463,12 @@ __global__ void __launch_bounds__(threads_for(EPI), 1) schur_kernel(const __grid
 		uint32_t acc_phase = 0;
 		int epi_buf = 0;
 		for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
-			int tm = 0, tn = 0, crow, ccol;
+			int tm = 0, tn = 0, crow, ccol, nch = BN / EPI_CHUNK;
 			if (p.tiles) {
 				const int4 t = p.tiles[tile];
 				crow = t.z;
-				ccol = t.w;
+				ccol = t.w < 0 ? ~t.w : t.w;
+				if (t.w < 0) nch /= 2;
 			} else {
 				tile_coords(tile, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
 				crow = p.crow0 + tm * BM;
@@ -489,7 +491,7 @@ __global__ void __launch_bounds__(threads_for(EPI), 1) schur_kernel(const __grid
 				// two 128-column halves (values past the region are exact zeros)
 				float vmax[2] = {0.f, 0.f};
 #pragma unroll 1
-				for (int ch = 0; ch < BN / EPI_CHUNK; ++ch) {
+				for (int ch = 0; ch < nch; ++ch) {
 					const int cc = ch * EPI_CHUNK;
 					float *sb = sEpi + (epi_buf % EPI_BUFS) * (BM * EPI_CHUNK);
 					// the reduce issued EPI_BUFS chunks ago read this buffer; let it finish
@@ -1187,15 +1189,15 @@ int launch_schur_deck(const SchurMaps &maps, bool fp8, const float *sl, int sl0,
 		true, dscale, max_ctas, st);
 }
 
-int launch_schur_tiles(const SchurMaps &maps, const int4 *tiles, int ntiles, int max_ctas, cudaStream_t st)
+int launch_schur_tiles(const SchurMaps &maps, const int4 *tiles, int ntiles, int k, int max_ctas, cudaStream_t st)
 {
 	if (ntiles <= 0) return HPLAI_OK;
-	if (!maps.has_cmap || !TALL || !tiles) return HPLAI_EINVAL;
+	if (!maps.has_cmap || !TALL || !tiles || k <= 0 || k > maps.k) return HPLAI_EINVAL;
 	Params p;
 	std::memset(&p, 0, sizeof p);
 	p.c = maps.cbase;
 	p.ldc = maps.cld;
-	p.num_kc = (maps.k + BK - 1) / BK;
+	p.num_kc = (k + BK - 1) / BK;
 	p.tiles = tiles;
 	p.ntiles = ntiles;
 	p.group_m = kGroupM;
