@@ -275,13 +275,14 @@ __global__ void __launch_bounds__(kGetrfThreads) bgetrf_kernel(const BSys *__res
 // 256 threads; thread (lane, warp) holds 4 panel rows (side 0; columns for
 // side 1) 4 lane .. 4 lane + 3 times 16 elements 16 warp .. 16 warp + 15 in
 // registers.
-// Bound by FP32 issue, so the 128 steps run 16 at a time: warp oi solves its
+// The 128 steps run 16 at a time: warp oi solves its
 // own 16 elements against the triangle alone, in registers, and publishes
 // them; after one barrier every later warp applies the 16 updates, 64 FMAs a
-// step from two 16-byte shared-memory reads, warp oi + 1 first of all going on
-// to its own solve.  512 systems' first panels: 343 us (661 with a barrier and
-// a publication per step, a quarter of the FP32 rate).  Within a warp's 16 steps every index is a compile-time
-// constant.
+// step from five 16-byte shared-memory reads, warp oi + 1 first of all going on
+// to its own solve.  Within a warp's 16 steps every index is a compile-time
+// constant.  512 systems: 343 us a launch on average (661 with a barrier and a
+// publication per step); the eight dependent solves set the time, not the FMA
+// pipe (24 %).
 constexpr int kMicro = 16;
 
 template <bool UPPER>

@@ -32,7 +32,8 @@ namespace hplai {
 // hc[(row0 + r)*ldh + j] = half(scale * X[r][j]) in both cases (the L copy is
 // row-major; the U copy stores column j of U as row j).
 //
-// Bound by FP32 issue.  A CTA owns 32 RL rows; a thread holds RL rows (lane,
+// Bound by the chain of 16-column solves, and by FP32 issue and the operands'
+// shared-memory reads in the products.  A CTA owns 32 RL rows; a thread holds RL rows (lane,
 // lane + 32) of 16 columns (its warp's) of a 128-column block in registers.
 // Per block: the products with the columns solved before (X and T in chunks
 // of 32 p through three cp.async stages), then the block's own triangle 16

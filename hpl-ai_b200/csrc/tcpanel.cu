@@ -287,9 +287,9 @@ __device__ __forceinline__ float tri_t(const float *lu, int64_t lda, int b, int 
 }
 
 // grid (128-blocks, 2): blockIdx.y = 0 -> U11, 1 -> L11^T.  Latency-bound: one
-// launch (TRIBLK) in place of a one-warp substitution per 32 x 32 tile and the products
-// of the h = 32 and 64 levels.  With one block in all (hi given) its TF32
-// split follows here as well.
+// launch (17 us at b = 1024, 18 at 240) in place of a one-warp substitution per
+// 32 x 32 tile and the products of the h = 32 and 64 levels, each a launch.
+// With one block in all (hi given) its TF32 split follows here as well.
 __global__ void __launch_bounds__(kTriThreads) tri_block_kernel(int b, int bp, const float *__restrict__ lu,
 	int64_t lda, float *__restrict__ xu, float *__restrict__ xl, int64_t ldp, float *__restrict__ uhi,
 	float *__restrict__ ulo, float *__restrict__ lhi, float *__restrict__ llo)
