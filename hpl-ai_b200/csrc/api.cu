@@ -114,9 +114,10 @@ struct hplai_ctx {
 	double *rhs = nullptr, *d = nullptr, *x = nullptr, *r = nullptr, *scal = nullptr;
 	void *gemv_work = nullptr;
 	size_t gemv_bytes = 0;
+	uint8_t *zeroed = nullptr;    // one allocation, zeroed once: kstatus, trsv_work, getrf_work
 	void *trsv_work = nullptr;
 	size_t trsv_bytes = 0;
-	void *getrf_work = nullptr;   // tile flags of the diagonal block LU
+	void *getrf_work = nullptr;   // tagged tiles of the diagonal block LU
 	void *check_work = nullptr;   // hplai_checksum: per-CTA partial sums, then the three results
 	double *dinv = nullptr;       // FP64 inverses of the factors' 128 x 128 diagonal blocks
 	unsigned *kstatus = nullptr;  // timeout words of this context's Schur [0] and panel [1] kernels
@@ -198,11 +199,9 @@ int ctx_free(hplai_ctx *c)
 	cudaFree(c->r);
 	cudaFree(c->scal);
 	cudaFree(c->gemv_work);
-	cudaFree(c->trsv_work);
-	cudaFree(c->getrf_work);
+	cudaFree(c->zeroed);
 	cudaFree(c->check_work);
 	cudaFree(c->dinv);
-	cudaFree(c->kstatus);
 	cudaFree(c->f16s);
 	cudaFree(c->gm_v);
 	cudaFree(c->gm_z);
@@ -453,15 +452,16 @@ extern "C" int hplai_create(hplai_ctx **out, int n, int b, int precision, unsign
 	c->gemv_bytes = otf_gemv_workspace(n);
 	CTX_ALLOC(c->gemv_work, c->gemv_bytes);
 	c->trsv_bytes = trsv_workspace(n);
-	CTX_ALLOC(c->trsv_work, c->trsv_bytes);
-	CTX_ALLOC(c->getrf_work, getrf_workspace(b));
+	const size_t at_trsv = 256, at_getrf = at_trsv + round_up(static_cast<int64_t>(c->trsv_bytes), 256);
+	const size_t zeroed_bytes = at_getrf + getrf_workspace(b);
+	CTX_ALLOC(c->zeroed, zeroed_bytes);
+	c->kstatus = reinterpret_cast<unsigned *>(c->zeroed);
+	c->trsv_work = c->zeroed + at_trsv;
+	c->getrf_work = c->zeroed + at_getrf;
 	CTX_ALLOC(c->check_work, panel_check_workspace(n) + 3 * sizeof(double));
 	CTX_ALLOC(c->dinv, sizeof(double) * trsv_dinv_doubles(n));
-	CTX_ALLOC(c->kstatus, 2 * sizeof(unsigned));
 	CTX_ALLOC(c->f16s, 4 * sizeof(unsigned));
-	if (cudaMemset(c->trsv_work, 0, c->trsv_bytes) != cudaSuccess ||
-		cudaMemset(c->getrf_work, 0, getrf_workspace(b)) != cudaSuccess ||
-		cudaMemset(c->kstatus, 0, 2 * sizeof(unsigned)) != cudaSuccess ||
+	if (cudaMemset(c->zeroed, 0, zeroed_bytes) != cudaSuccess ||
 		cudaMemset(c->tcbuf, 0, sizeof(float) * tc_elems) != cudaSuccess) {
 		ctx_free(c);
 		return HPLAI_ECUDA;
