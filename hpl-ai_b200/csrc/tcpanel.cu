@@ -266,8 +266,8 @@ __global__ void __launch_bounds__(256) tri_f16_kernel(int b, const float *__rest
 // ---------------------------------------------------------------------------
 // Triangular inverses by recursive doubling.  X = T^{-1}, T upper triangular
 // and padded with the identity to bp = ldp rows/columns:
-//   TRANS_T = false: T = U11, T[p][j] at lu[j*lda + p], non-unit diagonal
-//   TRANS_T = true : T = L11^T, T[p][j] = L[j][p] at lu[p*lda + j], unit diagonal
+//   U11:   T[p][j] at lu[j*lda + p], non-unit diagonal
+//   L11^T: T[p][j] = L[j][p] at lu[p*lda + j], unit diagonal
 // The 128 x 128 diagonal blocks are inverted by one CTA each in shared memory
 // (invert_block).  Then level by level pairs of inverted blocks of h = 128,
 // 256, 512 are joined,
@@ -277,15 +277,6 @@ __global__ void __launch_bounds__(256) tri_f16_kernel(int b, const float *__rest
 // is built in place; its strictly lower part stays zero.
 // A final pass writes the hi/lo TF32 split of X for the tensor-core panels.
 // ---------------------------------------------------------------------------
-template <bool TRANS_T>
-__device__ __forceinline__ float tri_t(const float *lu, int64_t lda, int b, int p, int j)
-{
-	if (p >= b || j >= b) return (p == j) ? 1.f : 0.f;
-	if (p > j) return 0.f;
-	if (TRANS_T) return (p == j) ? 1.f : lu[static_cast<int64_t>(p) * lda + j];
-	return lu[static_cast<int64_t>(j) * lda + p];
-}
-
 // grid (128-blocks, 2): blockIdx.y = 0 -> U11, 1 -> L11^T.  Latency-bound: one
 // launch (17 us at b = 1024, 18 at 240) in place of a one-warp substitution per
 // 32 x 32 tile and the products of the h = 32 and 64 levels, each a launch.
@@ -320,14 +311,18 @@ __global__ void __launch_bounds__(kTriThreads) tri_block_kernel(int b, int bp, c
 // output tiles of an h x h block (clipped), grid.y = pair, grid.z = triangle.
 //   STEP 0: W[o:o+h, o+h:o+h+h2] = T[o:o+h, o+h:..] X[o+h:.., o+h:..]
 //   STEP 1: X[o:o+h, o+h:..]     = -X[o:o+h, o:o+h] W[o:o+h, o+h:..]
-// K runs in chunks of 32; the next chunk is loaded into registers while the
-// current one is multiplied from shared memory.
+// K runs in chunks of 32 through three asynchronous stages: a tile's chunks are
+// few and dependent, so their loads' latency and the shared-memory reads set
+// the time (a thread has 4 rows x 2 columns, six 16-byte reads per 32 FMAs;
+// b = 1024, a level: 21.5 + 18.0 us with one chunk ahead and scalar reads, now
+// 15.0 + 12.1; b = 240 8.1 + 7.6, now 4.8 + 4.3).
+// h, bp and ldp are multiples of 32, so every tile is whole.
 template <int STEP>
 __global__ void __launch_bounds__(128) tri_level_kernel(int b, int bp, int h, const float *__restrict__ lu, int64_t lda,
 	float *__restrict__ xu, float *__restrict__ xl, float *__restrict__ wu, float *__restrict__ wl, int64_t ldp)
 {
-	__shared__ float As[2][32][33];   // [buffer][k][row]
-	__shared__ float Bs[2][32][33];   // [buffer][k][col]
+	__shared__ __align__(16) float As[3][32][36];   // [stage][k][row]
+	__shared__ __align__(16) float Bs[3][32][36];   // [stage][column][k]
 	const bool lower = blockIdx.z != 0;
 	float *x = lower ? xl : xu;
 	float *w = lower ? wl : wu;
@@ -348,73 +343,69 @@ __global__ void __launch_bounds__(128) tri_level_kernel(int b, int bp, int h, co
 	// B element (k, col) is contiguous along k.  Consecutive threads take the
 	// contiguous index so every load is coalesced.
 	const bool a_k_fast = (STEP == 0) && lower;
-	float ra[8], rb[8];
-	auto load = [&](int k0) {
+	auto copy4 = [](float *dst, const float *src, bool in) {
+		asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 4 : 0) : "memory");
+	};
+	auto stage = [&](int st, int k0) {
+		if (k0 < k_end) {
 #pragma unroll
-		for (int q = 0; q < 8; ++q) {
-			const int e = tid + 128 * q;
-			const int r = a_k_fast ? (e >> 5) : (e & 31), kk = a_k_fast ? (e & 31) : (e >> 5);
-			const int k = k0 + kk, row = row0 + r;
-			float av = 0.f;
-			if (k < k_end && row < rend) {
-				if (STEP == 0)
-					av = lower ? tri_t<true>(lu, lda, b, row, k) : tri_t<false>(lu, lda, b, row, k);
-				else
-					av = x[static_cast<int64_t>(k) * ldp + row];
+			for (int q = 0; q < 8; ++q) {
+				const int e = tid + 128 * q;
+				const int r = a_k_fast ? (e >> 5) : (e & 31), kk = a_k_fast ? (e & 31) : (e >> 5);
+				const int k = k0 + kk, row = row0 + r;
+				if (STEP == 0) {   // off the diagonal: zero where the padding is
+					const bool in = row < b && k < b;
+					copy4(&As[st][kk][r], in ? lu + (lower ? static_cast<int64_t>(row) * lda + k : static_cast<int64_t>(k) * lda + row) : lu, in);
+				} else {
+					copy4(&As[st][kk][r], x + static_cast<int64_t>(k) * ldp + row, true);
+				}
+				const int kb = e & 31, cc = e >> 5;
+				copy4(&Bs[st][cc][kb], (STEP == 0 ? x : w) + static_cast<int64_t>(col0 + cc) * ldp + k0 + kb, true);
 			}
-			ra[q] = av;
-			const int kb = e & 31, cc = e >> 5;
-			const int kq = k0 + kb, col = col0 + cc;
-			float bv = 0.f;
-			if (kq < k_end && col < cend)
-				bv = (STEP == 0) ? x[static_cast<int64_t>(col) * ldp + kq] : w[static_cast<int64_t>(col) * ldp + kq];
-			rb[q] = bv;
 		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
 	};
-	auto stash = [&](int buf) {
-#pragma unroll
-		for (int q = 0; q < 8; ++q) {
-			const int e = tid + 128 * q;
-			const int r = a_k_fast ? (e >> 5) : (e & 31), kk = a_k_fast ? (e & 31) : (e >> 5);
-			As[buf][kk][r] = ra[q];
-			Bs[buf][e & 31][e >> 5] = rb[q];
-		}
-	};
-	// thread: output column `c`, rows 8g .. 8g+7
-	const int c = tid & 31, g = tid >> 5;
-	float acc[8] = {};
+	// thread: rows r4 .. r4 + 3, columns c2, c2 + 1
+	const int r4 = 4 * (tid & 7), c2 = 2 * (tid >> 3);
+	float acc[2][4] = {};
+	stage(0, k_begin);
+	stage(1, k_begin + 32);
 	int buf = 0;
-	if (k_begin < k_end) {
-		load(k_begin);
-		stash(0);
-	}
-	__syncthreads();
 	for (int k0 = k_begin; k0 < k_end; k0 += 32) {
-		const bool more = k0 + 32 < k_end;
-		if (more) load(k0 + 32);
+		asm volatile("cp.async.wait_group 1;" ::: "memory");
+		__syncthreads();   // the chunk is here; everyone is done with the one before it
+		stage(buf == 0 ? 2 : buf - 1, k0 + 64);
 #pragma unroll
-		for (int kk = 0; kk < 32; ++kk) {
-			const float bv = Bs[buf][kk][c];
+		for (int kk = 0; kk < 32; kk += 4) {
+			float bv[2][4];
 #pragma unroll
-			for (int i = 0; i < 8; ++i) acc[i] = fmaf(As[buf][kk][8 * g + i], bv, acc[i]);
+			for (int j = 0; j < 2; ++j) {
+				const float4 v = *reinterpret_cast<const float4 *>(&Bs[buf][c2 + j][kk]);
+				bv[j][0] = v.x;
+				bv[j][1] = v.y;
+				bv[j][2] = v.z;
+				bv[j][3] = v.w;
+			}
+#pragma unroll
+			for (int k = 0; k < 4; ++k) {
+				const float4 v = *reinterpret_cast<const float4 *>(&As[buf][kk + k][r4]);
+#pragma unroll
+				for (int j = 0; j < 2; ++j) {
+					acc[j][0] = fmaf(v.x, bv[j][k], acc[j][0]);
+					acc[j][1] = fmaf(v.y, bv[j][k], acc[j][1]);
+					acc[j][2] = fmaf(v.z, bv[j][k], acc[j][2]);
+					acc[j][3] = fmaf(v.w, bv[j][k], acc[j][3]);
+				}
+			}
 		}
-		if (more) stash(buf ^ 1);
-		__syncthreads();
-		buf ^= 1;
+		buf = buf == 2 ? 0 : buf + 1;
 	}
-	// write through shared memory so the stores run along the rows
 	float *out = (STEP == 0) ? w : x;
 	const float sgn = (STEP == 0) ? 1.f : -1.f;
 #pragma unroll
-	for (int i = 0; i < 8; ++i) As[0][c][8 * g + i] = sgn * acc[i];
-	__syncthreads();
-#pragma unroll
-	for (int q = 0; q < 8; ++q) {
-		const int e = tid + 128 * q;
-		const int r = e & 31, cc = e >> 5;
-		const int row = row0 + r, col = col0 + cc;
-		if (row < rend && col < cend) out[static_cast<int64_t>(col) * ldp + row] = As[0][cc][r];
-	}
+	for (int j = 0; j < 2; ++j)
+		*reinterpret_cast<float4 *>(out + static_cast<int64_t>(col0 + c2 + j) * ldp + row0 + r4) =
+			make_float4(sgn * acc[j][0], sgn * acc[j][1], sgn * acc[j][2], sgn * acc[j][3]);
 }
 
 // X (work, ldp x ldp) -> hi/lo copies: column col < b is map row col of

@@ -87,6 +87,25 @@ def test_small_panels_are_the_substitution_panels(hplai, torch_cuda, n, b, flags
     assert _same_bits(lu(flags), lu(flags | hplai.FLAG_SIMT_PANELS))
 
 
+@pytest.mark.parametrize("n,b", [(9248, 136), (5520, 240), (5200, 260), (3840, 384), (2560, 640), (2700, 900)])
+def test_inverse_panels_at_block_edges(hplai, torch_cuda, n, b):
+    """Panels above the size rule, b past one, two, three and five 128-blocks of the triangular inverses: against the
+    substitution, within the products' 2^-18 and the substitution's b eps, both of |X| |T| |T^-1|."""
+    def first(f):
+        with hplai.Solver(n, b, flags=f) as s:
+            s.generate(42)
+            s.factor_steps(1)
+            lu = s.lu()
+        return lu[:b, :b].astype(np.float64), lu[-400:, :b].astype(np.float64), lu[:b, -400:].astype(np.float64)
+    d, lcol, urow = first(0)
+    d2, lref, uref = first(hplai.FLAG_SIMT_PANELS)
+    assert np.array_equal(d, d2)
+    u, l = np.triu(d), np.tril(d, -1) + np.eye(b)
+    eps = 2.0 ** -18 + b * 2.0 ** -23
+    assert np.all(np.abs(lcol - lref) <= eps * (np.abs(lref) @ np.abs(u) @ np.abs(np.linalg.inv(u))))
+    assert np.all(np.abs(urow - uref) <= eps * (np.abs(np.linalg.inv(l)) @ np.abs(l) @ np.abs(uref)))
+
+
 @pytest.mark.parametrize("n,i0,j0,nr,nc,lda,off", [(1000, 3, 5, 1, 1, 1, 0), (1000, 0, 100, 127, 33, 127, 0),
                                                    (4000, 1, 7, 1023, 31, 1024, 0), (4000, 9, 0, 1025, 65, 1025, 0),
                                                    (4000, 0, 2000, 2050, 40, 2052, 1)])
