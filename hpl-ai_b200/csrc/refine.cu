@@ -394,6 +394,71 @@ __device__ __forceinline__ void stage_block(float *blk, const float *a, int64_t 
 	asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
+// x <- T^{-1} x by substitution, T (column-major, TB x TB) and x in shared
+// memory: unit LOWER or non-unit upper.  32 rows at a time: the first warp
+// solves them, a shuffle and a multiply-add (and a division) per step, and a
+// thread per row left applies them.  Ends with a barrier.
+template <bool LOWER>
+__device__ __noinline__ void substitute_block(const float *T, double *x, int rows)
+{
+	const int t = threadIdx.x, lane = t & 31;
+	for (int k = 0; k < TB / 32; ++k) {
+		const int c0 = LOWER ? 32 * k : TB - 32 * (k + 1);
+		if (t < 32) {
+			const int i = c0 + lane;
+			double v = x[i];
+			const double d = !LOWER && i < rows ? static_cast<double>(T[i * TB + i]) : 1.0;
+#pragma unroll
+			for (int q = 0; q < 32; ++q) {
+				const int j = LOWER ? q : 31 - q;
+				if (!LOWER && lane == j) v /= d;
+				const double xj = __shfl_sync(0xffffffffu, v, j);
+				if (LOWER ? lane > j : lane < j) v = fma(-static_cast<double>(T[(c0 + j) * TB + i]), xj, v);
+			}
+			x[i] = v;
+		}
+		__syncthreads();
+		if (t < TB && (LOWER ? t >= c0 + 32 : t < c0)) {
+			double v = x[t];
+			for (int j = 0; j < 32; ++j) v = fma(-static_cast<double>(T[(c0 + j) * TB + t]), x[c0 + j], v);
+			x[t] = v;
+		}
+		__syncthreads();
+	}
+}
+
+// Whether the diagonal block's inverse may be applied: its condition number
+// max_i (|T^{-1}| |T| e)_i is at most 32.  Substitution is backward stable for every
+// triangle, the product with an explicit inverse only for a well-conditioned one.
+// Row by row |b - T x| / (|T| |x| + |b|) over 128 rows, in units of 2^-53, by
+// substitution / by the inverse: the factors of dominant matrices (condition 1 to 4)
+// 5.9 to 7.6 / 1.0 to 1.4, unit lower entries in (-0.1, 0.1) (condition 40) 2.8 / 1.3,
+// (-0.2, 0.2) (170) 2.1 / 2.2, (-0.5, 0.5) (1e4) 1.9 / 82, (-1, 1) (2e9) 1.2 / 1e7.
+// inv[q] = T^{-1}[lr][64 grp + q] (NaN and infinities fail the test); part: two rows
+// of TB.  The same answer in every thread; ends with a barrier.
+__device__ __forceinline__ bool inverse_serves(const double (&inv)[TB / 2], const float *a, int64_t lda, int r0,
+	int rows, bool lower, double (*part)[TB])
+{
+	const int lr = threadIdx.x % TB, grp = threadIdx.x / TB;
+	const float *row = a + static_cast<int64_t>(r0 + grp * (TB / 2)) * lda + r0 + lr;
+	float sum = 0.f;
+#pragma unroll 32
+	for (int q = 0; q < TB / 2; ++q) {
+		const int j = grp * (TB / 2) + q;
+		if (lr < rows && j < rows && (lower ? j < lr : j >= lr)) sum += fabsf(__ldcg(row + static_cast<int64_t>(q) * lda));
+	}
+	part[grp][lr] = lower && grp == 0 ? 1.0 + sum : sum;
+	__syncthreads();
+	double c[2] = {0.0, 0.0};
+#pragma unroll
+	for (int q = 0; q < TB / 2; ++q)
+		c[q & 1] = fma(fabs(inv[q]), part[0][grp * (TB / 2) + q] + part[1][grp * (TB / 2) + q], c[q & 1]);
+	__syncthreads();
+	part[grp][lr] = c[0] + c[1];
+	__syncthreads();
+	return __syncthreads_and(part[0][lr] + part[1][lr] <= 32.0) != 0;
+}
+
 // TRANS: the triangle solved is the transpose of the stored one, M[i][j] =
 // a[i*lda + j]: lower = U^T (non-unit), upper = L^T (unit).  Otherwise
 // M[i][j] = a[j*lda + i]: lower = L (unit), upper = U (non-unit).
@@ -411,10 +476,12 @@ __device__ __forceinline__ void stage_block(float *blk, const float *a, int64_t 
 //  - this thread's 64 entries of the diagonal inverse sit in registers (read
 //    from dinv, or, where the caller keeps no inverses (HAVE_INV = false),
 //    computed here by invert_block), so the diagonal is one product of four
-//    short FMA chains.
+//    short FMA chains.  Nothing behind a leaf call corrects that product, so
+//    without dinv a block that fails inverse_serves is solved by substitution.
 // Measured per triangle, before (flag word and fence, 128-step substitution
 // without dinv) and now: n = 8192 197 -> 111 us, transposed 584 -> 135;
-// n = 65536 2.64 -> 2.40 ms (3.6 TB/s); without dinv n = 16384 2350 -> 250 us.
+// n = 65536 2.64 -> 2.40 ms (3.6 TB/s); without dinv n = 16384 2370 -> 270 us
+// (6 of them the condition numbers; 790 where every block is substituted).
 template <bool TRANS, bool HAVE_INV>
 __global__ void __launch_bounds__(TRSV_THREADS, 1) trsv_kernel(int lower, int n, const float *__restrict__ a,
 	int64_t lda, double *x, TrsvWork *w, ulonglong2 *xt, const double *__restrict__ dinv)
@@ -438,11 +505,12 @@ __global__ void __launch_bounds__(TRSV_THREADS, 1) trsv_kernel(int lower, int n,
 		const int r0 = r * TB;
 		const int rows = min(TB, n - r0);
 		const int nblk = lower ? r : nbt - 1 - r;
+		int extra = 0;   // 1: the diagonal block is substituted, and staged last (col_of(nblk) == r)
 		auto col_of = [&](int q) { return lower ? q : nbt - 1 - q; };
 		// the first NB - 1 off-diagonal blocks in flight before anything waits;
 		// one copy group per block (empty past the last) keeps the count fixed
 		auto stage_q = [&](int q) {
-			if (q < nblk) {
+			if (q < nblk + extra) {
 				const int cb = col_of(q);
 				stage_block<TRANS>(dyn_smem + (q % NB) * TB * TB, a, lda, r0, cb * TB, rows, min(TB, n - cb * TB), vec);
 			} else {
@@ -474,6 +542,7 @@ __global__ void __launch_bounds__(TRSV_THREADS, 1) trsv_kernel(int lower, int n,
 #pragma unroll
 			for (int q = 0; q < TB / 2; ++q) dv[q] = lower ? X[lr * kInvLd + jb + q] : X[(jb + q) * kInvLd + lr];
 			__syncthreads();
+			extra = inverse_serves(dv, a, lda, r0, rows, lower != 0, part) ? 0 : 1;
 		}
 		double acc4[4] = {0.0, 0.0, 0.0, 0.0};
 		// TRANS: warp `wv` takes rows wv, wv + 8, ...; lane takes 4 columns
@@ -568,8 +637,27 @@ __global__ void __launch_bounds__(TRSV_THREADS, 1) trsv_kernel(int lower, int n,
 			part[grp][lr] = (acc4[0] + acc4[1]) + (acc4[2] + acc4[3]);
 		}
 		__syncthreads();
-		if (t < TB) rhs[t] = (t < rows) ? xr - (part[0][t] + part[1][t]) : 0.0;
-		__syncthreads();
+		const double br = (t < rows) ? xr - (part[0][t] + part[1][t]) : 0.0;
+		if (t < TB) rhs[t] = br;
+		// an infinity or NaN reaches only the rows that depend on it, which the
+		// inverse's zeros would not see to
+		const bool finite = __syncthreads_and(isfinite(br)) != 0;
+		if (!HAVE_INV && (extra || !finite)) {
+			float *T = dyn_smem + (nblk % NB) * TB * TB;
+			if (!extra) stage_block<false>(T, a, lda, r0, r0, rows, rows, vec);
+			asm volatile("cp.async.wait_all;" ::: "memory");
+			__syncthreads();
+			if (lower)
+				substitute_block<true>(T, rhs, rows);
+			else
+				substitute_block<false>(T, rhs, rows);
+			if (t < rows) {
+				const double v = rhs[t];
+				xt_publish(xt + r0 + t, v, epoch);
+				x[r0 + t] = v;
+			}
+			continue;
+		}
 		// x_r = M_rr^{-1} rhs
 		double v4[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll

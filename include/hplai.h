@@ -514,7 +514,9 @@ size_t hplai_trsv_workspace(int n);
 /* panel_trsvL / panel_trsvU (panel_trsv.hpp:310-758): x <- L^{-1} x with L
  * the unit lower triangle of a, or x <- U^{-1} x with U the upper triangle
  * of a (FP32 factors, FP64 vector).  `work` holds at least
- * hplai_trsv_workspace(n) bytes and must be zeroed before its first use. */
+ * hplai_trsv_workspace(n) bytes and must be zeroed before its first use.
+ * A 128 x 128 diagonal block T whose condition number || |T^-1| |T| ||_inf is
+ * at most 32 is applied as its FP64 inverse, any other by substitution. */
 int hplai_trsv_lower(int n, const float *a, int64_t lda, double *x, void *work, size_t work_bytes, void *stream);
 int hplai_trsv_upper(int n, const float *a, int64_t lda, double *x, void *work, size_t work_bytes, void *stream);
 

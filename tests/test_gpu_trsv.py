@@ -30,7 +30,7 @@ def _solve(m, x, lower):
 @pytest.mark.parametrize("n,lda,off", [(1, 1, 0), (31, 32, 0), (127, 129, 0), (128, 128, 0), (129, 132, 0), (257, 257, 1),
                                        (1000, 1004, 0), (2500, 2501, 3), (19200, 19264, 0)])
 def test_trsv_leaf_edges(hplai, torch_cuda, n, lda, off):
-    """Backward error bound of a triangular solve, n eps |T| |x|, dominated here by a few eps of |x|_inf."""
+    """Dominant factors as the LU leaves them: their blocks are well conditioned, so the forward error is a few eps."""
     torch = torch_cuda
     rng = np.random.default_rng(n)
     if n <= 2500:
@@ -63,6 +63,60 @@ def test_trsv_leaf_edges(hplai, torch_cuda, n, lda, off):
                                                 unitriangular=lower)[:, 0].cpu().numpy()
             del d
         assert np.abs(got - ref).max() <= 1e-13 * np.abs(ref).max(), lower
+
+
+def _leaf(hplai, torch, m, x, lower):
+    n = len(x)
+    a = torch.from_numpy(np.ascontiguousarray(m.T)).cuda()
+    xd = torch.from_numpy(x).cuda()
+    w = torch.zeros(hplai.trsv_workspace(n), dtype=torch.uint8, device="cuda")
+    fn = hplai.trsv_lower if lower else hplai.trsv_upper
+    hplai.check(fn(n, a.data_ptr(), n, xd.data_ptr(), w.data_ptr(), w.numel(), None))
+    return xd.cpu().numpy()
+
+
+@pytest.mark.parametrize("n", [20, 33, 65, 97, 128, 130, 300, 513])
+@pytest.mark.parametrize("lower", [True, False])
+def test_trsv_leaf_any_triangle(hplai, torch_cuda, n, lower):
+    """Triangles from dominant to condition numbers of 1e9 a block, a solution that does not grow: substitution is
+    backward stable for each, row by row |T x - b| <= g (|T| |x| + |b|) with g = (n + 4) eps of FP64 for its n products,
+    sums and one quotient."""
+    rng = np.random.default_rng(n)
+    for size in (0.1, 0.5, 1.0):
+        m = rng.uniform(-size, size, (n, n)).astype(np.float32)
+        m[np.arange(n), np.arange(n)] = np.where(rng.random(n) < 0.5, -1, 1) * rng.uniform(0.5, 1, n)
+        t = m.astype(np.longdouble)
+        t = np.tril(t, -1) + np.eye(n) if lower else np.triu(t)
+        b = (t @ np.ones(n)).astype(np.float64)
+        x = _leaf(hplai, torch_cuda, m, b, lower)
+        r = np.abs(t @ x.astype(np.longdouble) - b)
+        assert np.all(r <= (n + 4) * 2.0 ** -53 * (np.abs(t) @ np.abs(x) + np.abs(b))), size
+
+
+def test_trsv_leaf_quotients(hplai, torch_cuda):
+    """A diagonal U: the quotients of FP64, to one unit in the last place, over zeros, the smallest and the largest."""
+    rng = np.random.default_rng(3)
+    n = 200
+    d = (rng.uniform(1, 2, n) * 2.0 ** rng.integers(-20, 20, n)).astype(np.float32)
+    b = rng.uniform(-1, 1, n)
+    d[5], d[40], d[70], d[71], d[150] = 2.0 ** -140, 2.0 ** 127, np.inf, 1e-45, 3e-39
+    b[20], b[21], b[60], b[90], b[130], b[150] = 0.0, -0.0, 1e-300, 5e-324, 1e300, 1e250
+    x = _leaf(hplai, torch_cuda, np.diag(d), b, False)
+    ref = b / d.astype(np.float64)
+    assert np.all(np.abs(x - ref) <= 2.0 ** -52 * np.abs(ref))
+
+
+@pytest.mark.parametrize("lower", [True, False])
+def test_trsv_leaf_infinite_entry(hplai, torch_cuda, lower):
+    """The rows solved before the one with an infinite right-hand side do not see it."""
+    rng = np.random.default_rng(9)
+    m, b = _factors(rng, 200), rng.uniform(-1, 1, 200)
+    ref = _solve(m, b, lower)
+    b[70] = np.inf
+    x = _leaf(hplai, torch_cuda, m, b, lower)
+    clean = slice(0, 70) if lower else slice(71, 200)
+    assert np.abs(x[clean] - ref[clean]).max() <= 1e-13 * np.abs(ref).max()
+    assert not np.any(np.isfinite(x[71:] if lower else x[:70])) and not np.isfinite(x[70])
 
 
 def test_trsv_leaf_workspace_limits(hplai, torch_cuda):
