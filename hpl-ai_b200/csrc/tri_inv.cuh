@@ -16,7 +16,7 @@ constexpr int kTriThreads = 256;
 // (so X is the transpose of U_rr^{-1}), padded with the identity past `rows`.
 // The FP32 factor entries convert exactly.
 // The 16 x 16 diagonal blocks are inverted by substitution, one thread per
-// column, in registers; then pairs of inverted blocks of h = 16, 32, 64 are
+// row, in registers; then pairs of inverted blocks of h = 16, 32, 64 are
 // joined, [A 0; B C]^{-1} = [A^{-1} 0; -C^{-1} B A^{-1}, C^{-1}], as two
 // products whose zero triangles are skipped 16 rows (or a column group) at a
 // time.  Threads take interleaved rows and columns, so that the operands of a
@@ -27,7 +27,7 @@ constexpr int kTriThreads = 256;
 constexpr int kInvLd = kTriBlock + 1;
 constexpr int kInvLdW = kTriBlock / 2 + 1;
 template <typename R>
-constexpr size_t kInvSmem = sizeof(R) * (static_cast<size_t>(kTriBlock) * kInvLd + kTriBlock / 2 * kInvLdW + kTriBlock);
+constexpr size_t kInvSmem = sizeof(R) * (static_cast<size_t>(kTriBlock) * kInvLd + kTriBlock / 2 * kInvLdW);
 
 template <typename R, int H>
 __device__ __forceinline__ void invert_join(R *X, R *W)
@@ -100,7 +100,7 @@ template <typename R>
 __device__ __noinline__ void invert_block(R *smem, const float *__restrict__ a, int64_t lda, int r0, int rows,
 	bool upper)
 {
-	R *X = smem, *W = X + kTriBlock * kInvLd, *rd = W + kTriBlock / 2 * kInvLdW;
+	R *X = smem, *W = X + kTriBlock * kInvLd;
 	const int t = threadIdx.x;
 	// T[i][j] from the stored block, line l (a column), place s in it
 	auto put = [&](int l, int s, float f) {
@@ -138,26 +138,26 @@ __device__ __noinline__ void invert_block(R *smem, const float *__restrict__ a, 
 		}
 	}
 	__syncthreads();
-	if (t < kTriBlock) rd[t] = R(1) / X[t * kInvLd + t];
-	__syncthreads();
 	R v[16];
 	const int b0 = (t / 16) * 16, c = t % 16;
 	if (t < kTriBlock) {
+		// row c of the block's inverse, from the last column down.  A division and
+		// no product with a reciprocal, so that a zero over a tiny or infinite
+		// diagonal entry stays a zero (with corrected reciprocals n = 9600 took 8.82
+		// and not 8.93 ms, a batch of 512 systems 49.8 and not 50.6).
 #pragma unroll
 		for (int i = 0; i < 16; ++i) v[i] = (i == c) ? R(1) : R(0);
 #pragma unroll
-		for (int j = 0; j < 16; ++j) {
-			// v_j / t_jj: the product with the reciprocal, corrected once
-			const R d = X[(b0 + j) * kInvLd + b0 + j], q = v[j] * rd[b0 + j];
-			v[j] = fma(fma(-d, q, v[j]), rd[b0 + j], q);
+		for (int j = 15; j >= 0; --j) {
+			if (upper) v[j] = v[j] / X[(b0 + j) * kInvLd + b0 + j];
 #pragma unroll
-			for (int i = j + 1; i < 16; ++i) v[i] = fma(-X[(b0 + i) * kInvLd + b0 + j], v[j], v[i]);
+			for (int i = 0; i < j; ++i) v[i] = fma(-X[(b0 + j) * kInvLd + b0 + i], v[j], v[i]);
 		}
 	}
 	__syncthreads();
 	if (t < kTriBlock) {
 #pragma unroll
-		for (int i = 0; i < 16; ++i) X[(b0 + i) * kInvLd + b0 + c] = v[i];
+		for (int i = 0; i < 16; ++i) X[(b0 + c) * kInvLd + b0 + i] = v[i];
 	}
 	__syncthreads();
 	// rows past `rows` are the identity's: nothing to join there

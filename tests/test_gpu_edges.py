@@ -106,6 +106,27 @@ def test_inverse_panels_at_block_edges(hplai, torch_cuda, n, b):
     assert np.all(np.abs(urow - uref) <= eps * (np.abs(np.linalg.inv(l)) @ np.abs(l) @ np.abs(uref)))
 
 
+def test_inverse_panels_of_extreme_diagonals(hplai, torch_cuda):
+    """The panels by inverses (the precision form's TF32 path) under a diagonal block with an infinite pivot, one whose
+    reciprocal is subnormal and, last, one whose reciprocal overflows: as in the substitution, x / inf is 0 and every other
+    column is finite, x / d to TF32's 2^-10."""
+    n, b = 90, 30
+    rng = np.random.default_rng(11)
+    a = np.asfortranarray(rng.uniform(0.25, 0.5, (n, n)).astype(np.float32))
+    d = rng.uniform(1, 2, b).astype(np.float32)
+    d[3], d[7], d[b - 1] = 2.0 ** 127, np.inf, 2.0 ** -140
+    a[:b, :b] = np.diag(d)
+    a[b:, b:] += 100 * np.eye(n - b, dtype=np.float32)
+    with hplai.Solver(n, b, precision=hplai.F32_F8) as s:
+        s.upload(a, np.ones(n), np.full(n, 100.0))
+        s.factor_steps(1)
+        lu = s.lu()
+    got, ref = lu[b:, :b - 1].astype(np.float64), a[b:, :b - 1] / d[:b - 1].astype(np.float64)
+    assert np.all(got[:, 7] == 0)
+    assert np.all(np.abs(got - ref) <= 2.0 ** -9 * np.abs(ref) + 2.0 ** -126)
+    assert np.all(np.abs(lu[:b, b:] - a[:b, b:]) <= 2.0 ** -9 * a[:b, b:])
+
+
 @pytest.mark.parametrize("n,i0,j0,nr,nc,lda,off", [(1000, 3, 5, 1, 1, 1, 0), (1000, 0, 100, 127, 33, 127, 0),
                                                    (4000, 1, 7, 1023, 31, 1024, 0), (4000, 9, 0, 1025, 65, 1025, 0),
                                                    (4000, 0, 2000, 2050, 40, 2052, 1)])
