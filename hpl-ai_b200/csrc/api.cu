@@ -243,8 +243,9 @@ struct PhaseEvents {
 	size_t used = 0;
 	std::vector<Span> spans;
 	// everything of this call runs on one stream, phase after phase: a phase
-	// begins where the last one ended
+	// begins where the last one ended, unless the stream waited in between
 	bool chained;
+	bool waited = false;
 	explicit PhaseEvents(std::vector<cudaEvent_t> &p, bool one_stream = false) : pool(p), chained(one_stream) {}
 	int take(cudaEvent_t *e)
 	{
@@ -259,12 +260,13 @@ struct PhaseEvents {
 	int record(cudaStream_t st, int ph)
 	{
 		Span sp{ph, nullptr, nullptr};
-		if (chained && !spans.empty()) {
+		if (chained && !waited && !spans.empty()) {
 			sp.begin = spans.back().end;
 		} else {
 			HPLAI_TRY(take(&sp.begin));
 			HPLAI_CUDA_TRY(cudaEventRecord(sp.begin, st));
 		}
+		waited = false;
 		HPLAI_TRY(take(&sp.end));
 		spans.push_back(sp);
 		return HPLAI_OK;
@@ -960,7 +962,10 @@ int factor_impl(hplai_ctx *c, int kend, const float *host_a = nullptr, int64_t h
 		}
 	}
 	auto wait_copy = [&](int j) -> int {
-		if (host_a) HPLAI_CUDA_TRY(cudaStreamWaitEvent(sd, c->ev_copy[j], 0));
+		if (host_a) {
+			HPLAI_CUDA_TRY(cudaStreamWaitEvent(sd, c->ev_copy[j], 0));
+			pe.waited = true;   // the wait for the copy belongs to no phase
+		}
 		return HPLAI_OK;
 	};
 	// the side stream starts from the generated matrix: group 0's panels
