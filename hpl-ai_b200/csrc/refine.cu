@@ -12,7 +12,6 @@
 #include "tri_inv.cuh"
 
 #include <mutex>
-#include <type_traits>
 
 namespace hplai {
 
@@ -60,37 +59,118 @@ __device__ __forceinline__ void block_max(double m, double *out)
 }
 
 // ---------------------------------------------------------------------------
-// On-the-fly GEMV.  CTA = 512/SPLIT rows x GEMV_COLS columns; the columns of
-// a chunk are divided into SPLIT pieces, and each thread walks two rows (32
-// apart) across one piece with two interleaved LCG chains and two FP64
-// accumulators a row.  The pieces are folded in shared memory and the chunks
-// by a second kernel, both in a fixed order, so the result does not depend on
-// scheduling.
+// On-the-fly GEMV: partial sums of GEMV_COLS columns by one of two kernels,
+// and the chunks folded by a third, all in a fixed order, so the result does
+// not depend on scheduling.
 //
 // Bound by the integer multiplies of the LCG (three of a 64-bit product, one
 // of them wide) together with the FP64 multiply-add, which issue to the same
-// port; hence two rows per thread, which share the reads of x, and the
-// hardware's 64-bit integer conversion, which has a pipe of its own (the
-// conversion through the mantissas of 2^84 and 2^52 costs two FP64 additions
-// and was 25 % slower here).
+// port; hence the hardware's 64-bit integer conversion, which has a pipe of
+// its own (the conversion through the mantissas of 2^84 and 2^52 costs two
+// FP64 additions and was 25 % slower here).
 // ---------------------------------------------------------------------------
 constexpr int GEMV_THREADS = 256;
 constexpr int GEMV_ROWS = 256;
 constexpr int GEMV_COLS = 2048;
 
+// The state of row lane's first column, for a warp whose first element is idx0
+// and whose rows are `lp` apart; lp becomes the jump by 32 rows.
+__device__ __forceinline__ uint64_t row_state(const Coeff *tab, uint64_t idx0, uint64_t state00, Coeff &lp)
+{
+	uint64_t s = coeff_apply(warp_jump(tab, idx0), state00);
+#pragma unroll
+	for (int b = 0; b < 5; ++b) {
+		if ((threadIdx.x >> b) & 1) s = coeff_apply(lp, s);
+		lp = coeff_mul(lp, lp);
+	}
+	return s;
+}
+
+// Large orders: CTA = 256 rows x GEMV_COLS columns, a row per thread with four
+// interleaved LCG chains and two FP64 accumulators.
 // TRANS: y = A^T x, output i walks column i of A (element (j, i) is state
 // j + n*i, so the chain steps by 1 instead of n).  jn: the jump by n.
-template <bool TRANS, int SPLIT>
-__global__ void __launch_bounds__(GEMV_THREADS) otf_partial_kernel(int64_t n, int mb, int nb, double alpha,
+template <bool TRANS>
+__global__ void __launch_bounds__(GEMV_ROWS) otf_rows_kernel(int64_t n, int mb, int nb, double alpha,
 	const double *__restrict__ x, uint64_t state00, int with_diag, const double *__restrict__ diag,
 	double *__restrict__ part, JumpTable64 tab, Coeff jn, double *norms)
 {
-	constexpr int W = GEMV_THREADS / SPLIT / 32;   // warps that share a piece, 64 rows each
-	constexpr int R = 64 * W;
-	static_assert(W >= 1, "a warp's threads share one piece");
 	__shared__ __align__(16) double xs[GEMV_COLS];
 	__shared__ Coeff stab[64];
-	__shared__ double fold[SPLIT > 1 ? SPLIT * R : 1];
+	const int t = threadIdx.x, lane = t & 31;
+	if (norms && blockIdx.x == 0 && blockIdx.y == 0 && t < 2) norms[t] = 0.0;   // for otf_reduce_kernel
+	const int j0 = blockIdx.y * GEMV_COLS;
+	const int j1 = min(j0 + GEMV_COLS, nb);
+	for (int j = t; j < j1 - j0; j += GEMV_ROWS) xs[j] = x[j0 + j];
+	if (t < 64) stab[t] = tab.p[t];
+	__syncthreads();
+	const int i = blockIdx.x * GEMV_ROWS + t;
+	if (i - lane >= mb) return;   // whole warps
+	const uint64_t iu = static_cast<uint64_t>(i - lane), ju = static_cast<uint64_t>(j0);
+	Coeff lp = TRANS ? jn : stab[0];
+	uint64_t s0 = row_state(stab, TRANS ? ju + static_cast<uint64_t>(n) * iu : iu + static_cast<uint64_t>(n) * ju, state00, lp);
+	const Coeff jc = TRANS ? stab[0] : jn;
+	const Coeff jc4 = coeff_mul(coeff_mul(jc, jc), coeff_mul(jc, jc));
+	uint64_t s1 = coeff_apply(jc, s0);
+	uint64_t s2 = coeff_apply(jc, s1);
+	uint64_t s3 = coeff_apply(jc, s2);
+	auto val = [](uint64_t v) { return __ll2double_rn(static_cast<long long>(v)); };
+	double a0 = 0.0, a1 = 0.0;
+	const int len = j1 - j0;
+	const int dj = (with_diag && i >= j0 && i < j1) ? i - j0 : -1;   // diagonal column inside the chunk
+	int j = 0;
+	if (!__any_sync(0xffffffffu, dj >= 0)) {
+		// no diagonal in this chunk for any row of the warp
+		for (; j + 3 < len; j += 4) {
+			const double2 x01 = *reinterpret_cast<const double2 *>(&xs[j]);
+			const double2 x23 = *reinterpret_cast<const double2 *>(&xs[j + 2]);
+			a0 = fma(val(s0), x01.x, a0);
+			a1 = fma(val(s1), x01.y, a1);
+			a0 = fma(val(s2), x23.x, a0);
+			a1 = fma(val(s3), x23.y, a1);
+			s0 = coeff_apply(jc4, s0);
+			s1 = coeff_apply(jc4, s1);
+			s2 = coeff_apply(jc4, s2);
+			s3 = coeff_apply(jc4, s3);
+		}
+	} else {
+		for (; j + 3 < len; j += 4) {
+			const double v0 = j == dj ? 0.0 : val(s0), v1 = j + 1 == dj ? 0.0 : val(s1);
+			const double v2 = j + 2 == dj ? 0.0 : val(s2), v3 = j + 3 == dj ? 0.0 : val(s3);
+			a0 = fma(v0, xs[j], a0);
+			a1 = fma(v1, xs[j + 1], a1);
+			a0 = fma(v2, xs[j + 2], a0);
+			a1 = fma(v3, xs[j + 3], a1);
+			s0 = coeff_apply(jc4, s0);
+			s1 = coeff_apply(jc4, s1);
+			s2 = coeff_apply(jc4, s2);
+			s3 = coeff_apply(jc4, s3);
+		}
+	}
+	for (; j < len; ++j) {
+		a0 = fma(j == dj ? 0.0 : val(s0), xs[j], a0);
+		s0 = coeff_apply(jc, s0);
+	}
+	if (i >= mb) return;
+	double r = (a0 + a1) * (alpha * kValueScale);
+	if (dj >= 0) r = fma(alpha * diag[i], xs[dj], r);
+	part[static_cast<int64_t>(blockIdx.y) * mb + i] = r;
+}
+
+// Smaller orders, whose rows alone would not fill the GPU: CTA = 64 rows x
+// GEMV_COLS columns, divided into eight pieces, a warp each.  A thread walks
+// two rows (32 apart, which share the reads of x) across its piece with two
+// LCG chains and two FP64 accumulators a row; the pieces are folded in shared
+// memory.
+template <bool TRANS>
+__global__ void __launch_bounds__(GEMV_THREADS) otf_pieces_kernel(int64_t n, int mb, int nb, double alpha,
+	const double *__restrict__ x, uint64_t state00, int with_diag, const double *__restrict__ diag,
+	double *__restrict__ part, JumpTable64 tab, Coeff jn, double *norms)
+{
+	constexpr int SPLIT = GEMV_THREADS / 32, R = 64;
+	__shared__ __align__(16) double xs[GEMV_COLS];
+	__shared__ Coeff stab[64];
+	__shared__ double fold[SPLIT * R];
 	const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
 	if (norms && blockIdx.x == 0 && blockIdx.y == 0 && t < 2) norms[t] = 0.0;   // for otf_reduce_kernel
 	const int j0 = blockIdx.y * GEMV_COLS;
@@ -98,23 +178,16 @@ __global__ void __launch_bounds__(GEMV_THREADS) otf_partial_kernel(int64_t n, in
 	for (int j = t; j < j1 - j0; j += GEMV_THREADS) xs[j] = x[j0 + j];
 	if (t < 64) stab[t] = tab.p[t];
 	__syncthreads();
-	const int piece = warp / W, row = (warp % W) * 64 + lane;   // and row + 32
-	const int iw = blockIdx.x * R + (warp % W) * 64;            // the warp's first row
+	const int iw = blockIdx.x * R;   // rows iw + lane and iw + lane + 32
 	const int width = ((j1 - j0 + SPLIT - 1) / SPLIT + 3) & ~3;
-	const int p0 = min(piece * width, j1 - j0), p1 = min(p0 + width, j1 - j0);
+	const int p0 = min(warp * width, j1 - j0), p1 = min(p0 + width, j1 - j0);
 	double r[2] = {0.0, 0.0};
-	// whole warps past the last row or without columns have nothing to do
-	if (iw < mb && p0 < p1) {
+	// whole warps without columns have nothing to do
+	if (p0 < p1) {
 		const uint64_t iu = static_cast<uint64_t>(iw), ju = static_cast<uint64_t>(j0 + p0);
 		uint64_t s[2][2];   // [row][column parity]
-		s[0][0] = coeff_apply(warp_jump(stab, TRANS ? ju + static_cast<uint64_t>(n) * iu
-		                                              : iu + static_cast<uint64_t>(n) * ju), state00);
 		Coeff lp = TRANS ? jn : stab[0];
-#pragma unroll
-		for (int b = 0; b < 5; ++b) {
-			if ((lane >> b) & 1) s[0][0] = coeff_apply(lp, s[0][0]);
-			lp = coeff_mul(lp, lp);
-		}
+		s[0][0] = row_state(stab, TRANS ? ju + static_cast<uint64_t>(n) * iu : iu + static_cast<uint64_t>(n) * ju, state00, lp);
 		const Coeff jc = TRANS ? stab[0] : jn;
 		const Coeff jc2 = coeff_mul(jc, jc);
 		s[1][0] = coeff_apply(lp, s[0][0]);   // 32 rows on
@@ -168,14 +241,8 @@ __global__ void __launch_bounds__(GEMV_THREADS) otf_partial_kernel(int64_t n, in
 			if (dj >= 0 && dj < len && i < mb) r[q] = fma(alpha * diag[i], xp[dj], r[q]);
 		}
 	}
-	if (SPLIT == 1) {
-#pragma unroll
-		for (int q = 0; q < 2; ++q)
-			if (iw + lane + 32 * q < mb) part[static_cast<int64_t>(blockIdx.y) * mb + iw + lane + 32 * q] = r[q];
-		return;
-	}
-	fold[piece * R + row] = r[0];
-	fold[piece * R + row + 32] = r[1];
+	fold[warp * R + lane] = r[0];
+	fold[warp * R + lane + 32] = r[1];
 	__syncthreads();
 	for (int e = t; e < R; e += GEMV_THREADS) {
 		double v = fold[e];
@@ -220,25 +287,17 @@ int otf_launch(int64_t n, int mb, int nb, double alpha, const double *x, double 
 	double *part = static_cast<double *>(work);
 	if (nb > 0) {
 		const Coeff jn = coeff_pow(static_cast<uint64_t>(n));
-		auto launch = [&](auto split) {
-			constexpr int S = decltype(split)::value, R = 2 * GEMV_THREADS / S;
-			const dim3 grid((mb + R - 1) / R, nchunks);
-			if (trans)
-				otf_partial_kernel<true, S><<<grid, GEMV_THREADS, 0, st>>>(n, mb, nb, alpha, x, state00, with_diag, diag,
-					part, table(), jn, norms);
-			else
-				otf_partial_kernel<false, S><<<grid, GEMV_THREADS, 0, st>>>(n, mb, nb, alpha, x, state00, with_diag, diag,
-					part, table(), jn, norms);
-		};
-		// Short pieces spread a small order over the SMs (n = 1200: 30 us in one
-		// piece, 13 in eight) and balance the last wave of a large one (32768: 434
-		// in two, 425 in eight).  For A^T, whose set-up is longer (the lanes' jumps
-		// are by n), two pieces are faster once there is work enough (32768: 442
-		// against 483; 16384: 137 against 129).
-		if (trans && static_cast<int64_t>((mb + 255) / 256) * nchunks >= 888)
-			launch(std::integral_constant<int, 2>{});
-		else
-			launch(std::integral_constant<int, 8>{});
+		// A row per thread once there are waves enough of such CTAs,
+		// else pieces, which spread a small order over the SMs and balance the last
+		// wave; for A^T, whose set-up is longer (the lanes' jumps are by n), sooner.
+		// Rows / pieces, us: n = 1200 35 / 14.5, 16384 143 / 117, 24576 255 / 249,
+		// 32768 426 / 427, 65536 1592 / 1662, 131072 6220 / 6600; A^T 9600 71 / 55,
+		// 16384 131 / 123, 20480 183 / 186, 32768 405 / 457, 131072 5950 / 7090.
+		const bool wide = static_cast<int64_t>((mb + GEMV_ROWS - 1) / GEMV_ROWS) * nchunks >= (trans ? 800 : 2048);
+		const dim3 grid((mb + (wide ? GEMV_ROWS : 64) - 1) / (wide ? GEMV_ROWS : 64), nchunks);
+		const auto kernel = wide ? (trans ? otf_rows_kernel<true> : otf_rows_kernel<false>)
+		                         : (trans ? otf_pieces_kernel<true> : otf_pieces_kernel<false>);
+		kernel<<<grid, GEMV_THREADS, 0, st>>>(n, mb, nb, alpha, x, state00, with_diag, diag, part, table(), jn, norms);
 		count_launches();
 		HPLAI_CUDA_TRY(cudaGetLastError());
 	}

@@ -161,6 +161,39 @@ def test_gemv_edges(hplai, oracle, torch_cuda, n):
         assert np.abs(yd.cpu().numpy() - ref).max() <= 1e-14 * (np.abs(a).sum(1).max() + 1)
 
 
+# a row per thread from 2048 blocks of 256 rows x 2048 columns on (transposed: 800): odd orders past the rules' lines
+def test_gemv_of_large_orders(hplai, oracle, torch_cuda):
+    torch = torch_cuda
+    n = 33001
+    rng = np.random.default_rng(n)
+    x, y0 = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    dd = torch.empty(n, dtype=torch.float64, device="cuda")
+    hplai.check(hplai.gen_diag(n, 42, 0, n, dd.data_ptr(), None))
+    xd, yd = torch.from_numpy(x).cuda(), torch.from_numpy(y0).cuda()
+    ws = hplai.otf_gemv_workspace(n)
+    w = torch.empty(ws, dtype=torch.uint8, device="cuda")
+    hplai.check(hplai.otf_gemv(n, -1.0, xd.data_ptr(), 1.0, yd.data_ptr(), 42, dd.data_ptr(), w.data_ptr(), ws, None))
+    got = yd.cpu().numpy()
+    rows = np.array([0, 31, 32, 255, 256, 2047, 2048, 16384, 32767, 32768, 32999, 33000])
+    ref = oracle.residual_rows(n, x, rows, rhs_v=y0)
+    assert np.abs(got[rows] - ref).max() <= 1e-14 * 2 * float(dd.max())
+
+
+def test_transposed_residual_of_large_orders(hplai, oracle, torch_cuda):
+    """lambda of A^T lambda = g has the residual that the refinement reports for it, on sampled rows."""
+    n, b = 20808, 72
+    g = np.random.default_rng(n).uniform(-1, 1, n)
+    with hplai.Solver(n, b) as s:
+        s.generate(42)
+        s.factor()
+        lam, r = s.solve_transpose(g)
+        d = s.diag()
+    assert r.status == hplai.HPLAI_OK
+    rows = np.array([0, 1, 31, 255, 256, 2048, 10007, 20479, 20480, 20735, 20807])
+    res = oracle.residual_rows(n, lam, rows, trans=True, rhs_v=g)
+    assert np.abs(res).max() <= r.residual + 1e-14 * 2 * d.max() * np.abs(lam).max()
+
+
 @pytest.mark.parametrize("n", [[2], [127, 129, 128], [640, 100, 36], [1500, 1536]])
 def test_batch_edges(hplai, oracle, torch_cuda, n):
     """Orders around the 128-wide steps, one to eight right-hand sides."""
