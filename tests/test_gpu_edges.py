@@ -38,6 +38,20 @@ def test_getrf_tile_edges(hplai, oracle, torch_cuda, b, lda, off):
     assert _same_bits(_take(t, b, b, lda, off), oracle.getrf_nopiv(m))
 
 
+@pytest.mark.parametrize("n,b,side", [(3072, 1024, 2), (3072, 1024, 7), (3072, 1024, 16), (2700, 900, 9), (2048, 512, 4),
+                                      (1280, 320, 3)])
+def test_getrf_on_few_sms(hplai, torch_cuda, n, b, side):
+    """More tiles than a team has places for in shared memory, odd numbers of teams: the factors of the whole GPU."""
+    def lu(flags):
+        with hplai.Solver(n, b, flags=flags) as s:
+            if flags:
+                s.set_schedule(flags, side)
+            s.generate(42)
+            s.factor()
+            return s.lu()
+    assert _same_bits(lu(0), lu(hplai.FLAG_LOOKAHEAD))
+
+
 @pytest.mark.parametrize("scale", [2.0 ** -127, 2.0 ** -140, 2.0 ** 120])
 def test_getrf_pivots_without_normal_reciprocals(hplai, oracle, torch_cuda, scale):
     """Subnormal pivots, and pivots whose reciprocals are subnormal, take the reciprocal that keeps subnormals."""
