@@ -15,9 +15,7 @@
 // (the LU of [[A, 0], [0, I]] is [[L, 0], [0, I]] [[U, 0], [0, I]], exactly:
 // the padding receives only zero updates), and the systems sit side by side
 // in one FP32 matrix of P_max rows (ld = P_max): system s's A(i, j) is at
-// row i, column C_s + j, with 128 unused columns after each system (the
-// last 256-column Schur tile of a step may reach past a system's columns).
-// A system's columns are contiguous in memory, so a 128-column block spans a
+// row i, column C_s + j.  A system's columns are contiguous in memory, so a 128-column block spans a
 // few pages.  Its L and U panels of a group of steps are FP16 copies in two
 // stacked K-major buffers (row R_s + i of L16 = row i of L, row R_s + j of U16
 // = column j of U).  Systems are ordered by decreasing P_s, so the systems
@@ -58,8 +56,9 @@ constexpr int kBB = 128;          // panel width
 // panels so far (still one update launch per step).  An update of K = 128 is
 // bound by the traffic of C: 512 systems' updates 16.5 ms one panel at a time,
 // 5.9 ms in groups of four.
+// Each panel of a group has its slot of kBB in a row's FP16 copies, so where
+// four do not fit in memory a batch goes one panel at a time.
 constexpr int kGroup = 4;
-constexpr int kLdK = kGroup * kBB;   // a panel row's FP16 copies: one slot of kBB per panel of the group
 constexpr int kGemvRows = 256;    // GEMV rows per CTA
 constexpr int kGemvCols = 512;    // GEMV columns per CTA (one partial-sum chunk)
 constexpr int kMaxRhs = 8;
@@ -93,7 +92,7 @@ __device__ __forceinline__ Coeff jump(const JumpT &t, uint64_t m)
 struct BSys {
 	int n, P, nrhs, orig;   // order, padded order, right-hand sides, index in the caller's arrays
 	int64_t R;              // its first row in the stacked FP16 panel buffers
-	int64_t C;              // its first column in A (ld P_max; 128 unused columns after each system)
+	int64_t C;              // its first column in A (ld P_max)
 	int64_t voff;           // its n x nrhs vectors (rhs, x, r), column-major with ld n
 	int64_t doff;           // its n diagonal entries
 	int64_t poff;           // its GEMV partial sums: ceil(n / kGemvCols) x nrhs x n
@@ -356,7 +355,7 @@ __device__ __forceinline__ void trsm_steps(float (&b)[4][kMicro], const float *t
 constexpr int kTrsmThreads = 256;
 __global__ void __launch_bounds__(kTrsmThreads, 2) btrsm_kernel(const BSys *__restrict__ sys,
 	const int4 *__restrict__ items, float *__restrict__ A, int64_t lda, __half *__restrict__ L16,
-	__half *__restrict__ U16, int k)
+	__half *__restrict__ U16, int k, int ldk, int slot)
 {
 	extern __shared__ __align__(16) float sm[];
 	// side 0: tri[i * kLdT + j] = U(i, j) (rows of U); side 1: tri[i * kLdT + r] = L(r, i) (columns of L)
@@ -437,7 +436,7 @@ __global__ void __launch_bounds__(kTrsmThreads, 2) btrsm_kernel(const BSys *__re
 	}
 #pragma unroll
 	for (int r = 0; r < 4; ++r) {
-		__half *o = (upper ? U16 : L16) + (S.R + off + p0 + r) * kLdK + (k % kGroup) * kBB + e0;
+		__half *o = (upper ? U16 : L16) + (S.R + off + p0 + r) * ldk + slot * kBB + e0;
 #pragma unroll
 		for (int q = 0; q < 2; ++q) {
 			uint4 w;
@@ -769,6 +768,7 @@ __global__ void __launch_bounds__(128) bxupd_kernel(const BSys *__restrict__ sys
 // ---------------------------------------------------------------------------
 struct BatchEngine {
 	int count = 0, pmax = 0, nsteps = 0, npairs = 0;
+	int group = kGroup;                    // panels per update of the trailing matrices
 	int64_t rows = 0, cols = 0, lda = 0;
 	std::vector<BSys> sys;                 // factorisation order
 	std::vector<int> active;               // systems still factoring at step k (a prefix)
@@ -864,11 +864,11 @@ int enqueue_factor(BatchEngine *e)
 		++launches;
 		if (e->trsm_cnt[k] <= 0) continue;
 		btrsm_kernel<<<e->trsm_cnt[k], kTrsmThreads, kTrsmSmem, st>>>(e->dsys, e->trsm_items + e->trsm_off[k], e->A, e->lda,
-			e->L16, e->U16, k);
+			e->L16, e->U16, k, e->group * kBB, k % e->group);
 		HPLAI_CUDA_TRY(cudaGetLastError());
 		++launches;
 		if (e->tile_cnt[k] > 0) {
-			HPLAI_TRY(launch_schur_tiles(e->maps, e->tiles + e->tile_off[k], e->tile_cnt[k], (k % kGroup + 1) * kBB, 0, st));
+			HPLAI_TRY(launch_schur_tiles(e->maps, e->tiles + e->tile_off[k], e->tile_cnt[k], (k % e->group + 1) * kBB, 0, st));
 			++launches;
 		}
 	}
@@ -918,16 +918,12 @@ int capture(BatchEngine *e, cudaGraph_t *graph, cudaGraphExec_t *exec, F enqueue
 	return cudaGraphInstantiate(exec, g, 0) == cudaSuccess ? HPLAI_OK : HPLAI_ECUDA;
 }
 
-} // namespace
-
-int batched_create(BatchEngine **out, int count, const int *n, const int *nrhs, const uint64_t *seeds)
+// An engine whose updates take `group` panels at a time.
+int engine_make(BatchEngine **out, int group, int count, const int *n, const int *nrhs, const uint64_t *seeds)
 {
-	*out = nullptr;
-	if (count <= 0) return HPLAI_EINVAL;
-	for (int s = 0; s < count; ++s)
-		if (n[s] < 1 || nrhs[s] < 1 || nrhs[s] > kMaxRhs) return HPLAI_EINVAL;
 	BatchEngine *e = new BatchEngine;
 	e->count = count;
+	e->group = group;
 	std::vector<int> order(count);
 	std::iota(order.begin(), order.end(), 0);
 	std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return n[p] > n[q]; });
@@ -948,7 +944,7 @@ int batched_create(BatchEngine **out, int count, const int *n, const int *nrhs, 
 		S.pair0 = pair;
 		S.state0 = state_initial(seeds[s]);
 		rows += S.P;
-		cols += S.P + kBB;
+		cols += S.P;
 		voff += static_cast<int64_t>(S.n) * S.nrhs;
 		doff += S.n;
 		poff += static_cast<int64_t>((S.n + kGemvCols - 1) / kGemvCols) * S.nrhs * S.n;
@@ -1006,11 +1002,12 @@ int batched_create(BatchEngine **out, int count, const int *n, const int *nrhs, 
 		for (int i = 0; i < e->active[k]; ++i) {
 			const BSys &S = e->sys[i];
 			const int t0 = (k + 1) * kBB, t1 = t0 + kBB;
+			// half: the system's last 128 columns, nothing past them is written
 			auto tile = [&](int rr, int c, bool half) {
 				const int col = static_cast<int>(S.C + c);
 				tiles.push_back(make_int4(static_cast<int>(S.R + rr), static_cast<int>(S.R + c), rr, half ? ~col : col));
 			};
-			if ((k + 1) % kGroup == 0) {
+			if ((k + 1) % group == 0) {
 				for (int c = t0; c < S.P; c += 256)
 					for (int rr = t0; rr < S.P; rr += kBB) tile(rr, c, c + kBB == S.P);
 			} else {
@@ -1024,6 +1021,7 @@ int batched_create(BatchEngine **out, int count, const int *n, const int *nrhs, 
 	e->n_rows = static_cast<int>(rowi.size());
 	e->n_gemv = static_cast<int>(gemv.size());
 
+	const int ldk = group * kBB;   // a row's FP16 copies
 	int rc = HPLAI_OK;
 	auto alloc = [&](void **p, size_t bytes) {
 		if (rc == HPLAI_OK && cudaMalloc(p, bytes) != cudaSuccess) {
@@ -1033,8 +1031,8 @@ int batched_create(BatchEngine **out, int count, const int *n, const int *nrhs, 
 	};
 	if (rows > (int64_t(1) << 31) - 1 || cols > (int64_t(1) << 31) - 1) rc = HPLAI_EUNSUPPORTED;   // int tile coordinates
 	alloc(reinterpret_cast<void **>(&e->A), sizeof(float) * static_cast<size_t>(e->lda) * e->cols);
-	alloc(reinterpret_cast<void **>(&e->L16), sizeof(__half) * static_cast<size_t>(rows) * kLdK);
-	alloc(reinterpret_cast<void **>(&e->U16), sizeof(__half) * static_cast<size_t>(rows) * kLdK);
+	alloc(reinterpret_cast<void **>(&e->L16), sizeof(__half) * static_cast<size_t>(rows) * ldk);
+	alloc(reinterpret_cast<void **>(&e->U16), sizeof(__half) * static_cast<size_t>(rows) * ldk);
 	alloc(reinterpret_cast<void **>(&e->d), sizeof(double) * static_cast<size_t>(doff));
 	alloc(reinterpret_cast<void **>(&e->rhs), sizeof(double) * static_cast<size_t>(voff));
 	alloc(reinterpret_cast<void **>(&e->x), sizeof(double) * static_cast<size_t>(voff));
@@ -1062,7 +1060,7 @@ int batched_create(BatchEngine **out, int count, const int *n, const int *nrhs, 
 		rc = HPLAI_ECUDA;
 	if (rc == HPLAI_OK && cudaMemset(e->status, 0, sizeof(unsigned)) != cudaSuccess) rc = HPLAI_ECUDA;
 	if (rc == HPLAI_OK) rc = schur_make_maps(&e->maps, reinterpret_cast<const uint16_t *>(e->L16),
-		static_cast<int>(rows), kLdK, reinterpret_cast<const uint16_t *>(e->U16), static_cast<int>(rows), kLdK, kLdK);
+		static_cast<int>(rows), ldk, reinterpret_cast<const uint16_t *>(e->U16), static_cast<int>(rows), ldk, ldk);
 	if (rc == HPLAI_OK) rc = schur_set_cmap(&e->maps, e->A, e->pmax, static_cast<int>(e->cols), e->lda);
 	if (rc == HPLAI_OK && !e->maps.has_cmap) rc = HPLAI_EINVAL;
 	e->maps.status = e->status;
@@ -1081,6 +1079,20 @@ int batched_create(BatchEngine **out, int count, const int *n, const int *nrhs, 
 	e->h_iters.assign(pair, 0);
 	*out = e;
 	return HPLAI_OK;
+}
+
+} // namespace
+
+int batched_create(BatchEngine **out, int count, const int *n, const int *nrhs, const uint64_t *seeds)
+{
+	*out = nullptr;
+	if (count <= 0) return HPLAI_EINVAL;
+	for (int s = 0; s < count; ++s)
+		if (n[s] < 1 || nrhs[s] < 1 || nrhs[s] > kMaxRhs) return HPLAI_EINVAL;
+	const int rc = engine_make(out, kGroup, count, n, nrhs, seeds);
+	// out of memory shows as either: the copies of four panels take 2 KB a matrix
+	// row, of one 512 bytes
+	return rc == HPLAI_ENOMEM || rc == HPLAI_ECUDA ? engine_make(out, 1, count, n, nrhs, seeds) : rc;
 }
 
 void batched_destroy(BatchEngine *e) { engine_free(e); }

@@ -133,10 +133,9 @@ int launch_schur_store(const SchurMaps &maps, int lrow0, int urow0, int m, int n
 int launch_schur_deck(const SchurMaps &maps, bool fp8, const float *sl, int sl0, const float *su, int su0, int lrow0,
 	int urow0, int m, int n, int crow0, int ccol0, float dscale, int max_ctas, cudaStream_t st);
 // The batched form: `ntiles` 128 x 256 tiles, tile t updating C rows
-// tiles[t].z.. and columns tiles[t].w.. of the matrix given to
-// schur_set_cmap with L rows tiles[t].x.. and U rows tiles[t].y.. (FP16
-// maps); a tile may reach past the columns of its system into columns nobody
-// reads (or past the matrix, where it is clipped).
+// tiles[t].z.. and columns tiles[t].w.. (given as ~c: the 128 columns from c on
+// alone) of the matrix given to schur_set_cmap with L rows tiles[t].x.. and U
+// rows tiles[t].y.. (FP16 maps), the first k columns of both.
 int launch_schur_tiles(const SchurMaps &maps, const int4 *tiles, int ntiles, int k, int max_ctas, cudaStream_t st);
 int schur_status();          // the library's word: HPLAI_ETIMEOUT if a device wait ran out since the last reset
 void schur_status_reset();

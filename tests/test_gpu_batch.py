@@ -134,3 +134,34 @@ def test_batch_workload_512_systems(hplai, oracle, torch_cuda):
                 bound = np.abs(r).max() / (norma * np.abs(x[:, c]).max() + np.abs(bs[:, c]).max()) * 2.0 / (m * eps)
                 assert bound < 16.0, (s, c, bound)
         assert dense_checked > 100
+
+
+def test_batch_systems_leave_their_neighbours_alone(hplai, torch_cuda):
+    """Systems side by side, odd and even numbers of 128-blocks: each has the factors that it has alone."""
+    n = [640, 384, 129, 1152, 128, 900, 5, 512]
+    with hplai.Batch(n, [1] * len(n), list(range(11, 11 + len(n)))) as bt:
+        assert bt.solve() == hplai.HPLAI_OK
+        together = [bt.lu(s) for s in range(len(n))]
+    for s, m in enumerate(n):
+        with hplai.Batch([m], [1], [11 + s]) as bt:
+            assert bt.solve() == hplai.HPLAI_OK
+            assert np.array_equal(bt.lu(0).view(np.uint32), together[s].view(np.uint32)), m
+
+
+def test_batch_where_memory_is_short(hplai, oracle, torch_cuda):
+    """With room for the matrices and the FP16 copies of one panel (2.1 and 0.53 GB), not of four (2.1 GB), a batch is
+    created and solves one panel at a time."""
+    torch = torch_cuda
+    n = [500] * 2000
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    filler = torch.empty(free - (3400 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        with hplai.Batch(n, [1] * len(n), list(range(len(n)))) as bt:
+            assert bt.solve() == hplai.HPLAI_OK
+            for s in (0, 999, 1999):
+                ref = np.linalg.solve(oracle.dense_matrix_f64(500, s), oracle.rhs_cols(500, s, 0, 1))
+                assert np.abs(bt.x(s) - ref).max() <= 1e-12 * np.abs(ref).max()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
