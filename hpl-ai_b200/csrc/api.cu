@@ -579,10 +579,12 @@ bool f16_panel_form(const hplai_ctx *c, bool simt)
 // products are seven or more dependent launches that a small panel does not
 // fill.  Measured (tensor cores / one launch): b = 60, 600 rows 42 / 11 us,
 // 9600 43 / 31, 39960 69 / 86; b = 128, 9600 48 / 45, 19968 56 / 76; b = 256,
-// 2304 71 / 36, 9472 79 / 83; b = 512, 2048 109 / 94, 4608 118 / 189.
+// 2304 71 / 36, 9472 79 / 83; b = 512, 1536 104 / 96, 2048 109 / 94, 4608
+// 118 / 189.  In wider blocks the substitution's chain alone takes longer:
+// b = 640, 640 rows 131 / 137; 768 145 / 189; 1024 178 / 315.
 bool pair_panel_form(const hplai_ctx *c, int rem)
 {
-	return c->precision == HPLAI_F32_F16 && static_cast<int64_t>(rem) * c->b <= 1200000;
+	return c->precision == HPLAI_F32_F16 && c->b <= 512 && static_cast<int64_t>(rem) * c->b <= 1200000;
 }
 
 // Factor the diagonal block of step k and form its two panels with their

@@ -120,6 +120,12 @@ def test_inverse_panels_at_block_edges(hplai, torch_cuda, n, b):
     assert np.all(np.abs(urow - uref) <= eps * (np.abs(np.linalg.inv(l)) @ np.abs(l) @ np.abs(uref)))
 
 
+@pytest.mark.parametrize("n,b", [(1539, 513), (1280, 640), (2048, 1024)])
+def test_inverse_panels_of_wide_blocks(hplai, torch_cuda, n, b):
+    """Past b = 512 the last panels, however small, are formed by the inverses as well."""
+    test_inverse_panels_at_block_edges(hplai, torch_cuda, n, b)
+
+
 def test_inverse_panels_of_extreme_diagonals(hplai, torch_cuda):
     """The panels by inverses (the precision form's TF32 path) under a diagonal block with an infinite pivot, one whose
     reciprocal is subnormal and, last, one whose reciprocal overflows: as in the substitution, x / inf is 0 and every other
