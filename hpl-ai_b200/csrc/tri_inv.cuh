@@ -130,8 +130,8 @@ __device__ __noinline__ void invert_block(R *smem, const float *__restrict__ a, 
 			float f[16];
 #pragma unroll
 			for (int q = 0; q < 16; ++q) {
-				const int l = l0 + 2 * (16 * h + q);
-				f[q] = s < rows && l < rows ? __ldcg(&a[static_cast<int64_t>(r0 + l) * lda + r0 + s]) : 0.f;
+				const int l = min(l0 + 2 * (16 * h + q), rows - 1);   // put() drops what is past the last
+				f[q] = __ldcg(&a[static_cast<int64_t>(r0 + l) * lda + r0 + min(s, rows - 1)]);
 			}
 #pragma unroll
 			for (int q = 0; q < 16; ++q) put(l0 + 2 * (16 * h + q), s, f[q]);
