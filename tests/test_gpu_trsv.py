@@ -106,6 +106,18 @@ def test_trsv_leaf_quotients(hplai, torch_cuda):
     assert np.all(np.abs(x - ref) <= 2.0 ** -52 * np.abs(ref))
 
 
+def test_trsv_leaf_inverse_quotients(hplai, torch_cuda):
+    """An ordinary diagonal U takes its inverse: the corrected reciprocal (1/2 ulp but for a few parts in 2^50) and the
+    product's rounding, 2^-53 of the quotient each."""
+    rng = np.random.default_rng(4)
+    n = 1000
+    d = (rng.uniform(1, 2, n) * 2.0 ** rng.integers(-55, 55, n) * rng.choice((-1, 1), n)).astype(np.float32)
+    b = rng.uniform(-1, 1, n)
+    ref = b / d.astype(np.float64)
+    x = _leaf(hplai, torch_cuda, np.diag(d), b, False)
+    assert np.all(np.abs(x - ref) <= 2.0 ** -52 * (1 + 2.0 ** -20) * np.abs(ref))
+
+
 @pytest.mark.parametrize("lower", [True, False])
 def test_trsv_leaf_infinite_entry(hplai, torch_cuda, lower):
     """The rows solved before the one with an infinite right-hand side do not see it."""
