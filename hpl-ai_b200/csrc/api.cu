@@ -930,9 +930,10 @@ int factor_impl(hplai_ctx *c, int kend, const float *host_a = nullptr, int64_t h
 	// starting at block e: a fixed count (side_sms > 0) or, with side_sms < 0,
 	// a share of c = -side_sms panels against the remaining trailing blocks,
 	// sms * c / (rem / b + c): the panel work grows with rem, the update with
-	// rem^2, so the side stream needs more SMs as the matrix shrinks.  A share
-	// above one half forms the group's panels on the whole GPU before the
-	// rest of the update (no overlap).  0: no overlap.
+	// rem^2, so the side stream needs more SMs as the matrix shrinks.  With a
+	// share above one half nothing overlaps: the update in one launch, then the
+	// group's panels on the whole GPU (b % 4 != 0: the panels before the rest of
+	// the split update).  0: no overlap.
 	auto side_for = [&](int e) -> int {
 		if (serial) return 0;
 		int side = c->side_sms;
@@ -1016,10 +1017,8 @@ int factor_impl(hplai_ctx *c, int kend, const float *host_a = nullptr, int64_t h
 	HPLAI_CUDA_TRY(cudaEventRecord(c->ev_panel, sd));
 	HPLAI_CUDA_TRY(cudaStreamWaitEvent(st, c->ev_panel, 0));
 	// inverses of the factors' 128 x 128 diagonal blocks for the refinement's
-	// solves, in one launch of all blocks (made per panel instead, each
-	// block's ~0.2 ms substitution lengthened the panel chain: 7 ms more at
-	// n = 8192, b = 256 and 11 ms at n = 65536, b = 1024 with look-ahead,
-	// against 0.24 and 1.5 ms here)
+	// solves, in one launch of all blocks (0.03 ms at n = 8192, 0.2 at 65536)
+	// and not on the chain of the panels
 	HPLAI_TRY(pe.record(st, HPLAI_PH_IR_TRSV));
 	HPLAI_TRY(launch_trsv_dinv(n, c->A, c->lda, c->dinv, st));
 	HPLAI_TRY(pe.end(st));

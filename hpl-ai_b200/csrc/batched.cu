@@ -635,7 +635,7 @@ __device__ __forceinline__ bool any_live(const BSys &S, const int *__restrict__ 
 // nbk-1-t) inverted in FP64 in shared memory (invert_block: short chains over
 // all threads instead of 128 dependent steps of one warp) and applied as one
 // product, thread (row, half) taking every other right-hand side.  512
-// systems' blocks: 41 us (75 as a substitution, a warp per right-hand side).
+// systems' blocks: 44 us (75 as a substitution, a warp per right-hand side).
 __global__ void __launch_bounds__(kTrsvThreads) btrsv_diag_kernel(const BSys *__restrict__ sys,
 	const float *__restrict__ A, int64_t lda, const int *__restrict__ state, double *__restrict__ r, int t, int up)
 {

@@ -24,9 +24,10 @@
 // last two being applied by CTA 0.  A worker team keeps its tiles in shared
 // memory where they fit, so a trailing update reads only its two operands and
 // writes nothing until the tile is final or handed over.
-// One block alone, before (a tile per warp, the chain on one eight-warp CTA,
-// progress words behind fences) / now: b = 60 26 / 15 us, 240 120 / 54, 512
-// 277 / 107, 1024 522 / 235.
+// A block within a factorisation, before (a tile per warp, the chain on one
+// eight-warp CTA, progress words behind fences) / now: b = 60 29 / 16 us, 240
+// 125 / 57, 512 257 / 108, 1024 517 / 226; through the leaf entry point, which
+// waits for the status, 512 276 / 125.
 // Every wait is on work the producer reaches without waiting on the waiter,
 // so the dataflow always completes (all CTAs are resident: cooperative
 // launch); every wait is bounded, and a timeout sets the status word and the

@@ -538,9 +538,10 @@ __device__ __forceinline__ bool inverse_serves(const double (&inv)[TB / 2], cons
 //    short FMA chains.  Nothing behind a leaf call corrects that product, so
 //    without dinv a block that fails inverse_serves is solved by substitution.
 // Measured per triangle, before (flag word and fence, 128-step substitution
-// without dinv) and now: n = 8192 197 -> 111 us, transposed 584 -> 135;
-// n = 65536 2.64 -> 2.40 ms (3.6 TB/s); without dinv n = 16384 2370 -> 270 us
-// (6 of them the condition numbers; 790 where every block is substituted).
+// without dinv) and now: n = 8192 204 -> 114 us, transposed 590 -> 139;
+// n = 65536 2.45 -> 2.13 ms (4.0 TB/s), 131072 8.28 -> 7.70; without dinv
+// n = 16384 2370 -> 263 us (256 without the condition numbers; 785 where every
+// block is substituted).
 template <bool TRANS, bool HAVE_INV>
 __global__ void __launch_bounds__(TRSV_THREADS, 1) trsv_kernel(int lower, int n, const float *__restrict__ a,
 	int64_t lda, double *x, TrsvWork *w, ulonglong2 *xt, const double *__restrict__ dinv)
@@ -1058,7 +1059,8 @@ int launch_axpy1(int n, const double *x, double *y, cudaStream_t st)
 // solve loop that must not call cudaMalloc because it can synchronise the
 // device) get the GEMV's partial-sum scratch from this fixed array instead
 // of a caller workspace.  It is part of the library image: every GPU that
-// loads libhplai holds its 4 MiB until the process exits.  It covers orders
+// loads libhplai holds its 4 MiB until the process exits (beside the 8 MiB of
+// the leaf diagonal LU, getrf.cu).  It covers orders
 // up to kNoAllocMaxN (ceil(n/2048) * n doubles).  All calls share it.
 // ---------------------------------------------------------------------------
 constexpr int kNoAllocMaxN = 32768;

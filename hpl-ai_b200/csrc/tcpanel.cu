@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(256) tri_f16_kernel(int b, const float *__rest
 // A final pass writes the hi/lo TF32 split of X for the tensor-core panels.
 // ---------------------------------------------------------------------------
 // grid (128-blocks, 2): blockIdx.y = 0 -> U11, 1 -> L11^T.  Latency-bound: one
-// launch (17 us at b = 1024, 18 at 240) in place of a one-warp substitution per
+// launch (19 us at b = 1024, 22 at 240) in place of a one-warp substitution per
 // 32 x 32 tile and the products of the h = 32 and 64 levels, each a launch.
 // With one block in all (hi given) its TF32 split follows here as well.
 __global__ void __launch_bounds__(kTriThreads) tri_block_kernel(int b, int bp, const float *__restrict__ lu,

@@ -23,7 +23,7 @@ constexpr int kTriThreads = 256;
 // warp are 16 neighbouring doubles or a broadcast.  Bound by shared-memory
 // reads (two 64-bit ones per four multiply-adds of a product) after the one
 // latency of loading the block.  The diagonal blocks of both factors of
-// n = 9600: 415 us as one substitution thread per column, 35 us so.
+// n = 9600: 420 us as one substitution thread per column, 42 us so.
 constexpr int kInvLd = kTriBlock + 1;
 constexpr int kInvLdW = kTriBlock / 2 + 1;
 template <typename R>

@@ -418,7 +418,9 @@ int hplai_gen_rhs_cols(int n, uint64_t seed, int first, int count, double *out, 
 int hplai_gen_diag(int n, uint64_t seed, int i0, int count, double *d, void *stream);
 
 /* getrf_nopiv<float> (getrf_nopiv.hpp:124-141): b x b no-pivot LU in place,
- * b <= 1024. */
+ * b <= 1024.  Its workspace is part of the library (8 MiB on every GPU that
+ * loads it, held until the process exits); calls are serialised and wait for
+ * the result. */
 int hplai_getrf_nopiv(int b, float *a, int64_t lda, void *stream);
 
 /* update_left_panels + convert_left_panels (panel_trf.hpp:143-157,182-207):
