@@ -34,41 +34,46 @@ namespace hplai {
 //
 // Bound by the chain of 16-column solves, and by FP32 issue and the operands'
 // shared-memory reads in the products.  A CTA owns 32 RL rows; a thread holds RL rows (lane,
-// lane + 32) of 16 columns (its warp's) of a 128-column block in registers.
+// lane + 32) of 16 columns (its warp's) of a block of 16 columns per warp in registers.
 // Per block: the products with the columns solved before (X and T in chunks
-// of 32 p through three cp.async stages), then the block's own triangle 16
+// of 32 p through two or three cp.async stages), then the block's own triangle 16
 // columns at a time -- the owning warp solves them in registers and publishes
 // them, every later warp applies them (one barrier per 16 columns).  8200 rows,
 // b = 512: 124 us a panel (270 with rows staged in shared memory and 4 x 4
 // products, two shared-memory reads per four FMAs).
 // ---------------------------------------------------------------------------
-constexpr int kTrsmThreads = 256;
-constexpr int kTB = 128;          // columns per block: 16 per warp
 constexpr int kMicro = 16;
 constexpr int kKC = 32;           // p per chunk
-constexpr int kStages = 3;
-constexpr int kLdTri = kTB + 4;
 constexpr int kLdP = kKC + 4;     // chunk rows that run along p
 
-template <int RL, bool UPANEL>
-struct TrsmSmem {
+// NW warps: columns in blocks of 16 per warp, 32 RL rows.
+template <int NW, int RL, bool UPANEL>
+struct Trsm {
+	static constexpr int threads = 32 * NW;
+	static constexpr int TB = kMicro * NW;
 	static constexpr int R = 32 * RL;
+	static constexpr int STAGES = NW == 8 ? 3 : 2;   // two, where three CTAs share an SM
+	static constexpr int LDTRI = TB + 4;
 	static constexpr int LDX = UPANEL ? kLdP : R + 4;        // X chunk: [r][p] or [p][r]
-	static constexpr int LDT = UPANEL ? kLdTri : kLdP;       // T chunk: [p][c] or [c][p]
+	static constexpr int LDT = UPANEL ? LDTRI : kLdP;        // T chunk: [p][c] or [c][p]
 	static constexpr int XC = (UPANEL ? R : kKC) * LDX;
-	static constexpr int TC = (UPANEL ? kKC : kTB) * LDT;
-	static constexpr size_t bytes = sizeof(float) *
-		(kTB * kLdTri + kTB + 2 * kMicro * R + kStages * static_cast<size_t>(XC + TC));
+	static constexpr int TC = (UPANEL ? kKC : TB) * LDT;
+	// the chunks belong to the blocks after the first
+	static constexpr size_t bytes(int b)
+	{
+		return sizeof(float) * (TB * LDTRI + TB + 2 * kMicro * R + (b > TB ? STAGES * static_cast<size_t>(XC + TC) : 0));
+	}
 };
 
 // lines x len floats, line l at src + l * lds, to dst + l * ldd; lines from
 // nl on and elements from ne on are zero.
+template <int THREADS>
 __device__ __forceinline__ void stage_lines(float *dst, int ldd, const float *src, int64_t lds, int lines, int len,
 	int nl, int ne, bool vec)
 {
 	if (vec) {
 		const int g4 = len / 4;
-		for (int e = threadIdx.x; e < lines * g4; e += kTrsmThreads) {
+		for (int e = threadIdx.x; e < lines * g4; e += THREADS) {
 			const int l = e / g4, g = (e % g4) * 4;
 			int bytes = l < nl ? (ne - g) * 4 : 0;
 			bytes = bytes < 0 ? 0 : (bytes > 16 ? 16 : bytes);
@@ -77,7 +82,7 @@ __device__ __forceinline__ void stage_lines(float *dst, int ldd, const float *sr
 				"r"(bytes) : "memory");
 		}
 	} else {
-		for (int e = threadIdx.x; e < lines * len; e += kTrsmThreads) {
+		for (int e = threadIdx.x; e < lines * len; e += THREADS) {
 			const int l = e / len, g = e % len;
 			if (l < nl && g < ne)
 				dst[l * ldd + g] = __ldcg(src + static_cast<int64_t>(l) * lds + g);
@@ -87,65 +92,66 @@ __device__ __forceinline__ void stage_lines(float *dst, int ldd, const float *sr
 	}
 }
 
-template <int RL, bool UPANEL>
+template <int NW, int RL, bool UPANEL>
 __device__ __forceinline__ void trsm_rows(float *sm, int m, int b, const float *__restrict__ t, int64_t ldt, float *a,
 	int64_t lda, __half *__restrict__ hc, int64_t ldh, float scale, int vec_x, int vec_t)
 {
-	using S = TrsmSmem<RL, UPANEL>;
-	constexpr int R = S::R;
+	using S = Trsm<NW, RL, UPANEL>;
+	constexpr int R = S::R, TB = S::TB, LDTRI = S::LDTRI, THREADS = S::threads, STAGES = S::STAGES;
 	constexpr bool UNIT = UPANEL;   // L11^T has a unit diagonal
-	float *tri = sm;                      // tri[i * kLdTri + j] = T[j0 + i][j0 + j]
-	float *inv = tri + kTB * kLdTri;
-	float *pub = inv + kTB;               // [2][16][R]
-	float *chunks = pub + 2 * kMicro * R; // kStages x (X chunk, T chunk)
+	float *tri = sm;                      // tri[i * LDTRI + j] = T[j0 + i][j0 + j]
+	float *inv = tri + TB * LDTRI;
+	float *pub = inv + TB;               // [2][16][R]
+	float *chunks = pub + 2 * kMicro * R; // STAGES x (X chunk, T chunk)
 	const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
 	const int row0 = blockIdx.x * R, rows = min(R, m - row0);
 	const int e0 = kMicro * wp;
-	for (int j0 = 0; j0 < b; j0 += kTB) {
-		const int jw = min(kTB, b - j0), nc = j0 / kKC;
+	for (int j0 = 0; j0 < b; j0 += TB) {
+		const int jw = min(TB, b - j0), nc = j0 / kKC;
 		auto stage = [&](int q) {
 			if (q < nc) {
-				float *xc = chunks + (q % kStages) * (S::XC + S::TC), *tc = xc + S::XC;
+				float *xc = chunks + (q % STAGES) * (S::XC + S::TC), *tc = xc + S::XC;
 				const int p0 = q * kKC;
 				if (UPANEL) {
-					stage_lines(xc, S::LDX, a + static_cast<int64_t>(row0) * lda + p0, lda, R, kKC, rows, kKC, vec_x != 0);
-					stage_lines(tc, S::LDT, t + static_cast<int64_t>(p0) * ldt + j0, ldt, kKC, kTB, kKC, jw, vec_t != 0);
+					stage_lines<THREADS>(xc, S::LDX, a + static_cast<int64_t>(row0) * lda + p0, lda, R, kKC, rows, kKC, vec_x != 0);
+					stage_lines<THREADS>(tc, S::LDT, t + static_cast<int64_t>(p0) * ldt + j0, ldt, kKC, TB, kKC, jw, vec_t != 0);
 				} else {
-					stage_lines(xc, S::LDX, a + static_cast<int64_t>(p0) * lda + row0, lda, kKC, R, kKC, rows, vec_x != 0);
-					stage_lines(tc, S::LDT, t + static_cast<int64_t>(j0) * ldt + p0, ldt, kTB, kKC, jw, kKC, vec_t != 0);
+					stage_lines<THREADS>(xc, S::LDX, a + static_cast<int64_t>(p0) * lda + row0, lda, kKC, R, kKC, rows, vec_x != 0);
+					stage_lines<THREADS>(tc, S::LDT, t + static_cast<int64_t>(j0) * ldt + p0, ldt, TB, kKC, jw, kKC, vec_t != 0);
 				}
 			}
 			asm volatile("cp.async.commit_group;" ::: "memory");
 		};
-		for (int q = 0; q < kStages - 1; ++q) stage(q);
+		for (int q = 0; q < STAGES - 1; ++q) stage(q);
 		// this block's triangle (rows and columns past jw zero) and columns; the
 		// loads of each are all in flight together
 		if (UPANEL) {
-			stage_lines(tri, kLdTri, t + static_cast<int64_t>(j0) * ldt + j0, ldt, kTB, kTB, jw, jw, vec_t != 0);
+			stage_lines<THREADS>(tri, LDTRI, t + static_cast<int64_t>(j0) * ldt + j0, ldt, TB, TB, jw, jw, vec_t != 0);
 			asm volatile("cp.async.commit_group;" ::: "memory");
 		} else if (vec_t && jw % 4 == 0) {
 			const int c = tid % 32, r4 = (tid / 32) * 4;   // lanes along the columns: rows of T without bank conflicts
-			float4 f[16];
+			constexpr int G = TB / 32;   // groups of 32 columns
+			float4 f[4 * G];
 #pragma unroll
-			for (int q = 0; q < 16; ++q) {
-				const int cc = c + 32 * (q & 3), rr = r4 + 32 * (q >> 2);
+			for (int q = 0; q < 4 * G; ++q) {
+				const int cc = c + 32 * (q % G), rr = r4 + 4 * NW * (q / G);
 				f[q] = make_float4(0.f, 0.f, 0.f, 0.f);
 				if (cc < jw && rr < jw)
 					f[q] = __ldcg(reinterpret_cast<const float4 *>(t + static_cast<int64_t>(j0 + cc) * ldt + j0 + rr));
 			}
 #pragma unroll
-			for (int q = 0; q < 16; ++q) {
-				const int cc = c + 32 * (q & 3), rr = r4 + 32 * (q >> 2);
-				tri[rr * kLdTri + cc] = f[q].x;
-				tri[(rr + 1) * kLdTri + cc] = f[q].y;
-				tri[(rr + 2) * kLdTri + cc] = f[q].z;
-				tri[(rr + 3) * kLdTri + cc] = f[q].w;
+			for (int q = 0; q < 4 * G; ++q) {
+				const int cc = c + 32 * (q % G), rr = r4 + 4 * NW * (q / G);
+				tri[rr * LDTRI + cc] = f[q].x;
+				tri[(rr + 1) * LDTRI + cc] = f[q].y;
+				tri[(rr + 2) * LDTRI + cc] = f[q].z;
+				tri[(rr + 3) * LDTRI + cc] = f[q].w;
 			}
 		} else {
 #pragma unroll 16
-			for (int e = tid; e < kTB * kTB; e += kTrsmThreads) {
-				const int p = e % kTB, j = e / kTB;
-				tri[p * kLdTri + j] = (p < jw && j < jw) ? __ldcg(t + static_cast<int64_t>(j0 + j) * ldt + j0 + p) : 0.f;
+			for (int e = tid; e < TB * TB; e += THREADS) {
+				const int p = e % TB, j = e / TB;
+				tri[p * LDTRI + j] = (p < jw && j < jw) ? __ldcg(t + static_cast<int64_t>(j0 + j) * ldt + j0 + p) : 0.f;
 			}
 		}
 		float x[RL][kMicro];
@@ -172,10 +178,10 @@ __device__ __forceinline__ void trsm_rows(float *sm, int m, int b, const float *
 			}
 		}
 		for (int q = 0; q < nc; ++q) {
-			asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+			asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
 			__syncthreads();   // chunk q is here; everyone is done with the one before it
-			stage(q + kStages - 1);
-			const float *xc = chunks + (q % kStages) * (S::XC + S::TC), *tc = xc + S::XC;
+			stage(q + STAGES - 1);
+			const float *xc = chunks + (q % STAGES) * (S::XC + S::TC), *tc = xc + S::XC;
 #pragma unroll 2
 			for (int p = 0; p < kKC; p += 4) {
 				float xp[RL][4];
@@ -223,7 +229,7 @@ __device__ __forceinline__ void trsm_rows(float *sm, int m, int b, const float *
 		}
 		asm volatile("cp.async.wait_all;" ::: "memory");
 		__syncthreads();   // the triangle is here
-		if (!UNIT && tid < kTB) inv[tid] = tid < jw ? 1.0f / tri[tid * kLdTri + tid] : 0.f;
+		if (!UNIT && tid < TB) inv[tid] = tid < jw ? 1.0f / tri[tid * LDTRI + tid] : 0.f;
 		if (!UNIT) __syncthreads();
 		const int nmicro = (jw + kMicro - 1) / kMicro;
 		for (int oi = 0; oi < nmicro; ++oi) {
@@ -237,7 +243,7 @@ __device__ __forceinline__ void trsm_rows(float *sm, int m, int b, const float *
 						if (!UNIT) x[r][li] *= inv[i];
 						pb[li * R + 32 * r] = x[r][li];
 					}
-					const float4 *row = reinterpret_cast<const float4 *>(tri + i * kLdTri + e0);
+					const float4 *row = reinterpret_cast<const float4 *>(tri + i * LDTRI + e0);
 #pragma unroll
 					for (int g = (li + 1) / 4; g < kMicro / 4; ++g) {
 						const float4 v = row[g];
@@ -259,7 +265,7 @@ __device__ __forceinline__ void trsm_rows(float *sm, int m, int b, const float *
 					float xi[RL];
 #pragma unroll
 					for (int r = 0; r < RL; ++r) xi[r] = pb[li * R + 32 * r];
-					const float4 *row = reinterpret_cast<const float4 *>(tri + (kMicro * oi + li) * kLdTri + e0);
+					const float4 *row = reinterpret_cast<const float4 *>(tri + (kMicro * oi + li) * LDTRI + e0);
 #pragma unroll
 					for (int g = 0; g < kMicro / 4; ++g) {
 						const float4 v = row[g];
@@ -312,40 +318,41 @@ __device__ __forceinline__ void trsm_rows(float *sm, int m, int b, const float *
 	}
 }
 
-template <int RL, bool UPANEL>
-__global__ void __launch_bounds__(kTrsmThreads) trsm_kernel(int m, int b, const float *__restrict__ t, int64_t ldt,
+template <int NW, int RL, bool UPANEL>
+__global__ void __launch_bounds__(32 * NW) trsm_kernel(int m, int b, const float *__restrict__ t, int64_t ldt,
 	float *a, int64_t lda, __half *__restrict__ hc, int64_t ldh, float scale, int vec_x, int vec_t)
 {
 	extern __shared__ __align__(16) float sm[];
-	trsm_rows<RL, UPANEL>(sm, m, b, t, ldt, a, lda, hc, ldh, scale, vec_x, vec_t);
+	trsm_rows<NW, RL, UPANEL>(sm, m, b, t, ldt, a, lda, hc, ldh, scale, vec_x, vec_t);
 }
 
 // Both panels of a step in one launch (blockIdx.y = 0: L, 1: U), the
 // triangles and panels in one matrix.
+constexpr int kPairWarps = 8;
 template <int RL>
-__global__ void __launch_bounds__(kTrsmThreads) trsm_pair_kernel(int rem, int b, const float *__restrict__ lu, float *acol,
+__global__ void __launch_bounds__(32 * kPairWarps) trsm_pair_kernel(int rem, int b, const float *__restrict__ lu, float *acol,
 	float *arow, int64_t lda, __half *__restrict__ lh, __half *__restrict__ uh, int64_t ldh, int vec)
 {
 	extern __shared__ __align__(16) float sm[];
 	if (blockIdx.y == 0)
-		trsm_rows<RL, false>(sm, rem, b, lu, lda, acol, lda, lh, ldh, 1.0f, vec, vec);
+		trsm_rows<kPairWarps, RL, false>(sm, rem, b, lu, lda, acol, lda, lh, ldh, 1.0f, vec, vec);
 	else
-		trsm_rows<RL, true>(sm, rem, b, lu, lda, arow, lda, uh, ldh, 1.0f, vec, vec);
+		trsm_rows<kPairWarps, RL, true>(sm, rem, b, lu, lda, arow, lda, uh, ldh, 1.0f, vec, vec);
 }
 
-template <int RL, bool UPANEL>
+template <int NW, int RL, bool UPANEL>
 static int trsm_launch(int m, int b, const float *t, int64_t ldt, float *a, int64_t lda, uint16_t *hc, int64_t ldh,
 	float scale, cudaStream_t st)
 {
-	constexpr size_t smem = TrsmSmem<RL, UPANEL>::bytes;
+	using S = Trsm<NW, RL, UPANEL>;
 	static DeviceOnce attr;
 	HPLAI_TRY(attr.get([](int, int *) -> int {
-		HPLAI_CUDA_TRY(cudaFuncSetAttribute(trsm_kernel<RL, UPANEL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			static_cast<int>(smem)));
+		HPLAI_CUDA_TRY(cudaFuncSetAttribute(trsm_kernel<NW, RL, UPANEL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			static_cast<int>(S::bytes(1024))));
 		return HPLAI_OK;
 	}));
 	auto vec = [](const float *p, int64_t ld) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0 && ld % 4 == 0 ? 1 : 0; };
-	trsm_kernel<RL, UPANEL><<<(m + 32 * RL - 1) / (32 * RL), kTrsmThreads, smem, st>>>(m, b, t, ldt, a, lda,
+	trsm_kernel<NW, RL, UPANEL><<<(m + 32 * RL - 1) / (32 * RL), 32 * NW, S::bytes(b), st>>>(m, b, t, ldt, a, lda,
 		reinterpret_cast<__half *>(hc), ldh, scale, vec(a, lda), vec(t, ldt));
 	count_launches();
 	HPLAI_CUDA_TRY(cudaGetLastError());
@@ -353,13 +360,24 @@ static int trsm_launch(int m, int b, const float *t, int64_t ldt, float *a, int6
 }
 
 // 64 rows per CTA reuse each triangle read twice; below 74 such CTAs half the
-// GPU would idle, and 32 rows per CTA are faster.
+// GPU would idle, and 32 rows per CTA are faster.  Eight warps have the shortest
+// chain, but one such CTA fills an SM: past one wave of them (9472 rows) four
+// warps, three CTAs an SM, are faster (L panel, four / eight warps: b = 128, 10000
+// rows 29 / 35 us, 40000 61 / 87; b = 200, 40000 135 / 177; b = 512, 10000 211 / 238,
+// 8200 157 / 123).  A narrower panel has no work for more warps than 16 columns
+// each: b = 60, 40000 rows 24 / 49 us, b = 31 two / eight warps 14 / 40.
 template <bool UPANEL>
 static int trsm_pick(int m, int b, const float *t, int64_t ldt, float *a, int64_t lda, uint16_t *hc, int64_t ldh,
 	float scale, cudaStream_t st)
 {
-	if (m > 64 * 74) return trsm_launch<2, UPANEL>(m, b, t, ldt, a, lda, hc, ldh, scale, st);
-	return trsm_launch<1, UPANEL>(m, b, t, ldt, a, lda, hc, ldh, scale, st);
+	if (b <= 32) {
+		if (m > 16000) return trsm_launch<2, 2, UPANEL>(m, b, t, ldt, a, lda, hc, ldh, scale, st);
+		return trsm_launch<2, 1, UPANEL>(m, b, t, ldt, a, lda, hc, ldh, scale, st);
+	}
+	if (m > 64 * (b <= 64 ? 74 : 148)) return trsm_launch<4, 2, UPANEL>(m, b, t, ldt, a, lda, hc, ldh, scale, st);
+	if (b <= 64) return trsm_launch<4, 1, UPANEL>(m, b, t, ldt, a, lda, hc, ldh, scale, st);
+	if (m > 64 * 74) return trsm_launch<8, 2, UPANEL>(m, b, t, ldt, a, lda, hc, ldh, scale, st);
+	return trsm_launch<8, 1, UPANEL>(m, b, t, ldt, a, lda, hc, ldh, scale, st);
 }
 
 static bool vec_ok(const uint16_t *hc, int64_t ldh)
@@ -387,15 +405,17 @@ template <int RL>
 static int pair_launch(int rem, int b, const float *diag, float *acol, float *arow, int64_t lda, uint16_t *lh,
 	uint16_t *uh, int64_t ldh, cudaStream_t st)
 {
-	constexpr size_t sl = TrsmSmem<RL, false>::bytes, su = TrsmSmem<RL, true>::bytes, smem = sl > su ? sl : su;
+	using SL = Trsm<kPairWarps, RL, false>;
+	using SU = Trsm<kPairWarps, RL, true>;
+	auto bytes = [](int w) { return SL::bytes(w) > SU::bytes(w) ? SL::bytes(w) : SU::bytes(w); };
 	static DeviceOnce attr;
 	HPLAI_TRY(attr.get([](int, int *) -> int {
 		HPLAI_CUDA_TRY(cudaFuncSetAttribute(trsm_pair_kernel<RL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			static_cast<int>(smem)));
+			static_cast<int>(SL::bytes(1024) > SU::bytes(1024) ? SL::bytes(1024) : SU::bytes(1024))));
 		return HPLAI_OK;
 	}));
 	const int vec = (reinterpret_cast<uintptr_t>(diag) & 15u) == 0 && lda % 4 == 0 && b % 4 == 0 ? 1 : 0;
-	trsm_pair_kernel<RL><<<dim3((rem + 32 * RL - 1) / (32 * RL), 2), kTrsmThreads, smem, st>>>(rem, b, diag, acol, arow,
+	trsm_pair_kernel<RL><<<dim3((rem + 32 * RL - 1) / (32 * RL), 2), 32 * kPairWarps, bytes(b), st>>>(rem, b, diag, acol, arow,
 		lda, reinterpret_cast<__half *>(lh), reinterpret_cast<__half *>(uh), ldh, vec);
 	count_launches();
 	HPLAI_CUDA_TRY(cudaGetLastError());

@@ -88,6 +88,14 @@ def test_panel_solve_edges(hplai, oracle, torch_cuda, m, b, off):
     assert np.array_equal(h.cpu().numpy()[:, :b], ref.T.astype(np.float16))
 
 
+# around the rules' 32 and 64 columns and their 4736, 9472 and 16000 rows, blocks of 64 columns and remainders
+@pytest.mark.parametrize("m,b,off", [(33, 32, 0), (16001, 31, 0), (16001, 32, 0), (16000, 20, 1), (65, 33, 0), (40, 64, 0),
+                                     (4737, 64, 0), (9473, 65, 0), (9473, 128, 0), (9472, 129, 0), (9473, 200, 3),
+                                     (9500, 260, 0)])
+def test_panel_solve_widths(hplai, oracle, torch_cuda, m, b, off):
+    test_panel_solve_edges(hplai, oracle, torch_cuda, m, b, off)
+
+
 @pytest.mark.parametrize("n,b,flags", [(1200, 60, 0), (770, 70, 0), (1000, 125, 0), (1280, 128, 0), (2048, 512, 2),
                                        (1200, 50, 2)])
 def test_small_panels_are_the_substitution_panels(hplai, torch_cuda, n, b, flags):
