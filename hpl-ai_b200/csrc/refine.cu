@@ -463,13 +463,15 @@ __device__ __noinline__ void substitute_block(const float *T, double *x, int row
 	const int t = threadIdx.x, lane = t & 31;
 	for (int k = 0; k < TB / 32; ++k) {
 		const int c0 = LOWER ? 32 * k : TB - 32 * (k + 1);
+		if (c0 >= rows) continue;
 		if (t < 32) {
 			const int i = c0 + lane;
 			double v = x[i];
 			const double d = !LOWER && i < rows ? static_cast<double>(T[i * TB + i]) : 1.0;
-#pragma unroll
-			for (int q = 0; q < 32; ++q) {
-				const int j = LOWER ? q : 31 - q;
+			const int w = min(32, rows - c0);
+#pragma unroll 4
+			for (int q = 0; q < w; ++q) {
+				const int j = LOWER ? q : w - 1 - q;
 				if (!LOWER && lane == j) v /= d;
 				const double xj = __shfl_sync(0xffffffffu, v, j);
 				if (LOWER ? lane > j : lane < j) v = fma(-static_cast<double>(T[(c0 + j) * TB + i]), xj, v);
@@ -596,6 +598,12 @@ __global__ void __launch_bounds__(TRSV_THREADS, 1) trsv_kernel(int lower, int n,
 #pragma unroll
 				for (int q = 0; q < TB / 2; ++q) dv[q] = __ldcg(&dblock[static_cast<int64_t>(jb + q) * TB + lr]);
 			}
+		} else if (lower ? nblk <= 1 : nblk == 0 && rows <= 64) {
+			// the first blocks have no wait to hide an inverse in, and substitution is
+			// shorter where it does not divide or is small (inverse / so: L n = 16
+			// 11.6 / 7.3 us, 128 21.7 / 11.9, 256 23.8 / 19.6; U n = 32 13.6 / 9.5, 60 17.7 /
+			// 17.9, 128 21.7 / 28)
+			extra = 1;
 		} else {
 			double *X = reinterpret_cast<double *>(dyn_smem);
 			invert_block(X, a, lda, r0, rows, lower == 0);
