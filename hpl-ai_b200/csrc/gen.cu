@@ -56,15 +56,16 @@ constexpr int kFillRows4 = 4 * kFillRows;   // rows per CTA of fill_kernel (four
 // costs one warp-wide jump, and the state's conversion to FP64 leaves the
 // conversion pipe to the rounding to FP32 (biased_state_value).  n = 32768:
 // 1380 us with a row and two jumps per thread, 601 us (7.1 TB/s written) so.
+template <int COLS>
 __global__ void __launch_bounds__(kFillRows) fill_kernel(int n, int i0, int j0, int nrow, int ncol, float *a,
-	int64_t lda, uint64_t seed, int vec, int cols, JumpTable tab, Coeff jn)
+	int64_t lda, uint64_t seed, int vec, JumpTable tab, Coeff jn)
 {
 	__shared__ Coeff stab[64];
 	const int t = threadIdx.x, lane = t & 31;
 	if (t < 64) stab[t] = tab.p[t];
 	__syncthreads();
 	const int rw = blockIdx.x * kFillRows4 + (t - lane) * 4;   // the warp's first row
-	const int c0 = blockIdx.y * cols;
+	const int c0 = blockIdx.y * COLS;
 	if (rw >= nrow) return;
 	uint64_t s[4];
 	s[0] = coeff_apply(warp_jump(stab, static_cast<uint64_t>(i0 + rw) +
@@ -78,7 +79,7 @@ __global__ void __launch_bounds__(kFillRows) fill_kernel(int n, int i0, int j0, 
 #pragma unroll
 	for (int q = 0; q < 4; ++q) s[q] ^= 1ULL << 63;
 	const int r = rw + 4 * lane;
-	const int c1 = min(c0 + cols, ncol);
+	const int c1 = min(c0 + COLS, ncol);
 	float *col = a + static_cast<int64_t>(c0) * lda + r;
 	const bool whole = vec && r + 3 < nrow;
 	for (int c = c0; c < c1; ++c) {
@@ -380,14 +381,16 @@ int launch_fill(int n, int i0, int j0, int nrow, int ncol, float *a, int64_t lda
 {
 	if (nrow <= 0 || ncol <= 0) return HPLAI_OK;
 	const int gx = (nrow + kFillRows4 - 1) / kFillRows4;
-	// fewer columns per CTA while the CTAs are few (60 x 1140 5.5 us by one row per
+	// eight columns per CTA where the CTAs are few (60 x 1140 5.5 us by one row per
 	// thread, 7.0 with 32 columns, 5.4 so)
-	int cols = kFillCols;
-	while (cols > 4 && static_cast<int64_t>(gx) * (ncol / cols) < 96) cols /= 2;
+	constexpr int kFewCols = 8;
+	const bool few = static_cast<int64_t>(gx) * (ncol / kFillCols) < 96;
+	const int cols = few ? kFewCols : kFillCols;
 	const dim3 grid(gx, (ncol + cols - 1) / cols);
 	const int vec = (reinterpret_cast<uintptr_t>(a) % 16 == 0 && lda % 4 == 0) ? 1 : 0;
 	const Coeff jn = coeff_pow(static_cast<uint64_t>(n));
-	fill_kernel<<<grid, kFillRows, 0, st>>>(n, i0, j0, nrow, ncol, a, lda, seed, vec, cols, jump_table(), jn);
+	const auto kernel = few ? fill_kernel<kFewCols> : fill_kernel<kFillCols>;
+	kernel<<<grid, kFillRows, 0, st>>>(n, i0, j0, nrow, ncol, a, lda, seed, vec, jump_table(), jn);
 	count_launches();
 	HPLAI_CUDA_TRY(cudaGetLastError());
 	if (calc_diag && i0 == j0 && nrow == ncol) {
