@@ -293,7 +293,7 @@ int otf_launch(int64_t n, int mb, int nb, double alpha, const double *x, double 
 		// Rows / pieces, us: n = 1200 35 / 14.5, 16384 143 / 117, 24576 255 / 249,
 		// 32768 426 / 427, 65536 1592 / 1662, 131072 6220 / 6600; A^T 9600 71 / 55,
 		// 16384 131 / 123, 20480 183 / 186, 32768 405 / 457, 131072 5950 / 7090.
-		const bool wide = static_cast<int64_t>((mb + GEMV_ROWS - 1) / GEMV_ROWS) * nchunks >= (trans ? 800 : 2048);
+		const bool wide = static_cast<int64_t>((mb + GEMV_ROWS - 1) / GEMV_ROWS) * nchunks > (trans ? 800 : 2048);
 		const dim3 grid((mb + (wide ? GEMV_ROWS : 64) - 1) / (wide ? GEMV_ROWS : 64), nchunks);
 		const auto kernel = wide ? (trans ? otf_rows_kernel<true> : otf_rows_kernel<false>)
 		                         : (trans ? otf_pieces_kernel<true> : otf_pieces_kernel<false>);

@@ -189,7 +189,7 @@ def test_gemv_edges(hplai, oracle, torch_cuda, n):
         assert np.abs(yd.cpu().numpy() - ref).max() <= 1e-14 * (np.abs(a).sum(1).max() + 1)
 
 
-# a row per thread from 2048 blocks of 256 rows x 2048 columns on (transposed: 800): odd orders past the rules' lines
+# a row per thread past 2048 blocks of 256 rows x 2048 columns (transposed: 800): odd orders past the rules' lines
 def test_gemv_of_large_orders(hplai, oracle, torch_cuda):
     torch = torch_cuda
     n = 33001
