@@ -167,12 +167,36 @@ __device__ __forceinline__ bool all_agree(bool p) { return __syncthreads_and(p) 
 // and its neighbour that have no place there, two for operands.
 constexpr int kRes = 11;
 constexpr int kTeamTiles = kRes + 4;
+constexpr size_t kSmemBytes = static_cast<size_t>(kTeams) * kTeamTiles * kTileFloats * sizeof(float);
+constexpr int kMaxUnits = 320;   // of one team: a third of the 959 units of 32 x 32 tiles
+
+// A worker team's unit: a tile, with its neighbour towards the diagonal where it is
+// two off it.
+struct Unit {
+	int m, d, ti, tj, at;   // min(ti, tj), |ti - tj|, the tile, its place in shared memory (-1: none)
+	bool left;              // below the diagonal
+	__device__ __forceinline__ explicit Unit(uint32_t e)
+	    : m(e & 31u), d((e >> 5) & 31u), at(static_cast<int>(e >> 11) - 1), left(((e >> 10) & 1u) != 0)
+	{
+		ti = left ? m + d : m;
+		tj = left ? m : m + d;
+	}
+	static __device__ __forceinline__ uint32_t pack(int m, int d, bool left)
+	{
+		return static_cast<uint32_t>(m) | static_cast<uint32_t>(d) << 5 | (left ? 1u << 10 : 0u);
+	}
+	static __device__ __forceinline__ uint32_t place(uint32_t e, int at) { return e | static_cast<uint32_t>(at + 1) << 11; }
+	__device__ __forceinline__ int tiles() const { return d == 2 ? 2 : 1; }
+	__device__ __forceinline__ int ti2() const { return left ? ti : ti + 1; }
+	__device__ __forceinline__ int tj2() const { return left ? tj + 1 : tj; }
+};
 
 __global__ void __launch_bounds__(kThreads) getrf_tiles_kernel(int b, float *a, int64_t lda, GetrfWork *w,
 	uint32_t epoch)
 {
 	extern __shared__ __align__(16) float dyn[];
 	__shared__ __align__(16) float xchs[kTeams][kXchFloats];
+	__shared__ uint32_t lists[kTeams][kMaxUnits];
 	const int team = threadIdx.x / kTeam;
 	const Team tm{static_cast<int>(threadIdx.x) % kTeam, static_cast<int>(threadIdx.x) & 31,
 		static_cast<int>(threadIdx.x) % kTeam / 32, 1 + team};
@@ -263,10 +287,9 @@ __global__ void __launch_bounds__(kThreads) getrf_tiles_kernel(int b, float *a, 
 	}
 
 	// ---------------- worker teams ----------------
-	// worker team g owns the tiles g, g + nteams, ... (column-major tile index)
-	// that are two or more off the diagonal, each with its neighbour towards
-	// the diagonal if that is one off it, and the diagonal tiles from (3, 3)
-	// on; team numbers run across the CTAs first, so that neighbouring tiles
+	// a worker team owns tiles that are two or more off the diagonal, each with its
+	// neighbour towards the diagonal if that is one off it, and diagonal tiles from
+	// (3, 3) on; team numbers run across the CTAs first, so that the units of a step
 	// sit on different SMs
 	const int gid = team * (gridDim.x - 1) + (blockIdx.x - 1), nteams = (gridDim.x - 1) * kTeams;
 	float *const mem = dyn + team * kTeamTiles * kTileFloats;
@@ -274,35 +297,36 @@ __global__ void __launch_bounds__(kThreads) getrf_tiles_kernel(int b, float *a, 
 	            *const opU = opL + kTileFloats;
 	bool ok = true;   // the same in the whole team
 	auto rows_of = [b](int ti) { return min(T, b - ti * T); };
-	// A unit: its tile and the place of that tile among the resident ones, negative
-	// where there are more tiles than places.  The first units, which are final
-	// soonest, are those that do without (b = 1024 on 16 SMs: 0.96 ms with the last
-	// ones without, 0.87 so).  The tile steps by sums: with a division per tile a
-	// step's walk over the units took longer than its updates (0.87 -> 0.72 ms; on 8
-	// SMs 1.85 -> 1.45).
-	struct Unit {
-		int ti, tj, at;
-	};
-	const int step_i = nteams % nt, step_j = nteams / nt;
-	// tiles of a unit: two with its neighbour; none one off the diagonal (the unit two
-	// off it has it) and where the tile is the diagonal CTA's
-	auto tiles_of = [](const Unit &u) {
-		const int d = u.ti > u.tj ? u.ti - u.tj : u.tj - u.ti;
-		if (d == 1 || (d == 0 && u.ti < 3)) return 0;
-		return d == 2 ? 2 : 1;
-	};
-	auto next = [&](Unit &u) {
-		u.at += tiles_of(u);
-		u.ti += step_i;
-		u.tj += step_j;
-		if (u.ti >= nt) {
-			u.ti -= nt;
-			++u.tj;
+	// This team's units in the order of their shells m = min(ti, tj): a unit is
+	// final after step m, so the ones left at a step are the end of the list.  A
+	// shell has its diagonal tile from 3 on, then (m + d, m) and (m, m + d), d = 2, 3, ..;
+	// the units of all shells are dealt to the teams in turn, which shares every
+	// step's work evenly whatever the number of teams (dealt column by column, 33
+	// teams had a diagonal of 32 tiles each: b = 1024 on 12 SMs 1.40 ms a block, 0.75
+	// so).  The list is made once: finding the next unit by divisions at every step
+	// took longer than its updates (on 8 SMs 1.58 -> 1.14 ms).
+	auto has_diag = [](int m) { return m >= 3 ? 1 : 0; };
+	auto count = [&](int m) { return has_diag(m) + 2 * max(nt - m - 2, 0); };
+	int units = 0;
+	for (int m = 0; m < nt; ++m) units += count(m);
+	uint32_t *const list = lists[team];
+	const int n = units > gid ? (units - gid + nteams - 1) / nteams : 0;
+	for (int i = tm.tid; i < n; i += kTeam) {
+		int m = 0, p = gid + i * nteams;
+		while (p >= count(m)) p -= count(m++);
+		const int d = p < has_diag(m) ? 0 : 2 + (p - has_diag(m)) / 2;
+		list[i] = Unit::pack(m, d, (p - has_diag(m)) % 2 == 0);
+	}
+	tm.sync();
+	// places in shared memory for the last tiles: where there are more tiles than
+	// places the first units, final soonest, do without
+	if (tm.tid == 0)
+		for (int i = n - 1, at = kRes; i >= 0; --i) {
+			at -= Unit(list[i]).tiles();
+			if (at < 0) break;
+			list[i] = Unit::place(list[i], at);
 		}
-	};
-	Unit first{gid % nt, gid / nt, 0}, all = first;
-	while (all.tj < nt) next(all);
-	first.at = min(kRes - all.at, 0);
+	tm.sync();
 	auto load = [&](float *t, int ti, int tj) {
 		stage_tile(t, a, lda, ti * T, tj * T, rows_of(ti), rows_of(tj), vec, tm.tid, kTeam);
 	};
@@ -341,24 +365,24 @@ __global__ void __launch_bounds__(kThreads) getrf_tiles_kernel(int b, float *a, 
 		}
 		if (slot < 0) tm.sync();
 	};
-	for (Unit u = first; u.tj < nt; next(u)) {
-		if (u.at < 0 || tiles_of(u) == 0) continue;
+	for (int i = 0; i < n; ++i) {
+		const Unit u(list[i]);
+		if (u.at < 0) continue;
 		load(mem + u.at * kTileFloats, u.ti, u.tj);
-		if (u.ti - u.tj == 2) load(mem + (u.at + 1) * kTileFloats, u.ti, u.tj + 1);
-		if (u.tj - u.ti == 2) load(mem + (u.at + 1) * kTileFloats, u.ti + 1, u.tj);
+		if (u.d == 2) load(mem + (u.at + 1) * kTileFloats, u.ti2(), u.tj2());
 	}
 	stage_wait();
 	tm.sync();
-	for (int r = 0; r < nt && ok; ++r) {
-		while (first.tj < r) next(first);   // columns before r are done
+	for (int r = 0, i0 = 0; r < nt && ok; ++r) {
 		// the panel tiles of step r, then the trailing updates
-		for (Unit u = first; u.tj < nt && ok; next(u)) {
-			const int ti = u.ti, tj = u.tj;
-			if (ti == tj || min(ti, tj) != r || tiles_of(u) == 0) continue;
+		for (; ok && i0 < n; ++i0) {
+			const Unit u(list[i0]);
+			if (u.m != r) break;
+			if (u.d == 0) continue;
 			float *x = u.at >= 0 ? mem + u.at * kTileFloats : tmp;
-			const bool left = tj == r;
+			const bool left = u.left;
 			// L tile X <- X U(r,r)^{-1}, or U tile X <- L(r,r)^{-1} X (tile (r, r) is a whole one)
-			if (u.at < 0) load(x, ti, tj);
+			if (u.at < 0) load(x, u.ti, u.tj);
 			const bool mine = get_tile(opL, slot_of(r, r), final_tag, tm.tid, left);
 			stage_wait();
 			if (!arrived(mine)) break;
@@ -366,27 +390,22 @@ __global__ void __launch_bounds__(kThreads) getrf_tiles_kernel(int b, float *a, 
 				op_solve_l(tm, x, opL);
 			else
 				op_solve_u(tm, x, opL);
-			put_tile(x, slot_of(ti, tj), final_tag, tm.tid);
+			put_tile(x, slot_of(u.ti, u.tj), final_tag, tm.tid);
 			// its neighbour's last update, and on to the diagonal CTA
-			if (tiles_of(u) == 2)
-				update(left ? ti : r + 1, left ? r + 1 : tj, u.at >= 0 ? u.at + 1 : -1, r, left ? x : nullptr, left ? nullptr : x,
-					true);
-			store(x, ti, tj);
+			if (u.d == 2)
+				update(u.ti2(), u.tj2(), u.at >= 0 ? u.at + 1 : -1, r, left ? x : nullptr, left ? nullptr : x, true);
+			store(x, u.ti, u.tj);
 			if (u.at < 0) tm.sync();
 		}
-		for (Unit u = first; u.tj < nt && ok; next(u)) {
-			const int nu = tiles_of(u);
-			if (nu == 0 || min(u.ti, u.tj) <= r || (u.ti == u.tj && u.ti < r + 3)) continue;
-#pragma unroll 1
-			for (int h = 0; h < nu && ok; ++h)
-				update(u.ti + (h && u.ti < u.tj), u.tj + (h && u.ti > u.tj), u.at >= 0 ? u.at + h : -1, r, nullptr, nullptr,
-					u.ti == u.tj && u.ti == r + 3);
+		for (int i = i0; ok && i < n; ++i) {
+			const Unit u(list[i]);
+			if (u.d == 0 && u.m < r + 3) continue;   // the diagonal CTA has it
+			update(u.ti, u.tj, u.at, r, nullptr, nullptr, u.d == 0 && u.m == r + 3);
+			if (ok && u.d == 2) update(u.ti2(), u.tj2(), u.at >= 0 ? u.at + 1 : -1, r, nullptr, nullptr, false);
 		}
 	}
 	if (!ok && tm.tid == 0) atomicOr(&w->status, 1u);
 }
-
-constexpr size_t kSmemBytes = static_cast<size_t>(kTeams) * kTeamTiles * kTileFloats * sizeof(float);
 
 std::mutex g_static_mu;
 __device__ GetrfWork g_static_work;

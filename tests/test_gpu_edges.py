@@ -38,7 +38,7 @@ def test_getrf_tile_edges(hplai, oracle, torch_cuda, b, lda, off):
     assert _same_bits(_take(t, b, b, lda, off), oracle.getrf_nopiv(m))
 
 
-@pytest.mark.parametrize("n,b,side", [(3072, 1024, 2), (3072, 1024, 7), (3072, 1024, 16), (2700, 900, 9), (2048, 512, 4),
+@pytest.mark.parametrize("n,b,side", [(3072, 1024, 2), (3072, 1024, 7), (3072, 1024, 16), (3072, 1024, 12), (2700, 900, 9), (2048, 512, 4),
                                       (1280, 320, 3)])
 def test_getrf_on_few_sms(hplai, torch_cuda, n, b, side):
     """More tiles than a team has places for in shared memory, odd numbers of teams: the factors of the whole GPU."""
