@@ -127,11 +127,13 @@ __device__ __noinline__ void invert_block(R *smem, const float *__restrict__ a, 
 		const int s = t % kTriBlock, l0 = t / kTriBlock;
 #pragma unroll 1
 		for (int h = 0; h < 4; ++h) {
-			float f[16];
+			float f[16] = {};
+			if (32 * h < rows) {
 #pragma unroll
-			for (int q = 0; q < 16; ++q) {
-				const int l = min(l0 + 2 * (16 * h + q), rows - 1);   // put() drops what is past the last
-				f[q] = __ldcg(&a[static_cast<int64_t>(r0 + l) * lda + r0 + min(s, rows - 1)]);
+				for (int q = 0; q < 16; ++q) {
+					const int l = min(l0 + 2 * (16 * h + q), rows - 1);   // put() drops what is past the last
+					f[q] = __ldcg(&a[static_cast<int64_t>(r0 + l) * lda + r0 + min(s, rows - 1)]);
+				}
 			}
 #pragma unroll
 			for (int q = 0; q < 16; ++q) put(l0 + 2 * (16 * h + q), s, f[q]);
